@@ -34,6 +34,7 @@ CUDA_UNITS = {
     "ss4d_api.cu": [],
     "ss4d_noalloc.cu": [],
     "ss4d_batch.cu": [],
+    "ss4d_loop.cu": [],
     "ss4d_ws.cu": [],
     "ss4d_nn.cu": [],
     "ss4d_conv_tc.cu": [],

@@ -12,7 +12,7 @@
 #include <thread>
 #include <vector>
 
-#include "ss4d_kernels.cuh"
+#include "ss4d_loop.cuh"
 
 using namespace ss4d;
 
@@ -93,6 +93,7 @@ struct ss4d_solver {
     int device;
     int sm_count;
     int use_graph;
+    int max_grid; // ss4d_solver_set_tiling's cap on the loop's grid (0: none)
     int asm_kblock; // block order of the float-float faces and coefficient kernels (launch_assemble_ff_faces_range)
     long long launches;
     size_t bytes;
@@ -114,11 +115,14 @@ struct ss4d_solver {
     DevParams *d_params;
     DevParams *h_params;
     // graphs
-    cudaGraph_t graph64, graphmx;
-    cudaGraphExec_t exec64, execmx;
-    unsigned long long cond64, condmx;
+    cudaGraph_t graphmx;
+    cudaGraphExec_t execmx;
     int graph_failed;
     int last_graphed; // the last solve ran as a graph
+    // the persistent loop (ss4d_loop.cu): its barrier and partial sums
+    LoopGroup *d_group;
+    double *d_loop_parts;
+    int loop_blocks[2];  // its grid per form; 0: not known, -1: the graph's loop instead
     // rescale balls
     int *d_frame_first, *d_frame_count;
     double *d_bx, *d_by, *d_bz;
@@ -296,16 +300,10 @@ fail:
 
 static void free_graphs(ss4d_solver *s)
 {
-    if (s->exec64)
-        cudaGraphExecDestroy(s->exec64);
-    if (s->graph64)
-        cudaGraphDestroy(s->graph64);
     if (s->execmx)
         cudaGraphExecDestroy(s->execmx);
     if (s->graphmx)
         cudaGraphDestroy(s->graphmx);
-    s->exec64 = nullptr;
-    s->graph64 = nullptr;
     s->execmx = nullptr;
     s->graphmx = nullptr;
 }
@@ -321,7 +319,8 @@ extern "C" ss4d_status ss4d_solver_destroy(ss4d_solver *s)
     void *dev[] = {s->d_partial, s->d_scalar, s->d_state, s->d_params, s->d_scratch, s->d_coef_nat,
                    s->sb.R[0], s->sb.P[0], s->sb.coef[0], s->sb.coefq[0], s->sb.dR[0], s->sb.r32[0], s->sb.fn[0],
                    s->d_frame_first, s->d_frame_count, s->d_bx, s->d_by, s->d_bz, s->ws_x0, s->ws_y,
-                   s->hist[0], s->hist[1], s->hist[2], s->hist[3], s->sb.fd[0], s->d_ff, s->d_proj};
+                   s->hist[0], s->hist[1], s->hist[2], s->hist[3], s->sb.fd[0], s->d_ff, s->d_proj,
+                   s->d_group, s->d_loop_parts};
     for (void *p : dev)
         if (p)
             cudaFree(p);
@@ -381,6 +380,7 @@ extern "C" ss4d_status ss4d_solver_set_tiling(ss4d_solver *s, int k_block, int m
         c.grid = max_grid;
     REQ(2LL * c.grid <= s->n_partial, "grid larger than the partial-sum buffer");
     s->cfg = c;
+    s->max_grid = max_grid;
     s->sb.partial[1] = s->d_partial + c.grid;
     free_graphs(s); // kernel arguments changed
     return SS4D_OK;
@@ -580,7 +580,8 @@ static ss4d_status sor_reference(ss4d_solver *s, const ss4d_params *p, double *u
     return isfinite(R) ? SS4D_OK : SS4D_ERR_NONFINITE;
 }
 
-static ss4d_status build_graph(ss4d_solver *s, int mixed)
+// the mixed form's loop as a CUDA graph's while loop
+static ss4d_status build_graph(ss4d_solver *s)
 {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -616,18 +617,12 @@ static ss4d_status build_graph(ss4d_solver *s, int mixed)
         return SS4D_ERR_CUDA;
     }
     const unsigned long long hv = (unsigned long long)h;
-    if (!mixed) {
-        launch_sweep64(s->geo, s->sp, s->cfg, 1, s->sb, s->d_params, s->d_state, s->cap);
-        launch_sweep64(s->geo, s->sp, s->cfg, 0, s->sb, s->d_params, s->d_state, s->cap);
-        launch_ctrl64(s->sb, s->cfg.grid, s->d_params, s->d_state, hv, 1, s->cap);
-    } else {
-        launch_refine(s->geo, s->sp, s->cfg, 0, s->sb, s->d_params, s->d_state, s->cap);
-        launch_refine(s->geo, s->sp, s->cfg, 1, s->sb, s->d_params, s->d_state, s->cap);
-        launch_zero_delta(s->sp, s->sb, s->d_state, s->cap);
-        launch_sweep32(s->geo, s->sp, s->cfg, 1, s->sb, s->d_params, s->d_state, 0, s->cap);
-        launch_sweep32(s->geo, s->sp, s->cfg, 0, s->sb, s->d_params, s->d_state, 0, s->cap);
-        launch_ctrl_mixed(s->sb, s->cfg.grid, s->d_params, s->d_state, hv, 1, s->cap);
-    }
+    launch_refine(s->geo, s->sp, s->cfg, 0, s->sb, s->d_state, s->cap);
+    launch_refine(s->geo, s->sp, s->cfg, 1, s->sb, s->d_state, s->cap);
+    launch_zero_delta(s->sp, s->sb, s->d_state, s->cap);
+    launch_sweep32(s->geo, s->sp, s->cfg, 1, s->sb, s->d_params, s->d_state, s->cap);
+    launch_sweep32(s->geo, s->sp, s->cfg, 0, s->sb, s->d_params, s->d_state, s->cap);
+    launch_ctrl_mixed(s->sb, s->cfg.grid, s->d_params, s->d_state, hv, 1, s->cap);
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(s->cap, &captured);
     if (e != cudaSuccess) {
@@ -643,15 +638,8 @@ static ss4d_status build_graph(ss4d_solver *s, int mixed)
         set_err("cudaGraphInstantiate: %s", cudaGetErrorString(e));
         return SS4D_ERR_CUDA;
     }
-    if (mixed) {
-        s->graphmx = graph;
-        s->execmx = exec;
-        s->condmx = hv;
-    } else {
-        s->graph64 = graph;
-        s->exec64 = exec;
-        s->cond64 = hv;
-    }
+    s->graphmx = graph;
+    s->execmx = exec;
     return SS4D_OK;
 }
 
@@ -671,6 +659,10 @@ static ss4d_status finish_stats(ss4d_solver *s, ss4d_step_stats *stats, int mixe
         stats->warm_started = L.warm;
         stats->near_tolerance = L.near;
         stats->projected = mixed ? L.proj : 0;
+    }
+    if (L.status == SS4D_ERR_TIMEOUT) {
+        set_err("the persistent loop's barrier gave up a wait");
+        return SS4D_ERR_TIMEOUT;
     }
     if (L.status != SS4D_OK) {
         set_err("SOR residual became non-finite at iteration %d", L.z);
@@ -717,8 +709,8 @@ static ss4d_status ensure_ws_buffers(ss4d_solver *s)
 static ss4d_status ws_first_pass(ss4d_solver *s)
 {
     const SweepCfg &cfg = s->cfg;
-    launch_refine(s->geo, s->sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream);
-    launch_refine(s->geo, s->sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream);
+    launch_refine(s->geo, s->sp, cfg, 0, s->sb, s->d_state, s->stream);
+    launch_refine(s->geo, s->sp, cfg, 1, s->sb, s->d_state, s->stream);
     launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
     s->launches += 4; // a refinement pass is 3 launches
     return last_launch();
@@ -822,16 +814,16 @@ static int pre_form(const ss4d_solver *s, int mixed)
 }
 
 // the mixed loop's start correction: zero, or the extrapolation the previous
-// step's unpack left in dR[0] / dB (applied by the first refinement pass, or
-// by the first-difference kernel when the assembly formed that pass)
-static ss4d_status clear_corrections(ss4d_solver *s)
+// step's unpack left in dR[0] / dB, for the first refinement pass to apply.
+// Where the assembly formed that pass nothing reads the corrections before
+// the round's start writes them (ghost and padding cells are zero always).
+static ss4d_status clear_corrections(ss4d_solver *s, int pre)
 {
+    if (pre || extrapolating(s))
+        return SS4D_OK;
     const size_t fb = sizeof(float) * s->sp.cs;
-    if (!extrapolating(s)) {
-        CK(cudaMemsetAsync(s->sb.dR[0], 0, fb, s->stream));
-        CK(cudaMemsetAsync(s->sb.dB, 0, fb, s->stream));
-    }
-    CK(cudaMemsetAsync(s->sb.dR[1], 0, fb, s->stream));
+    CK(cudaMemsetAsync(s->sb.dR[0], 0, fb, s->stream));
+    CK(cudaMemsetAsync(s->sb.dB, 0, fb, s->stream));
     return SS4D_OK;
 }
 
@@ -898,14 +890,11 @@ static ss4d_status run_split_loop(ss4d_solver *s, const ss4d_params *p, int mixe
     CKS(upload_params(s, p));
     if (!mixed) {
         launch_loop_init(s->d_state, 0, s->stream);
-        timed(s, SS4D_K_SWEEP64, true,
-              [&] { launch_sweep64(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
-        launch_advance(s->d_state, s->stream);
-        s->launches += 3;
+        s->launches += 1;
     } else {
         // the first refinement pass adds the correction in dR[0] / dB to u
         // (or the assembly did, and formed the pass's residual: pre_next)
-        CKS(clear_corrections(s));
+        CKS(clear_corrections(s, pre));
         launch_loop_init(s->d_state, 0, s->stream, pre, spec);
         s->launches += 1;
         if (ws_this_step(s, mixed))
@@ -917,23 +906,86 @@ static ss4d_status run_split_loop(ss4d_solver *s, const ss4d_params *p, int mixe
     return drive_loop(s, p, mixed, mixed && ws_this_step(s, mixed) ? 1 : 0);
 }
 
+// The loop as one persistent cooperative launch (ss4d_loop.cu) rather than
+// the graph's while loop?  The plain form always: its flat walk of the
+// targets and the missing launches win at every size (a step at 32^3 x 8
+// 886 -> 683 us, 161 x 143 x 61 x 9 15.4 -> 12.7 ms, 256 x 256 x 128 x 8
+// 61.0 -> 60.1 ms).  The mixed form up to 9e6 voxels: there the loop's data (about 30
+// bytes per voxel) stays in L2 or near it, and the graph's body costs seven
+// launches an iteration (32^3 x 8 850 -> 453 us, 64 x 64 x 64 x 10 1648 ->
+// 1386 us, 131 x 129 x 65 x 8 3.94 -> 3.90 ms); beyond, the launches are lost
+// in the half-sweeps' time and the separate FP32 kernel, at 40 warps per SM
+// instead of 32, streams faster (161 x 143 x 61 x 9 5.53 against 5.58 ms,
+// 256 x 256 x 128 x 8 24.1 against 26.0 ms).
+#define LOOP_THREADS 512
+#define LOOP_MIXED_MAX_VOXELS 9000000
+static bool loop_persistent(const ss4d_solver *s, int mixed)
+{
+    return !mixed || s->geo.nint <= LOOP_MIXED_MAX_VOXELS;
+}
+
+// launches it from the state in d_state; *done = false when it cannot run here
+static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixed, bool *done)
+{
+    *done = false;
+    if (!s->loop_blocks[mixed]) {
+        const int g = loop_grid(mixed, 1, LOOP_THREADS, s->sm_count);
+        s->loop_blocks[mixed] = g > 0 ? g : -1;
+    }
+    if (s->loop_blocks[mixed] < 0)
+        return SS4D_OK;
+    LoopVol V = make_loop_vol(s->geo, s->sp, s->sb);
+    const long long need = ((long long)(mixed ? V.F.npairs : V.F.ntargets) + LOOP_THREADS - 1) / LOOP_THREADS;
+    int grid = need < s->loop_blocks[mixed] ? (int)need : s->loop_blocks[mixed];
+    if (s->max_grid > 0 && grid > s->max_grid)
+        grid = s->max_grid;
+    share_blocks(&V, 1, grid);
+    if (!s->d_group)
+        CKS(dmalloc(s, (void **)&s->d_group, sizeof(LoopGroup)));
+    if (!s->d_loop_parts) {
+        const int a = loop_grid(0, 1, LOOP_THREADS, s->sm_count), b = loop_grid(1, 1, LOOP_THREADS, s->sm_count);
+        CKS(dmalloc(s, (void **)&s->d_loop_parts, sizeof(double) * 4 * (a > b ? a : b)));
+    }
+    CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
+    const int bodies = mixed ? 4 * (p->maxNoGSIteration + 4) + 16 : p->maxNoGSIteration + 8;
+    cudaError_t e = launch_loop(mixed, &V, 1, grid, LOOP_THREADS, s->d_state, s->d_params, s->d_loop_parts,
+                                s->d_group, bodies, s->stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        s->loop_blocks[mixed] = -1; // from now on the graph's loop
+        return SS4D_OK;
+    }
+    s->launches += 1;
+    *done = true;
+    return SS4D_OK;
+}
+
 // the loop from the state the controller left (mode: that state's mode),
-// as the graph's while loop or host-driven, until it stops or pauses
+// as the persistent launch, the graph's while loop or host-driven, until it stops or pauses
 static ss4d_status drive_loop(ss4d_solver *s, const ss4d_params *p, int mixed, int mode)
 {
     const Geo &g = s->geo;
     const Split &sp = s->sp;
     const SweepCfg &cfg = s->cfg;
     bool graphed = false;
-    if (s->use_graph && !s->graph_failed && !s->timing) {
-        cudaGraphExec_t ex = mixed ? s->execmx : s->exec64;
-        if (!ex) {
-            if (build_graph(s, mixed) != SS4D_OK)
-                s->graph_failed = 1; // fall back to the host loop from now on
-            ex = mixed ? s->execmx : s->exec64;
-        }
-        if (ex) {
-            CK(cudaGraphLaunch(ex, s->stream));
+    if (s->use_graph && !s->timing && loop_persistent(s, mixed)) {
+        bool done = false;
+        CKS(run_persistent(s, p, mixed, &done));
+        s->last_graphed = 0;
+        if (done)
+            return SS4D_OK;
+    }
+    if (!mixed) { // the first red half-sweep
+        timed(s, SS4D_K_SWEEP64, true,
+              [&] { launch_sweep64(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
+        launch_advance(s->d_state, s->stream);
+        s->launches += 2;
+    }
+    if (mixed && s->use_graph && !s->graph_failed && !s->timing) {
+        if (!s->execmx && build_graph(s) != SS4D_OK)
+            s->graph_failed = 1; // fall back to the host loop from now on
+        if (s->execmx) {
+            CK(cudaGraphLaunch(s->execmx, s->stream));
             graphed = true;
         }
     }
@@ -951,14 +1003,14 @@ static ss4d_status drive_loop(ss4d_solver *s, const ss4d_params *p, int mixed, i
                 // kernels whose mode does not match return at once: only the
                 // ones that do the work are timed
                 timed(s, SS4D_K_REFINE, mode == 0,
-                      [&] { launch_refine(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
+                      [&] { launch_refine(g, sp, cfg, 0, s->sb, s->d_state, s->stream); });
                 timed(s, SS4D_K_REFINE, mode == 0,
-                      [&] { launch_refine(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream); });
+                      [&] { launch_refine(g, sp, cfg, 1, s->sb, s->d_state, s->stream); });
                 launch_zero_delta(sp, s->sb, s->d_state, s->stream);
                 timed(s, SS4D_K_SWEEP32, mode == 2,
-                      [&] { launch_sweep32(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, 0, s->stream); });
+                      [&] { launch_sweep32(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream); });
                 timed(s, SS4D_K_SWEEP32, mode != 0,
-                      [&] { launch_sweep32(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, 0, s->stream); });
+                      [&] { launch_sweep32(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
                 launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
                 s->launches += 7;
             }
@@ -981,8 +1033,8 @@ static ss4d_status refine_paused(ss4d_solver *s)
     const Geo &g = s->geo;
     const Split &sp = s->sp;
     const SweepCfg &cfg = s->cfg;
-    timed(s, SS4D_K_REFINE, true, [&] { launch_refine(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
-    timed(s, SS4D_K_REFINE, true, [&] { launch_refine(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream); });
+    timed(s, SS4D_K_REFINE, true, [&] { launch_refine(g, sp, cfg, 0, s->sb, s->d_state, s->stream); });
+    timed(s, SS4D_K_REFINE, true, [&] { launch_refine(g, sp, cfg, 1, s->sb, s->d_state, s->stream); });
     launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
     s->launches += 4;
     return last_launch();
@@ -990,11 +1042,10 @@ static ss4d_status refine_paused(ss4d_solver *s)
 
 // count the kernels of a graphed loop after the fact: the controller counts
 // the loop bodies it ran
-static void count_graph_launches(ss4d_solver *s, int mixed)
+static void count_graph_launches(ss4d_solver *s)
 {
-    if (!s->last_graphed)
-        return;
-    s->launches += (long long)(mixed ? 7 : 3) * s->h_state->bodies;
+    if (s->last_graphed)
+        s->launches += 7LL * s->h_state->bodies;
 }
 
 extern "C" ss4d_status ss4d_solver_set_timing(ss4d_solver *s, int enable)
@@ -1414,7 +1465,7 @@ static ss4d_status split_solve(ss4d_solver *s, const ss4d_params *p, double *d_u
     CKS(run_split_loop(s, p, mixed));
     CKS(unpack_step(s, s->d_state, d_u, mixed));
     ss4d_status st = finish_stats(s, stats, mixed);
-    count_graph_launches(s, mixed);
+    count_graph_launches(s);
     return st;
 }
 
@@ -1691,7 +1742,7 @@ extern "C" ss4d_status ss4d_seg_time_step_host(ss4d_solver *s, const ss4d_params
     unpack_done(s, up);
     s->have_g = 0;
     ss4d_status st = finish_stats(s, stats, mixed);
-    count_graph_launches(s, mixed);
+    count_graph_launches(s);
     CK(cudaEventRecord(s->side_ev, s->side));
     CK(cudaStreamWaitEvent(s->stream, s->side_ev, 0));
     CK(cudaEventRecord(s->ev1, s->stream));
@@ -2027,7 +2078,7 @@ ss4d_status ss4d::solver_prepare_step(ss4d_solver *s, const ss4d_params *p, doub
     }
     if (mixed) {
         s->have_g = 1; // a segmentation step: its change feeds the extrapolation
-        CKS(clear_corrections(s));
+        CKS(clear_corrections(s, pre));
     }
     return last_launch();
 }

@@ -10,11 +10,10 @@
 // volume has stopped, or (mixed form) is in another phase of its loop, is
 // skipped.  Residual partial sums are kept per (volume, block) in a fixed
 // order, and one controller runs every volume's stopping test (the
-// single-volume state machines of ss4d_sweep.cuh).  By default the whole
-// loop is one persistent launch (k_bsolve: a co-resident grid, its phases
-// separated by a bounded grid barrier, the controller in block 0);
-// otherwise each phase is a kernel of a CUDA graph's while loop, which the
-// controller keeps going while any volume is active.
+// single-volume state machines of ss4d_sweep.cuh) as kernels of a CUDA
+// graph's while loop, which it keeps going while any volume is active.  By
+// default the whole loop is one persistent launch instead (k_loop in
+// ss4d_loop.cu: a group of blocks per volume).
 #include <cuda_runtime.h>
 
 #include <math.h>
@@ -23,7 +22,7 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include "ss4d_sweep.cuh"
+#include "ss4d_loop.cuh"
 
 using namespace ss4d;
 
@@ -446,115 +445,6 @@ __global__ void k_bctrl_mixed(const double *__restrict__ pred, const double *__r
         cudaGraphSetConditional(h, any ? 1u : 0u);
 }
 
-// ---- the whole loop in one launch
-
-// A grid-wide barrier for a co-resident grid (cooperative launch): the last
-// block to arrive resets the count and advances the generation the others
-// wait on.  The wait is bounded (about a second of clock cycles); one that
-// runs out sets err and returns false, and the caller leaves its loop.
-struct GridBar {
-    unsigned count, gen;
-    int err, any;
-};
-
-__device__ __forceinline__ bool grid_sync(GridBar *gb)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *gen = &gb->gen;
-        const unsigned g0 = *gen;
-        __threadfence();
-        if (atomicAdd(&gb->count, 1u) == gridDim.x - 1) {
-            gb->count = 0;
-            __threadfence();
-            atomicAdd(&gb->gen, 1u);
-        } else {
-            const long long t0 = clock64();
-            while (*gen == g0) {
-                if (clock64() - t0 > (1LL << 31)) {
-                    atomicExch(&gb->err, 1);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return *(volatile int *)&gb->err == 0;
-}
-
-// The SOR loop of every volume as one persistent launch: the loop body's
-// phases (those of the graph's body: refinement, zeroed corrections, FP32
-// black and red sweeps, controller; or the FP64 black and red sweeps and the
-// controller) run back to back with a grid barrier between them, until the
-// controller finds no volume active or max_bodies bodies have run.  In the
-// mixed form a phase (and its barrier) is left out when no active volume is
-// in a mode it works on; every block reads the modes at the start of the
-// body, after the controller's barrier, so the choice is the same in all.
-// Six blocks of 256 threads per SM, as the separate kernels run (42
-// registers at most).
-template <int MIXED>
-__global__ void __launch_bounds__(256, 6) k_bsolve(const BVol *__restrict__ vols, int nv, long long total,
-                                                   LoopState *st, const DevParams *__restrict__ par, double *pred,
-                                                   double *pblack, GridBar *gb, int max_bodies)
-{
-    __shared__ double wacc[BWARPS][BMAX];
-    const int grid = gridDim.x;
-    for (int body = 0; body < max_bodies; ++body) {
-        if (MIXED) {
-            int m0 = 0, m1 = 0, m2 = 0; // active volumes in mode 0 (refine), 1 (start a round), 2 (sweep)
-            for (int v = 0; v < nv; ++v) {
-                if (st[v].stop)
-                    continue;
-                const int mode = st[v].mode;
-                m0 |= mode == 0;
-                m1 |= mode == 1;
-                m2 |= mode == 2;
-            }
-            if (m0) {
-                bapply_black(vols, nv, total, st);
-                if (!grid_sync(gb))
-                    return;
-                brefine<0>(vols, nv, total, st, pred, wacc);
-                if (!grid_sync(gb))
-                    return;
-                brefine<1>(vols, nv, total, st, pblack, wacc);
-                if (!grid_sync(gb))
-                    return;
-            }
-            if (m1) {
-                bzero_delta(vols, nv, st);
-                if (!grid_sync(gb))
-                    return;
-            }
-            if (m2) {
-                bsweep32<1>(vols, nv, total, st, par, pblack, wacc);
-                if (!grid_sync(gb))
-                    return;
-            }
-            if (m1 || m2)
-                bsweep32<0>(vols, nv, total, st, par, pred, wacc);
-        } else {
-            bsweep64<1>(vols, nv, total, st, pblack, wacc);
-            if (!grid_sync(gb))
-                return;
-            bsweep64<0>(vols, nv, total, st, pred, wacc);
-        }
-        if (!grid_sync(gb))
-            return;
-        if (blockIdx.x == 0) {
-            const int any = MIXED ? bctrl_mixed(pred, pblack, grid, nv, par, st) : bctrl(pred, pblack, grid, nv, par, st);
-            if (threadIdx.x == 0)
-                *(volatile int *)&gb->any = any;
-        }
-        if (!grid_sync(gb))
-            return;
-        if (*(volatile int *)&gb->any == 0)
-            return;
-    }
-}
-
 int bsweep_blocks_per_sm()
 {
     int a = 0, b = 0;
@@ -586,10 +476,14 @@ struct ss4d_batch {
     int use_graph, graph_failed;
     int mixed;
     int *d_pre, *h_pre; // per volume: the assembly formed the step's first refinement pass
-    GridBar *d_bar;     // the persistent loop's grid barrier and its "any volume active" flag
+    LoopVol h_loop[BMAX]; // the persistent loop: its volumes, their groups' barriers, partial sums
+    LoopGroup *d_groups;
+    double *d_loop_parts;
+    size_t loop_parts; // blocks d_loop_parts holds
     int persistent;     // run the loop as one persistent launch (default) or as the graph's while loop
     int withhold_barrier; // test of the timeout path (ss4d_batch_set_test_withhold_barrier)
-    int pgrid[2];       // co-resident blocks of k_bsolve<0/1> (0: not yet known)
+    int pgrid[2];       // co-resident blocks of the persistent loop per form (0: not yet known)
+    int loop_form;      // the form h_loop describes, plus 1 (0: not described)
 };
 
 static void bfree_graph(ss4d_batch *b)
@@ -622,8 +516,10 @@ extern "C" ss4d_status ss4d_batch_destroy(ss4d_batch *b)
         cudaFree(b->d_partial);
     if (b->d_pre)
         cudaFree(b->d_pre);
-    if (b->d_bar)
-        cudaFree(b->d_bar);
+    if (b->d_groups)
+        cudaFree(b->d_groups);
+    if (b->d_loop_parts)
+        cudaFree(b->d_loop_parts);
     if (b->h_pre)
         cudaFreeHost(b->h_pre);
     if (b->h_st)
@@ -656,6 +552,38 @@ static ss4d_status bdescribe(ss4d_batch *b)
     BCK(cudaMemcpyAsync(b->d_vols, b->h_vols, sizeof(BVol) * b->n, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream)); // h_vols may change before the next call
     b->dirty = 0;
+    b->loop_form = 0;
+    return SS4D_OK;
+}
+
+// The persistent loop's volumes and groups for the current form: the
+// co-resident grid dealt out in proportion to the volumes' targets.  Blocks
+// of 256 threads, four per SM: with blocks of 512 a small volume's share
+// rounds to half as many steps.
+#define BLOOP_THREADS 256
+static ss4d_status bdescribe_loop(ss4d_batch *b)
+{
+    const int f = b->mixed;
+    if (!b->pgrid[f])
+        b->pgrid[f] = loop_grid(f, b->n, BLOOP_THREADS, solver_sm_count(b->vol[0]));
+    if (b->pgrid[f] < b->n) {
+        b->pgrid[f] = 0;
+        return SS4D_OK; // not one block per volume: the graph's loop
+    }
+    if (b->loop_form == f + 1)
+        return SS4D_OK;
+    if (b->loop_parts < (size_t)b->pgrid[f]) {
+        if (b->d_loop_parts)
+            cudaFree(b->d_loop_parts);
+        b->d_loop_parts = nullptr;
+        b->loop_parts = 0;
+        BCK(cudaMalloc((void **)&b->d_loop_parts, sizeof(double) * 4 * b->pgrid[f]));
+        b->loop_parts = (size_t)b->pgrid[f];
+    }
+    for (int v = 0; v < b->n; ++v)
+        b->h_loop[v] = make_loop_vol(b->h_vols[v].g, b->h_vols[v].sp, b->h_vols[v].b);
+    share_blocks(b->h_loop, b->n, b->pgrid[f]);
+    b->loop_form = f + 1;
     return SS4D_OK;
 }
 
@@ -702,7 +630,7 @@ extern "C" ss4d_status ss4d_batch_create(int n, const ss4d_dims *dims, void *str
     if (e == cudaSuccess)
         e = cudaMallocHost((void **)&b->h_pre, sizeof(int) * n);
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&b->d_bar, sizeof(GridBar));
+        e = cudaMalloc((void **)&b->d_groups, sizeof(LoopGroup) * n);
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
@@ -929,10 +857,6 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
     if (b->mixed) // each volume's projected start (when enabled), on its own loop state
         for (int v = 0; v < b->n; ++v)
             BCKS(solver_project_start(b->vol[v], b->h_pre[v], b->d_st + v));
-    if (!b->mixed) {
-        launch_bsweep(b, 0, b->stream); // the first red half-sweep
-        k_binit<<<ib, 64, 0, b->stream>>>(b->d_st, b->n, 1, nullptr);
-    }
     BCK(cudaGetLastError());
     int maxit = 0;
     for (int v = 0; v < b->n; ++v)
@@ -942,30 +866,21 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
     const int guard_max = b->mixed ? 4 * (maxit + 4) + 16 : maxit + 8;
     bool graphed = false, persisted = false;
     if (b->persistent) {
+        BCKS(bdescribe_loop(b));
         const int f = b->mixed;
-        if (!b->pgrid[f]) {
-            int per = 0;
-            BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f ? (const void *)k_bsolve<1> : (const void *)k_bsolve<0>,
-                                                             256, 0));
-            const int cap = per * solver_sm_count(b->vol[0]);
-            b->pgrid[f] = cap < b->grid ? cap : b->grid; // the partial arrays hold b->grid blocks
-        }
         if (b->pgrid[f] > 0) {
-            BCK(cudaMemsetAsync(b->d_bar, 0, sizeof(GridBar), b->stream));
-            if (b->withhold_barrier) // the arrival count starts beyond the grid: no arrival completes the barrier
-                BCK(cudaMemsetAsync(&b->d_bar->count, 0x80, sizeof(unsigned), b->stream));
-            const BVol *vols = b->d_vols;
-            int nv = b->n, mb = guard_max;
-            long long total = b->total;
-            LoopState *st = b->d_st;
-            const DevParams *par = b->d_par;
-            double *pred = bpart(b, 0), *pblack = bpart(b, 1);
-            GridBar *gb = b->d_bar;
-            void *args[] = {(void *)&vols, &nv, &total, &st, (void *)&par, &pred, &pblack, &gb, &mb};
-            BCK(cudaLaunchCooperativeKernel(f ? (const void *)k_bsolve<1> : (const void *)k_bsolve<0>,
-                                            dim3(b->pgrid[f]), dim3(256), args, 0, b->stream));
+            BCK(cudaMemsetAsync(b->d_groups, 0, sizeof(LoopGroup) * b->n, b->stream));
+            if (b->withhold_barrier) // arrival counts far below any target: no arrival completes a barrier
+                BCK(cudaMemset2DAsync(&b->d_groups->count, sizeof(LoopGroup), 0x80, sizeof(unsigned), b->n, b->stream));
+            BCK(launch_loop(f, b->h_loop, b->n, b->pgrid[f], BLOOP_THREADS, b->d_st, b->d_par, b->d_loop_parts,
+                            b->d_groups, guard_max, b->stream));
             persisted = true;
         }
+    }
+    if (!persisted && !b->mixed) {
+        launch_bsweep(b, 0, b->stream); // the first red half-sweep
+        k_binit<<<ib, 64, 0, b->stream>>>(b->d_st, b->n, 1, nullptr);
+        BCK(cudaGetLastError());
     }
     if (!persisted && b->use_graph && !b->graph_failed) {
         if (!b->exec[b->mixed] && bbuild_graph(b) != SS4D_OK)
@@ -995,16 +910,7 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
         BCKS(solver_finish_step(b->vol[v], b->d_st + v, d_u[v]));
     BCK(cudaEventRecord(e1, b->stream));
     BCK(cudaMemcpyAsync(b->h_st, b->d_st, sizeof(LoopState) * b->n, cudaMemcpyDeviceToHost, b->stream));
-    GridBar hb;
-    memset(&hb, 0, sizeof hb);
-    if (persisted)
-        BCK(cudaMemcpyAsync(&hb, b->d_bar, sizeof(GridBar), cudaMemcpyDeviceToHost, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
-    if (hb.err) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return bfail(SS4D_ERR_TIMEOUT, "the persistent batch loop's grid barrier gave up a wait");
-    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1022,9 +928,11 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
             stats[v].projected = b->mixed ? L.proj : 0;
             stats[v].ms = ms;
         }
-        if (L.status != SS4D_OK)
+        if (L.status != SS4D_OK && worst != SS4D_ERR_TIMEOUT)
             worst = (ss4d_status)L.status;
     }
+    if (worst == SS4D_ERR_TIMEOUT)
+        return bfail(worst, "the persistent batch loop's barrier gave up a wait");
     if (worst != SS4D_OK)
         return bfail(worst, "a volume's SOR residual became non-finite");
     return SS4D_OK;

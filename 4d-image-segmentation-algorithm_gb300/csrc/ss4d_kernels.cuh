@@ -228,11 +228,11 @@ void launch_ctrl64(SplitBufs b, int nparts, const DevParams *dp, LoopState *stat
                    int use_cond, cudaStream_t st);
 
 // mixed precision
-void launch_refine(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
-                   LoopState *state, cudaStream_t st);
+void launch_refine(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, LoopState *state,
+                   cudaStream_t st);
 void launch_zero_delta(const Split &s, SplitBufs b, LoopState *state, cudaStream_t st);
 void launch_sweep32(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
-                    LoopState *state, int start_mode, cudaStream_t st);
+                    LoopState *state, cudaStream_t st);
 void launch_ctrl_mixed(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, unsigned long long cond_handle,
                        int use_cond, cudaStream_t st);
 

@@ -385,65 +385,49 @@ __global__ void k_ctrl64(SplitBufs b, int nparts, const DevParams *__restrict__ 
 // values), then k_refine<1> (the black residual against the updated red
 // values); r32 receives the residual for the next round.  Applying the black
 // correction first spares the red pass adding it to each of 8 neighbours.
-__global__ void __launch_bounds__(256) k_apply_black(Geo g, Split sp, SweepCfg cfg, SplitBufs b,
-                                                     const LoopState *__restrict__ st)
+__global__ void __launch_bounds__(256) k_apply_black(FlatIndex F, SplitBufs b, const LoopState *__restrict__ st)
 {
     if (st->mode != 0 || st->stop || st->pre) // pre: the first-difference kernel added it
         return;
-    const int tx = threadIdx.x & (cfg.XT - 1), ty = threadIdx.x / cfg.XT;
-    for (long long t = blockIdx.x; t < cfg.ntiles; t += gridDim.x) {
-        const TileCoord tc = tile_coord(g, cfg, t, tx, ty);
-        if (!tc.ok)
-            continue;
-        const int p = (1 + tc.j + tc.k + tc.l) & 1;
-        if (2 * tc.xi + 2 - p > g.nx)
-            continue;
-        const long long s = (((long long)tc.l * g.kM + tc.k) * g.jM + tc.j) * sp.Hs + tc.xi + sp.A;
-        b.Bk[s] += f2d_bits(b.dB[s]);
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < F.ntargets; q += gridDim.x * blockDim.x) {
+        const Place a = place<1>(F, F.dX, 1, q);
+        if (a.i <= F.nx)
+            b.Bk[a.s] += f2d_bits(b.dB[a.s]);
     }
 }
 
 template <int COL>
-__global__ void __launch_bounds__(256) k_refine(Geo g, Split sp, SweepCfg cfg, SplitBufs b,
-                                                const DevParams *__restrict__ dp, const LoopState *__restrict__ st)
+__global__ void __launch_bounds__(256) k_refine(FlatIndex F, SplitBufs b, const LoopState *__restrict__ st)
 {
     if (st->mode != 0 || st->stop)
         return;
-    const int ds = st->dsrc;
     double *own = COL == 0 ? b.R[0] : b.Bk;
-    const float *__restrict__ down = pick(b.dR, ds); // only used for COL == 0
+    const float *__restrict__ down = pick(b.dR, st->dsrc); // only used for COL == 0
     const double *__restrict__ oth = COL == 0 ? b.Bk : b.R[0];
     const double *__restrict__ cf = b.coef[COL];
     const double *__restrict__ pv = b.P[COL];
     float *__restrict__ rr = b.r32[COL];
-    const long long Hy = sp.Hs, Hz = Hy * g.jM, Hw = Hz * g.kM;
-    const int tx = threadIdx.x & (cfg.XT - 1), ty = threadIdx.x / cfg.XT;
     // pre: the first pass of a step whose residual the coefficient kernel
     // formed (with the same operations on the same values) and whose
     // correction the first-difference kernel added; only read here
     const bool pre = st->pre;
     const double *__restrict__ rp = b.rpre[COL];
     double acc = 0.0;
-    for (long long t = blockIdx.x; t < cfg.ntiles; t += gridDim.x) {
-        const TileCoord tc = tile_coord(g, cfg, t, tx, ty);
-        if (!tc.ok)
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < F.ntargets; q += gridDim.x * blockDim.x) {
+        const Place a = place<1>(F, F.dX, COL, q);
+        if (a.i > F.nx)
             continue;
-        const int p = (COL + tc.j + tc.k + tc.l) & 1;
-        const int i = 2 * tc.xi + 2 - p;
-        if (i > g.nx)
-            continue;
-        const long long s = (((long long)tc.l * g.kM + tc.k) * g.jM + tc.j) * Hy + tc.xi + sp.A;
         double r;
         if (pre) {
-            r = ld_stream(rp + s);
+            r = ld_stream(rp + a.s);
         } else {
-            const RefineOut o = refine_target<COL>(g, sp, tc, p, s, Hy, Hz, Hw, own, down, oth, cf, pv);
+            const RefineOut o = refine_at<COL, false>(a.p, a.s, a.t, F.Hs, F.Hz, F.Hw, own, down, oth, cf, pv);
             r = o.r;
             if (COL == 0)
-                own[s] = o.u;
+                own[a.s] = o.u;
         }
         acc = fma(r, r, acc);
-        rr[s] = d2f_bits(-r);
+        rr[a.s] = d2f_bits(-r);
     }
     acc = block_sum(acc);
     if (threadIdx.x == 0)
@@ -464,13 +448,13 @@ __global__ void k_zero_delta(Split sp, SplitBufs b, const LoopState *__restrict_
 }
 
 // FP32 half-sweep of colour COL: each thread updates two adjacent targets of
-// a row (pc: make_pair_cfg), so the pair shares its index arithmetic and reads its
+// a row (flat index of pairs), so the pair shares its index arithmetic and reads its
 // own values, right-hand sides and the y/z/w neighbours as 8-byte pairs; each
 // target's arithmetic is sweep32_target's (resid32 and the relaxed update).
 // The launch has the solver's persistent grid, whose every block writes its
 // partial residual sum.
 template <int COL>
-__global__ void __launch_bounds__(256) k_sweep32(Geo g, Split sp, SweepCfg pc, SplitBufs b,
+__global__ void __launch_bounds__(256) k_sweep32(FlatIndex F, SplitBufs b,
                                                  const DevParams *__restrict__ dp, const LoopState *__restrict__ st)
 {
     const int mode = st->mode;
@@ -493,22 +477,13 @@ __global__ void __launch_bounds__(256) k_sweep32(Geo g, Split sp, SweepCfg pc, S
     const float *__restrict__ cs = b.coefs[COL];
     const float *__restrict__ rhs = b.r32[COL];
     const float omega = (float)dp->omega;
-    // 32-bit offsets: a colour array holds fewer than 2^31 elements
-    const unsigned Hy = (unsigned)sp.Hs, Hz = Hy * (unsigned)g.jM, Hw = Hz * (unsigned)g.kM;
-    const int tx = threadIdx.x & (pc.XT - 1), ty = threadIdx.x / pc.XT;
     float acc = 0.f;
-    for (long long t = blockIdx.x; t < pc.ntiles; t += gridDim.x) {
-        const TileCoord tc = tile_coord(g, pc, t, tx, ty);
-        if (!tc.ok)
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < F.npairs; q += gridDim.x * blockDim.x) {
+        const Place a = place<2>(F, F.dP, COL, q);
+        if (a.i > F.nx)
             continue;
-        const int p = (COL + tc.j + tc.k + tc.l) & 1;
-        const int xi = 2 * tc.xi; // the pair's first target; the second is xi + 1
-        const int i = 2 * xi + 2 - p;
-        if (i > g.nx)
-            continue;
-        const unsigned s = (((unsigned)tc.l * g.kM + tc.k) * g.jM + tc.j) * Hy + xi + sp.A;
-        const unsigned tq = ((((unsigned)tc.l - 1) * g.nz + (tc.k - 1)) * g.ny + (tc.j - 1)) * sp.nxh + xi;
-        acc = sweep32_pair(p, s, tq, i + 2 <= g.nx, Hy, Hz, Hw, src, dst, oth, cq, cs, rhs, omega, acc);
+        acc = sweep32_pair<false>(a.p, a.s, a.t, a.i + 2 <= F.nx, F.Hs, F.Hz, F.Hw, src, dst, oth, cq, cs, rhs, omega,
+                                  acc);
     }
     const double tot = block_sum((double)acc);
     if (threadIdx.x == 0)
@@ -701,14 +676,15 @@ void launch_ctrl64(SplitBufs b, int nparts, const DevParams *dp, LoopState *stat
     k_ctrl64<<<1, 256, 0, st>>>(b, nparts, dp, state, (cudaGraphConditionalHandle)cond_handle, use_cond);
 }
 
-void launch_refine(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
-                   LoopState *state, cudaStream_t st)
+void launch_refine(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, LoopState *state,
+                   cudaStream_t st)
 {
+    const FlatIndex F = make_flat(g, s);
     if (colour == 0) {
-        k_apply_black<<<cfg.grid, cfg.threads, 0, st>>>(g, s, cfg, b, state);
-        k_refine<0><<<cfg.grid, cfg.threads, 0, st>>>(g, s, cfg, b, dp, state);
+        k_apply_black<<<cfg.grid, cfg.threads, 0, st>>>(F, b, state);
+        k_refine<0><<<cfg.grid, cfg.threads, 0, st>>>(F, b, state);
     } else {
-        k_refine<1><<<cfg.grid, cfg.threads, 0, st>>>(g, s, cfg, b, dp, state);
+        k_refine<1><<<cfg.grid, cfg.threads, 0, st>>>(F, b, state);
     }
 }
 
@@ -734,14 +710,13 @@ SweepCfg make_pair_cfg(const Geo &g, const Split &s, const SweepCfg &cfg)
 }
 
 void launch_sweep32(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
-                    LoopState *state, int start_mode, cudaStream_t st)
+                    LoopState *state, cudaStream_t st)
 {
-    (void)start_mode;
-    const SweepCfg pc = make_pair_cfg(g, s, cfg);
+    const FlatIndex F = make_flat(g, s);
     if (colour == 0)
-        k_sweep32<0><<<cfg.grid, cfg.threads, 0, st>>>(g, s, pc, b, dp, state);
+        k_sweep32<0><<<cfg.grid, cfg.threads, 0, st>>>(F, b, dp, state);
     else
-        k_sweep32<1><<<cfg.grid, cfg.threads, 0, st>>>(g, s, pc, b, dp, state);
+        k_sweep32<1><<<cfg.grid, cfg.threads, 0, st>>>(F, b, dp, state);
 }
 
 void launch_ctrl_mixed(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, unsigned long long cond_handle,

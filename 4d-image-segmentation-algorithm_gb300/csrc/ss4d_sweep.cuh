@@ -67,6 +67,37 @@ __device__ __forceinline__ T ld_ro(const T *p)
     return __ldg(p);
 }
 
+// LIVE: an array that other blocks of the same launch write between two
+// barriers (the persistent loop): a plain coherent load, which the compiler
+// may neither hoist over a barrier nor take through the read-only path
+template <bool LIVE>
+__device__ __forceinline__ double ld_oth(const double *p)
+{
+    if (!LIVE)
+        return __ldg(p);
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+template <bool LIVE>
+__device__ __forceinline__ float ld_oth(const float *p)
+{
+    if (!LIVE)
+        return __ldg(p);
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+template <bool LIVE>
+__device__ __forceinline__ float2 ld_oth(const float2 *p)
+{
+    if (!LIVE)
+        return __ldg(p);
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+
 // Select one of a pair held in a by-value kernel parameter without a runtime
 // array index (which would copy the parameter struct to local memory).
 template <typename T>
@@ -109,6 +140,68 @@ __device__ __forceinline__ TileCoord tile_coord(const Geo &g, const SweepCfg &cf
     return c;
 }
 
+// ---------------------------------------------------------------------------
+// One flat index over a colour's targets: x (in units of W adjacent columns)
+// fastest, then j, l, k slowest.  A grid-stride walk of it keeps every lane
+// of a warp at work whatever the row length (tiles of a power of two along x
+// left up to half of them idle: 41 of 64 at 161 voxels), and covers a few k planes
+// of all frames at a time, so the neighbouring planes' reads of the other
+// colour hit in L2.
+struct FlatIndex {
+    int nx, ny, nz, jM, kM, nxh, A;
+    unsigned Hs, Hz, Hw;       // split strides of j, k, l
+    unsigned npairs, ntargets; // pairs of adjacent columns, columns
+    FastDiv dP, dX, dJ, dL;    // pairs and columns per row, rows per plane, frames
+};
+
+inline FlatIndex make_flat(const Geo &g, const Split &sp)
+{
+    FlatIndex F;
+    F.nx = g.nx;
+    F.ny = g.ny;
+    F.nz = g.nz;
+    F.jM = g.jM;
+    F.kM = g.kM;
+    F.nxh = sp.nxh;
+    F.A = sp.A;
+    F.Hs = (unsigned)sp.Hs;
+    F.Hz = F.Hs * (unsigned)g.jM;
+    F.Hw = F.Hz * (unsigned)g.kM;
+    const unsigned npr = (unsigned)(sp.nxh + 1) / 2, rows = (unsigned)(g.ny * g.nz * g.nt);
+    F.npairs = npr * rows;
+    F.ntargets = (unsigned)sp.nxh * rows;
+    F.dP = make_fastdiv(npr);
+    F.dX = make_fastdiv((unsigned)sp.nxh);
+    F.dJ = make_fastdiv((unsigned)g.ny);
+    F.dL = make_fastdiv((unsigned)g.nt);
+    return F;
+}
+
+struct Place {
+    unsigned s, t; // split index of the (first) target, its compact record index
+    int p, i;      // row phase, x coordinate
+};
+
+// the target at (or the pair's first target at) flat index q of colour col
+template <int W>
+__device__ __forceinline__ Place place(const FlatIndex &F, const FastDiv &dx, int col, unsigned q)
+{
+    unsigned r = fdiv(q, dx);
+    const unsigned x = W * (q - r * dx.d);
+    unsigned h = fdiv(r, F.dJ);
+    const unsigned j = 1 + (r - h * F.dJ.d);
+    r = h;
+    h = fdiv(r, F.dL);
+    const unsigned l = 1 + (r - h * F.dL.d);
+    const unsigned k = 1 + h;
+    Place a;
+    a.p = (col + j + k + l) & 1;
+    a.i = 2 * (int)x + 2 - a.p;
+    a.s = ((l * F.kM + k) * F.jM + j) * F.Hs + x + F.A;
+    a.t = (((l - 1) * F.nz + (k - 1)) * F.ny + (j - 1)) * F.nxh + x;
+    return a;
+}
+
 // compact per-colour interior index of voxel (i, j, k, l)
 __device__ __forceinline__ long long coef_index(const Geo &g, const Split &sp, int i, int j, int k, int l)
 {
@@ -121,30 +214,38 @@ __device__ __forceinline__ long long tile_coef_index(const Geo &g, const Split &
     return ((((long long)(tc.l - 1) * g.nz + (tc.k - 1)) * g.ny + (tc.j - 1)) * sp.nxh) + tc.xi;
 }
 
-// One FP64 update of the target at split index s (row phase p):
+// One FP64 update of the target at split index s (row phase p, record tq):
 //   r = diag*u - (prev + sum_f c a_f u_f),   dst = u - (omega/diag) r.
 // Returns the pre-update residual r.
+template <bool LIVE>
+__device__ __forceinline__ double sweep64_at(int p, long long s, long long tq, long long Hy, long long Hz,
+                                             long long Hw, const double *src, double *dst, const double *oth,
+                                             const double *__restrict__ cf, const double *__restrict__ pv)
+{
+    const double u0 = LIVE ? __ldcg(src + s) : src[s];
+    const double *cv = cf + coef_at(tq, 0, 10); // component f at cv[32 f]
+    double S = fma(ld_stream(cv), ld_oth<LIVE>(oth + s - p + 1), ld_stream(pv + s));
+    S = fma(ld_stream(cv + 32), ld_oth<LIVE>(oth + s - p), S);
+    S = fma(ld_stream(cv + 64), ld_oth<LIVE>(oth + s + Hy), S);
+    S = fma(ld_stream(cv + 96), ld_oth<LIVE>(oth + s - Hy), S);
+    S = fma(ld_stream(cv + 128), ld_oth<LIVE>(oth + s + Hz), S);
+    S = fma(ld_stream(cv + 160), ld_oth<LIVE>(oth + s - Hz), S);
+    S = fma(ld_stream(cv + 192), ld_oth<LIVE>(oth + s + Hw), S);
+    S = fma(ld_stream(cv + 224), ld_oth<LIVE>(oth + s - Hw), S);
+    const double diag = ld_stream(cv + 256);
+    const double winv = ld_stream(cv + 288);
+    const double r = fma(diag, u0, -S); // S includes prev
+    dst[s] = fma(-winv, r, u0);
+    return r;
+}
+
 __device__ __forceinline__ double sweep64_target(const Geo &g, const Split &sp, const TileCoord &tc, int p,
                                                  long long s, const double *src, double *dst,
                                                  const double *__restrict__ oth, const double *__restrict__ cf,
                                                  const double *__restrict__ pv)
 {
     const long long Hy = sp.Hs, Hz = Hy * g.jM, Hw = Hz * g.kM;
-    const double u0 = src[s];
-    const double *cv = cf + coef_at(tile_coef_index(g, sp, tc), 0, 10); // component f at cv[32 f]
-    double S = fma(ld_stream(cv), ld_ro(oth + s - p + 1), ld_stream(pv + s));
-    S = fma(ld_stream(cv + 32), ld_ro(oth + s - p), S);
-    S = fma(ld_stream(cv + 64), ld_ro(oth + s + Hy), S);
-    S = fma(ld_stream(cv + 96), ld_ro(oth + s - Hy), S);
-    S = fma(ld_stream(cv + 128), ld_ro(oth + s + Hz), S);
-    S = fma(ld_stream(cv + 160), ld_ro(oth + s - Hz), S);
-    S = fma(ld_stream(cv + 192), ld_ro(oth + s + Hw), S);
-    S = fma(ld_stream(cv + 224), ld_ro(oth + s - Hw), S);
-    const double diag = ld_stream(cv + 256);
-    const double winv = ld_stream(cv + 288);
-    const double r = fma(diag, u0, -S); // S includes prev
-    dst[s] = fma(-winv, r, u0);
-    return r;
+    return sweep64_at<false>(p, s, tile_coef_index(g, sp, tc), Hy, Hz, Hw, src, dst, oth, cf, pv);
 }
 
 // ---------------------------------------------------------------------------
@@ -161,6 +262,23 @@ __device__ __forceinline__ double sweep64_target(const Geo &g, const Split &sp, 
 struct RefineOut {
     double r, u;
 };
+template <int COL, bool LIVE>
+__device__ __forceinline__ RefineOut refine_at(int p, long long s, long long tq, long long Hy, long long Hz,
+                                               long long Hw, const double *own, const float *down, const double *oth,
+                                               const double *__restrict__ cf, const double *__restrict__ pv)
+{
+    const long long nb[8] = {s - p + 1, s - p, s + Hy, s - Hy, s + Hz, s - Hz, s + Hw, s - Hw};
+    const double own_u = LIVE ? __ldcg(own + s) : own[s];
+    const double u0 = COL == 0 ? own_u + f2d_bits(LIVE ? __ldcg(down + s) : down[s]) : own_u;
+    const double *cv = cf + coef_at(tq, 0, 10);
+    double S = ld_stream(pv + s); // prev + sum_f c a_f u_f
+#pragma unroll
+    for (int f = 0; f < 8; ++f)
+        S = fma(ld_stream(cv + 32 * f), LIVE ? ld_oth<true>(oth + nb[f]) : oth[nb[f]], S);
+    const double diag = ld_stream(cv + 256);
+    return RefineOut{fma(diag, u0, -S), u0};
+}
+
 template <int COL>
 __device__ __forceinline__ RefineOut refine_target(const Geo &g, const Split &sp, const TileCoord &tc, int p,
                                                    long long s, long long Hy, long long Hz, long long Hw,
@@ -168,15 +286,7 @@ __device__ __forceinline__ RefineOut refine_target(const Geo &g, const Split &sp
                                                    const double *__restrict__ oth, const double *__restrict__ cf,
                                                    const double *__restrict__ pv)
 {
-    const long long nb[8] = {s - p + 1, s - p, s + Hy, s - Hy, s + Hz, s - Hz, s + Hw, s - Hw};
-    const double u0 = COL == 0 ? own[s] + f2d_bits(down[s]) : own[s];
-    const double *cv = cf + coef_at(tile_coef_index(g, sp, tc), 0, 10);
-    double S = ld_stream(pv + s); // prev + sum_f c a_f u_f
-#pragma unroll
-    for (int f = 0; f < 8; ++f)
-        S = fma(ld_stream(cv + 32 * f), oth[nb[f]], S);
-    const double diag = ld_stream(cv + 256);
-    return RefineOut{fma(diag, u0, -S), u0};
+    return refine_at<COL, false>(p, s, tile_coef_index(g, sp, tc), Hy, Hz, Hw, own, down, oth, cf, pv);
 }
 
 // Records of the FP32 correction sweeps.  The sweeps stream their records
@@ -276,12 +386,13 @@ __device__ __forceinline__ Sweep32Out sweep32_target(const Geo &g, const Split &
 // values, right-hand sides and y/z/w neighbours as 8-byte pairs and shares
 // its index arithmetic; each target's arithmetic is sweep32_target's.
 // Returns acc plus the squared pre-update residuals (first target first).
+template <bool LIVE>
 __device__ __forceinline__ float sweep32_pair(int p, unsigned s, unsigned tq, bool two, unsigned Hy, unsigned Hz,
-                                              unsigned Hw, const float *src, float *dst, const float *__restrict__ oth,
+                                              unsigned Hw, const float *src, float *dst, const float *oth,
                                               const uint4 *__restrict__ cq, const float *__restrict__ cs,
                                               const float *__restrict__ rhs, float omega, float acc)
 {
-    const float2 u = *reinterpret_cast<const float2 *>(src + s);
+    const float2 u = LIVE ? __ldcg(reinterpret_cast<const float2 *>(src + s)) : *reinterpret_cast<const float2 *>(src + s);
     const float2 rh = __ldcs(reinterpret_cast<const float2 *>(rhs + s));
     float w0[8], w1[8];
     const float sc0 = load_coef16(cq, cs, tq, w0);
@@ -289,14 +400,14 @@ __device__ __forceinline__ float sweep32_pair(int p, unsigned s, unsigned tq, bo
     if (two)
         sc1 = load_coef16(cq, cs, tq + 1, w1);
     // x neighbours of the pair: the other colour's columns s - p .. s - p + 2
-    const float2 vx = ld_ro(reinterpret_cast<const float2 *>(oth + s));
-    const float ex = ld_ro(oth + (p ? s - 1 : s + 2));
-    const float2 yp = ld_ro(reinterpret_cast<const float2 *>(oth + s + Hy));
-    const float2 ym = ld_ro(reinterpret_cast<const float2 *>(oth + s - Hy));
-    const float2 zp = ld_ro(reinterpret_cast<const float2 *>(oth + s + Hz));
-    const float2 zm = ld_ro(reinterpret_cast<const float2 *>(oth + s - Hz));
-    const float2 wp = ld_ro(reinterpret_cast<const float2 *>(oth + s + Hw));
-    const float2 wm = ld_ro(reinterpret_cast<const float2 *>(oth + s - Hw));
+    const float2 vx = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s));
+    const float ex = ld_oth<LIVE>(oth + (p ? s - 1 : s + 2));
+    const float2 yp = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s + Hy));
+    const float2 ym = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s - Hy));
+    const float2 zp = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s + Hz));
+    const float2 zm = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s - Hz));
+    const float2 wp = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s + Hw));
+    const float2 wm = ld_oth<LIVE>(reinterpret_cast<const float2 *>(oth + s - Hw));
     // record order: +x (column s_t - p + 1), -x (s_t - p), +y, -y, +z, -z, +w, -w
     const float nb0[8] = {p ? vx.x : vx.y, p ? ex : vx.x, yp.x, ym.x, zp.x, zm.x, wp.x, wm.x};
     float d0;

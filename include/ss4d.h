@@ -133,9 +133,10 @@ ss4d_status ss4d_solver_create(const ss4d_dims *dims, ss4d_arith arith, void *st
 ss4d_status ss4d_solver_destroy(ss4d_solver *s);
 ss4d_status ss4d_solver_set_stream(ss4d_solver *s, void *stream);
 ss4d_status ss4d_solver_set_arith(ss4d_solver *s, ss4d_arith arith);
-/* Tile schedule of the colour-split sweeps: k_block = depth of the k blocks
- * in the tile order (>= 1), max_grid caps the persistent grid (0 = as many
- * blocks as fit on the device).  Results do not depend on either. */
+/* Schedule of the colour-split sweeps: k_block = depth of the k blocks in
+ * the tile order of the kernels that walk tiles (>= 1), max_grid caps the
+ * persistent grid (0 = as many blocks as fit on the device).  Results do not
+ * depend on either. */
 ss4d_status ss4d_solver_set_tiling(ss4d_solver *s, int k_block, int max_grid);
 /* Block order of the mixed form's coefficient assembly (its faces and
  * coefficient kernels): 0 = frame by frame; planes >= 1 = in blocks of that
@@ -168,7 +169,10 @@ ss4d_status ss4d_solver_set_projection(ss4d_solver *s, int enable);
  * depends on it: the stop rule is the FP64 residual of u.  No counterpart in
  * the reference. */
 ss4d_status ss4d_solver_set_inner_omega(ss4d_solver *s, double omega);
-/* Use (1) or bypass (0) the CUDA-graph form of the sweep loop (default 1). */
+/* Run the sweep loop on the device (1, the default: one persistent
+ * cooperative launch, or for large mixed-form volumes a CUDA graph's while
+ * loop) or drive it from the host, one readback per iteration (0).  Results
+ * do not depend on it except through the residual's summation order. */
 ss4d_status ss4d_solver_set_graph(ss4d_solver *s, int enable);
 /* Per-kernel timing.  While enabled, the sweep loop runs host-driven (not
  * as a graph) and every launch of the kernels below is bracketed by CUDA
@@ -391,13 +395,15 @@ ss4d_status ss4d_mcf_exact_solution(ss4d_solver *s, double h, double t, double *
 /* Many independent volumes, of different sizes and parameters, advanced
  * together in the plain FP64 form (default) or the mixed form
  * (ss4d_batch_set_arith).  The SOR loop of all volumes is ONE persistent
- * launch (a co-resident grid whose phases, the half-sweeps and in the mixed
- * form the refinement passes, walk the concatenated tiles of all volumes,
- * with a bounded grid barrier between phases: SS4D_ERR_TIMEOUT if one gives
- * up); ss4d_batch_set_persistent(b, 0) runs the same phases as kernels of a
- * CUDA graph's while loop instead.  Each volume keeps its own stopping test
- * (sum r^2 h^4 <= its gsTol, or its maxNoGSIteration) and once it has
- * stopped its tiles return at once.  In the mixed form each volume's
+ * launch: a co-resident grid of which every volume has a group of blocks of
+ * its own, in proportion to its voxels, that runs the volume's half-sweeps
+ * (and in the mixed form its refinement passes) with a bounded barrier of
+ * the group between them: SS4D_ERR_TIMEOUT if one gives up.
+ * ss4d_batch_set_persistent(b, 0) runs the phases of all volumes as kernels
+ * of a CUDA graph's while loop instead, over the concatenated tiles of the
+ * volumes; a volume that has stopped returns at once.  Each volume keeps its
+ * own stopping test (sum r^2 h^4 <= its gsTol, or its maxNoGSIteration).  In
+ * the mixed form each volume's
  * coefficient assembly also forms its step's first refinement pass, as
  * ss4d_seg_time_step does.  The
  * reference runs one volume per process, so these entry points have no
@@ -413,10 +419,10 @@ ss4d_status ss4d_batch_set_graph(ss4d_batch *b, int enable);
  * while loop (or host-driven, with ss4d_batch_set_graph(b, 0)).  Results do
  * not depend on it except through the residual's summation order. */
 ss4d_status ss4d_batch_set_persistent(ss4d_batch *b, int enable);
-/* Test of the timeout path, no fault: with enable the persistent loop's grid
- * barrier starts with its arrival count beyond the grid, so no arrival
- * completes it; every block's first wait runs out after about a second and
- * the step returns SS4D_ERR_TIMEOUT with the context usable.  The volumes'
+/* Test of the timeout path, no fault: with enable the persistent loop's
+ * barriers start with arrival counts that no arrival brings to the number
+ * awaited; every block's first wait runs out after about a second and the
+ * step returns SS4D_ERR_TIMEOUT with the context usable.  The volumes'
  * states after such a step are undefined. */
 ss4d_status ss4d_batch_set_test_withhold_barrier(ss4d_batch *b, int enable);
 /* Arithmetic form of the batched steps: SS4D_ARITH_FP64 (the default) or
@@ -430,7 +436,8 @@ ss4d_status ss4d_batch_set_extrapolation(ss4d_batch *b, int order);
 /* Mixed form with extrapolation of order 3: every volume's first FP32 round
  * starts from its projected start (ss4d_solver_set_projection per volume). */
 ss4d_status ss4d_batch_set_projection(ss4d_batch *b, int enable);
-/* Tile shape of volume v: xt threads along x (power of two, 8..256; 0 =
+/* Tile shape of volume v in the loops that walk tiles (not the persistent
+ * one, whose walk has none): xt threads along x (power of two, 8..256; 0 =
  * automatic) and k-block depth k_block (>= 1).  Results do not depend on it. */
 ss4d_status ss4d_batch_set_shape(ss4d_batch *b, int v, int xt, int k_block);
 /* Autotuner: for every volume, time candidate tile shapes on that volume's

@@ -12,7 +12,7 @@
 #include <thread>
 #include <vector>
 
-#include "ss4d_loop.cuh"
+#include "ss4d_front.cuh"
 
 using namespace ss4d;
 
@@ -105,7 +105,9 @@ struct ss4d_solver {
     double *h_scalar; // pinned mirror
     // natural-layout scratch
     double *d_scratch;
-    float2 *d_ff;      // mixed form's edge detector: 3 float-float volumes (image, thresholded image, prev)
+    float4 *d_fold[2]; // mixed form's edge detector: the smoothed images folded in k (ss4d_front_ff.cu)
+    FrontState *d_front, *h_front; // the presmoothing's outcome
+    double *d_front_parts;
     double *d_coef_nat; // 8 arrays (reference arithmetic)
     // split form
     SplitBufs sb;
@@ -319,7 +321,7 @@ extern "C" ss4d_status ss4d_solver_destroy(ss4d_solver *s)
     void *dev[] = {s->d_partial, s->d_scalar, s->d_state, s->d_params, s->d_scratch, s->d_coef_nat,
                    s->sb.R[0], s->sb.P[0], s->sb.coef[0], s->sb.coefq[0], s->sb.dR[0], s->sb.r32[0], s->sb.fn[0],
                    s->d_frame_first, s->d_frame_count, s->d_bx, s->d_by, s->d_bz, s->ws_x0, s->ws_y,
-                   s->hist[0], s->hist[1], s->hist[2], s->hist[3], s->sb.fd[0], s->d_ff, s->d_proj,
+                   s->hist[0], s->hist[1], s->hist[2], s->hist[3], s->sb.fd[0], s->d_fold[0], s->d_fold[1], s->d_proj, s->d_front, s->d_front_parts,
                    s->d_group, s->d_loop_parts};
     for (void *p : dev)
         if (p)
@@ -330,6 +332,8 @@ extern "C" ss4d_status ss4d_solver_destroy(ss4d_solver *s)
         cudaFreeHost(s->h_state);
     if (s->h_params)
         cudaFreeHost(s->h_params);
+    if (s->h_front)
+        cudaFreeHost(s->h_front);
     if (s->ev0)
         cudaEventDestroy(s->ev0);
     if (s->ev1)
@@ -425,10 +429,10 @@ static ss4d_status ensure_scratch(ss4d_solver *s)
     return SS4D_OK;
 }
 
-static ss4d_status ensure_ff_front(ss4d_solver *s)
+static ss4d_status ensure_fold(ss4d_solver *s, int image)
 {
-    if (!s->d_ff)
-        CKS(dmalloc(s, (void **)&s->d_ff, sizeof(float2) * 3 * s->geo.n));
+    if (!s->d_fold[image])
+        CKS(dmalloc(s, (void **)&s->d_fold[image], sizeof(float4) * fold_units(s->geo)));
     return SS4D_OK;
 }
 
@@ -441,22 +445,37 @@ static ss4d_status ensure_coef_nat(ss4d_solver *s)
     return SS4D_OK;
 }
 
+// the split copies of u (red twice, black) and prev; between steps they are
+// the presmoothing's workspace too (a step writes every cell it reads)
+static ss4d_status ensure_split_u(ss4d_solver *s)
+{
+    const long long cs = s->sp.cs;
+    if (!s->sb.R[0]) {
+        double *u3 = nullptr;
+        CKS(dmalloc(s, (void **)&u3, sizeof(double) * 3 * cs));
+        s->sb.R[0] = u3;
+        s->sb.R[1] = u3 + cs;
+        s->sb.Bk = u3 + 2 * cs;
+        CK(cudaMemsetAsync(u3, 0, sizeof(double) * 3 * cs, s->stream));
+    }
+    if (!s->sb.P[0]) {
+        double *p2 = nullptr;
+        CKS(dmalloc(s, (void **)&p2, sizeof(double) * 2 * cs));
+        s->sb.P[0] = p2;
+        s->sb.P[1] = p2 + cs;
+        CK(cudaMemsetAsync(p2, 0, sizeof(double) * 2 * cs, s->stream));
+    }
+    return SS4D_OK;
+}
+
 static ss4d_status ensure_split(ss4d_solver *s, int mixed)
 {
     const long long cs = s->sp.cs;
     if (!s->have_split) {
-        double *u3 = nullptr, *p2 = nullptr, *cf = nullptr;
-        CKS(dmalloc(s, (void **)&u3, sizeof(double) * 3 * cs));
-        CKS(dmalloc(s, (void **)&p2, sizeof(double) * 2 * cs));
+        double *cf = nullptr;
+        CKS(ensure_split_u(s));
         CKS(dmalloc(s, (void **)&cf, sizeof(double) * 20 * s->sp.ct));
-        CK(cudaMemsetAsync(u3, 0, sizeof(double) * 3 * cs, s->stream));
-        CK(cudaMemsetAsync(p2, 0, sizeof(double) * 2 * cs, s->stream));
         CK(cudaMemsetAsync(cf, 0, sizeof(double) * 20 * s->sp.ct, s->stream));
-        s->sb.R[0] = u3;
-        s->sb.R[1] = u3 + cs;
-        s->sb.Bk = u3 + 2 * cs;
-        s->sb.P[0] = p2;
-        s->sb.P[1] = p2 + cs;
         s->sb.coef[0] = cf;
         s->sb.coef[1] = cf + 10 * s->sp.ct;
         s->sb.partial[0] = s->d_partial;
@@ -1147,60 +1166,79 @@ extern "C" ss4d_status ss4d_reflect(ss4d_solver *s, double *d_img)
 {
     REQ(s && d_img, "NULL argument");
     launch_reflect(s->geo, d_img, s->stream);
-    s->launches += 4;
+    s->launches += 1;
     return last_launch();
 }
 
-// The mixed form's presmoothing: the same SOR on float-float copies of the
-// image (slot 0 or 1 of d_ff) and of its input (slot 2), written back to
-// the image's interior at the end; the float-float result stays in its slot
-// for the g faces.  prev (the reference's prev_u) receives the input as in
-// the FP64 forms.
-static ss4d_status presmooth_ff(ss4d_solver *s, const ss4d_params *p, double *d_img, double *prev, int slot,
-                                ss4d_step_stats *stats)
+// One presmoothing (ss4d_front.cuh) queued: d_img in place; its outcome goes
+// to slot `slot` of d_front.  fold (mixed form, may be null) receives the
+// smoothed image for the g faces; last: the residual after the last iteration
+// is wanted.
+static ss4d_status presmooth_queue(ss4d_solver *s, const ss4d_params *p, double *d_img, double *d_scratch, float4 *fold,
+                                   int last, int slot)
 {
-    CKS(ensure_ff_front(s));
+    CKS(ensure_split_u(s));
     const Geo &g = s->geo;
-    float2 *v = s->d_ff + (size_t)slot * g.n, *pf = s->d_ff + 2 * (size_t)g.n;
-    CK(cudaEventRecord(s->ev0, s->stream));
-    CK(cudaMemcpyAsync(prev, d_img, sizeof(double) * g.n, cudaMemcpyDeviceToDevice, s->stream));
-    launch_reflect(g, d_img, s->stream);
-    launch_to_ff(g, d_img, v, s->stream);
-    launch_to_ff(g, prev, pf, s->stream);
-    s->launches += 6;
-    const double c = p->sigma / (p->h * p->h), h4 = p->h * p->h * p->h * p->h;
-    const long long nb = front_resid_blocks(g);
-    // the residual's squares are summed in FP32 per thread: a test within
-    // 1e-6 of gsTol is reported as near the tolerance
-    const double band = fabs(p->gsTol) * 1e-6;
-    double R = 0.0, R1 = 0.0;
-    int z = 0, near = 0;
-    do {
-        z = z + 1;
-        launch_presmooth_half_ff(g, v, pf, c, p->omega_sigma, 0, s->stream);
-        launch_presmooth_half_ff(g, v, pf, c, p->omega_sigma, 1, s->stream);
-        launch_presmooth_resid_ff(g, v, pf, c, h4, s->d_partial, s->stream);
-        s->launches += 3 + launch_reduce_sum(s->d_partial, nb, s->d_scalar, s->stream);
-        CKS(last_launch());
-        CKS(read_scalar(s, 0, &R));
-        if (z == 1)
-            R1 = R;
-        near |= fabs(R - p->gsTol) <= band;
-    } while (R > p->gsTol && z < p->maxNoGSIteration_sigma);
-    launch_from_ff(g, v, d_img, s->stream);
-    s->launches += 1;
-    CKS(last_launch());
-    CK(cudaEventRecord(s->ev1, s->stream));
-    CK(cudaEventSynchronize(s->ev1));
-    if (stats) {
-        memset(stats, 0, sizeof *stats);
-        stats->iterations = z;
-        stats->residual = R;
-        stats->first_residual = R1;
-        stats->near_tolerance = near;
-        cudaEventElapsedTime(&stats->ms, s->ev0, s->ev1);
-        stats->status = isfinite(R) ? SS4D_OK : SS4D_ERR_NONFINITE;
+    const int mixed = s->arith == SS4D_ARITH_MIXED;
+    const int most = mixed ? presmooth_ff_grid(s->sm_count) : presmooth64_grid(s->sm_count);
+    if (!s->d_front) {
+        CKS(dmalloc(s, (void **)&s->d_front, 2 * sizeof(FrontState)));
+        CK(cudaMallocHost((void **)&s->h_front, 2 * sizeof(FrontState)));
     }
+    if (!s->d_group)
+        CKS(dmalloc(s, (void **)&s->d_group, sizeof(LoopGroup)));
+    if (!s->d_front_parts) {
+        const int a = presmooth_ff_grid(s->sm_count), b = presmooth64_grid(s->sm_count);
+        CKS(dmalloc(s, (void **)&s->d_front_parts, sizeof(double) * 4 * (a > b ? a : b)));
+    }
+    if (d_scratch) // the reference's prev_u
+        CK(cudaMemcpyAsync(d_scratch, d_img, sizeof(double) * g.n, cudaMemcpyDeviceToDevice, s->stream));
+    FrontArgs a;
+    memset(&a, 0, sizeof a);
+    a.g = g;
+    a.F = make_flat(g, s->sp);
+    a.img = d_img;
+    for (int c = 0; c < 2; ++c) {
+        a.P[c] = s->sb.P[c];
+        a.R[c] = s->sb.R[c];
+    }
+    a.B = s->sb.Bk;
+    a.fold = fold;
+    a.Hk = fold_of(g);
+    a.fold_scale = fold_scale(p->h);
+    a.c = p->sigma / (p->h * p->h);
+    a.omega = p->omega_sigma;
+    a.d = 1 + a.c * 8;
+    a.y = mixed ? 1.0 / a.d : div_const_recip(a.d);
+    a.h4 = p->h * p->h * p->h * p->h;
+    a.tol = p->gsTol;
+    a.maxit = p->maxNoGSIteration_sigma;
+    // float-float form: a residual is formed to about 1e-7 of itself in FP32
+    // squares, so a test within 1e-6 of gsTol is reported as near the tolerance
+    a.band = mixed ? fabs(p->gsTol) * 1e-6 : near_band(p->gsTol, g.nint);
+    a.last = last;
+    a.parts = s->d_front_parts;
+    a.group = s->d_group;
+    a.st = s->d_front + slot;
+    const int threads = mixed ? FRONT_FF_THREADS : FRONT64_THREADS;
+    const long long need = ((long long)a.F.npairs + threads - 1) / threads;
+    const int grid = need < most ? (int)need : most;
+    CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
+    CK(mixed ? launch_presmooth_ff(a, grid, s->stream) : launch_presmooth64(a, grid, s->stream));
+    s->launches += 1;
+    return SS4D_OK;
+}
+
+// the outcomes of the first n presmoothings queued
+static ss4d_status presmooth_wait(ss4d_solver *s, int n)
+{
+    CK(cudaMemcpyAsync(s->h_front, s->d_front, n * sizeof(FrontState), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    for (int k = 0; k < n; ++k)
+        if (s->h_front[k].status == SS4D_ERR_TIMEOUT) {
+            set_err("the presmoothing's barrier gave up a wait");
+            return SS4D_ERR_TIMEOUT;
+        }
     return SS4D_OK;
 }
 
@@ -1209,45 +1247,19 @@ extern "C" ss4d_status ss4d_presmooth_step(ss4d_solver *s, const ss4d_params *p,
 {
     REQ(s && d_img, "NULL argument");
     CKS(check_params(p));
-    double *prev = d_scratch;
-    if (!prev) {
-        CKS(ensure_scratch(s));
-        prev = s->d_scratch;
-    }
-    if (s->arith == SS4D_ARITH_MIXED)
-        return presmooth_ff(s, p, d_img, prev, 0, stats);
-    const Geo &g = s->geo;
     CK(cudaEventRecord(s->ev0, s->stream));
-    CK(cudaMemcpyAsync(prev, d_img, sizeof(double) * g.n, cudaMemcpyDeviceToDevice, s->stream));
-    launch_reflect(g, d_img, s->stream);
-    s->launches += 4;
-    const double c = p->sigma / (p->h * p->h), h4 = p->h * p->h * p->h * p->h;
-    const long long nb = resid_blocks(g);
-    const double band = near_band(p->gsTol, g.nint);
-    double R = 0.0, R1 = 0.0;
-    int z = 0, near = 0;
-    do {
-        z = z + 1;
-        launch_presmooth_half(g, d_img, prev, c, p->omega_sigma, 0, s->stream);
-        launch_presmooth_half(g, d_img, prev, c, p->omega_sigma, 1, s->stream);
-        launch_presmooth_resid(g, d_img, prev, c, h4, s->d_partial, s->stream);
-        s->launches += 3 + launch_reduce_sum(s->d_partial, nb, s->d_scalar, s->stream);
-        CKS(last_launch());
-        CKS(read_scalar(s, 0, &R));
-        if (z == 1)
-            R1 = R;
-        near |= fabs(R - p->gsTol) <= band;
-    } while (R > p->gsTol && z < p->maxNoGSIteration_sigma);
+    CKS(presmooth_queue(s, p, d_img, d_scratch, nullptr, stats != nullptr, 0));
     CK(cudaEventRecord(s->ev1, s->stream));
-    CK(cudaEventSynchronize(s->ev1));
+    CKS(presmooth_wait(s, 1));
     if (stats) {
+        const FrontState &f = s->h_front[0];
         memset(stats, 0, sizeof *stats);
-        stats->iterations = z;
-        stats->residual = R;
-        stats->first_residual = R1;
-        stats->near_tolerance = near;
+        stats->iterations = f.z;
+        stats->residual = f.R;
+        stats->first_residual = f.R1;
+        stats->near_tolerance = f.near;
         cudaEventElapsedTime(&stats->ms, s->ev0, s->ev1);
-        stats->status = isfinite(R) ? SS4D_OK : SS4D_ERR_NONFINITE;
+        stats->status = f.status;
     }
     return SS4D_OK;
 }
@@ -1266,14 +1278,14 @@ extern "C" ss4d_status ss4d_presmooth_explicit(ss4d_solver *s, const ss4d_params
     const Geo &g = s->geo;
     CK(cudaMemcpyAsync(prev, d_img, sizeof(double) * g.n, cudaMemcpyDeviceToDevice, s->stream));
     launch_reflect(g, d_img, s->stream);
-    s->launches += 4;
+    s->launches += 1;
     // prev is not refreshed between the reference's steps, so every step after
     // the first recomputes the same values: one step is the result of any
     // number >= 1 (bit for bit)
     if (timeStepsNum > 0) {
         launch_presmooth_explicit(g, d_img, prev, p->sigma / (p->h * p->h), s->stream);
         launch_reflect(g, d_img, s->stream);
-        s->launches += 5;
+        s->launches += 2;
     }
     return last_launch();
 }
@@ -1324,7 +1336,7 @@ extern "C" ss4d_status ss4d_gaussian_smooth(ss4d_solver *s, const double sigma[4
     if (src != d_img)
         CK(cudaMemcpyAsync(d_img, src, sizeof(double) * g.n, cudaMemcpyDeviceToDevice, s->stream));
     launch_reflect(g, d_img, s->stream);
-    s->launches += 4;
+    s->launches += 1;
     return last_launch();
 }
 
@@ -1341,11 +1353,13 @@ extern "C" ss4d_status ss4d_gfaces(ss4d_solver *s, const ss4d_params *p, const d
     }
     const Geo &g = s->geo;
     if (s->arith == SS4D_ARITH_MIXED) {
-        CKS(ensure_ff_front(s));
-        launch_to_ff(g, d_i0, s->d_ff, s->stream);
-        if (d_i0_thr)
-            launch_to_ff(g, d_i0_thr, s->d_ff + g.n, s->stream);
-        launch_gfaces_ff(g, s->d_ff, d_i0_thr ? s->d_ff + g.n : nullptr, go, p->h, p->K, p->theta_img, p->rho_thr,
+        CKS(ensure_fold(s, 0));
+        launch_to_fold(g, d_i0, s->d_fold[0], p->h, s->stream);
+        if (d_i0_thr) {
+            CKS(ensure_fold(s, 1));
+            launch_to_fold(g, d_i0_thr, s->d_fold[1], p->h, s->stream);
+        }
+        launch_gfaces_ff(g, s->d_fold[0], d_i0_thr ? s->d_fold[1] : nullptr, go, p->h, p->K, p->theta_img, p->rho_thr,
                          s->stream);
         s->launches += d_i0_thr ? 3 : 2;
     } else {
@@ -1366,28 +1380,23 @@ extern "C" ss4d_status ss4d_edge_detector(ss4d_solver *s, const ss4d_params *p, 
         REQ(d_g[f], "a g array is NULL");
         go.p[f] = d_g[f];
     }
-    if (s->arith == SS4D_ARITH_MIXED) {
-        // float-float presmoothing of both images, g faces from the
-        // float-float results
-        double *prev = d_scratch;
-        if (!prev) {
-            CKS(ensure_scratch(s));
-            prev = s->d_scratch;
-        }
-        CKS(presmooth_ff(s, p, d_i0, prev, 0, nullptr));
+    const int mixed = s->arith == SS4D_ARITH_MIXED;
+    if (mixed) {
+        CKS(ensure_fold(s, 0));
         if (d_i0_thr)
-            CKS(presmooth_ff(s, p, d_i0_thr, prev, 1, nullptr));
-        launch_gfaces_ff(s->geo, s->d_ff, d_i0_thr ? s->d_ff + s->geo.n : nullptr, go, p->h, p->K, p->theta_img,
-                         p->rho_thr, s->stream);
-        s->launches += 1;
-        return last_launch();
+            CKS(ensure_fold(s, 1));
     }
-    CKS(ss4d_presmooth_step(s, p, d_i0, d_scratch, nullptr));
+    CKS(presmooth_queue(s, p, d_i0, d_scratch, mixed ? s->d_fold[0] : nullptr, 0, 0));
     if (d_i0_thr)
-        CKS(ss4d_presmooth_step(s, p, d_i0_thr, d_scratch, nullptr));
-    launch_gfaces(s->geo, d_i0, d_i0_thr, go, p->h, p->K, p->theta_img, p->rho_thr, s->stream);
+        CKS(presmooth_queue(s, p, d_i0_thr, d_scratch, mixed ? s->d_fold[1] : nullptr, 0, 1));
+    if (mixed)
+        launch_gfaces_ff(s->geo, s->d_fold[0], d_i0_thr ? s->d_fold[1] : nullptr, go, p->h, p->K, p->theta_img,
+                         p->rho_thr, s->stream);
+    else
+        launch_gfaces(s->geo, d_i0, d_i0_thr, go, p->h, p->K, p->theta_img, p->rho_thr, s->stream);
     s->launches += 1;
-    return last_launch();
+    CKS(last_launch());
+    return presmooth_wait(s, d_i0_thr ? 2 : 1);
 }
 
 extern "C" ss4d_status ss4d_gs_coefficients(ss4d_solver *s, const ss4d_params *p, const double *d_u,

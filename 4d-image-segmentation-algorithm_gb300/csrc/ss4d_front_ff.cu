@@ -2,16 +2,20 @@
 // arithmetic: the presmoothing's red-black SOR (segmentation4D.c:337-409) and
 // the 8 face g values (segmentation4D.c:594-821, _gFunction_ :67-70), with
 // about 48 significant bits on the FP32 pipe instead of FP64.  The plain and
-// reference forms keep the reference's FP64 rounding (ss4d_kernels_ref.cu);
-// on GB300 that work is bound by the FP64 pipe, this form by memory.
+// reference forms keep the reference's FP64 rounding (ss4d_front64.cu,
+// ss4d_kernels_ref.cu).
 //
-// The image and the presmoothing's copy of its input (the reference's
-// prev_u) are converted to float-float arrays (float2) once; the SOR
-// iterations read and write those; the interior is written back as doubles
-// at the end (h + l is exact in a double), the ghosts of the double image
-// keep the values the reflection gave them.  Relative error of the results
-// against the FP64 forms: about 1e-14 for the smoothed image, 1e-13 for g.
-#include "ss4d_ff.cuh"
+// Both work on two values per instruction (ss4d_ff2.cuh).  The presmoothing
+// (ss4d_front.cuh) pairs two adjacent columns of a colour.  The g faces read
+// the image folded in k: a 16-byte unit holds voxel k = m and voxel
+// k = m + Hk of the same (i, j, l), so every neighbour of both is in one
+// unit too, and addresses, loads and arithmetic serve two voxels; planes 0
+// and Hk + 1 of the fold are both halves' halo.  Relative error of the
+// results against the FP64 forms: about 1e-14.
+#include <math.h>
+
+#include "ss4d_ff2.cuh"
+#include "ss4d_front.cuh"
 
 namespace ss4d {
 
@@ -19,184 +23,337 @@ using namespace ffa;
 
 namespace {
 
-__device__ __forceinline__ ff ffc(FFc c)
+__device__ __forceinline__ ff split_d(double v)
 {
-    return ff_make(c.h, c.l);
+    const float h = (float)v;
+    return ff_make(h, (float)(v - (double)h));
 }
 
-// sum over a 2D block (flattened thread index); the result in thread (0, 0)
-__device__ double block_sum_flat(double v)
+__device__ __forceinline__ unsigned fold_index(const Geo &g, int Hk, int i, int j, int m, int l)
 {
-    __shared__ double part[32];
-    const int t = threadIdx.y * blockDim.x + threadIdx.x, lane = t & 31, wid = t >> 5;
-    const int nw = (blockDim.x * blockDim.y + 31) >> 5;
-    v = warp_sum(v);
-    if (lane == 0)
-        part[wid] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (wid == 0) {
-        r = lane < nw ? part[lane] : 0.0;
-        r = warp_sum(r);
+    return (((unsigned)l * (Hk + 2) + m) * g.jM + j) * g.iM + i;
+}
+
+struct PairFF {
+    typedef float4 Q;
+    // sum of squares per lane: its rounding errors are kept beside it
+    struct Acc {
+        f2 s, e;
+    };
+    struct Const {
+        ff2 c, inv_d, omega;
+    };
+    static __device__ __forceinline__ Const constants(const FrontArgs &a)
+    {
+        return Const{both(split_d(a.c)), both(split_d(a.y)), both(split_d(a.omega))};
     }
-    return r;
-}
-
-// the voxels of one colour, one per thread (every lane busy): thread x
-// indexes the pairs (i, i+1) of a row
-__device__ __forceinline__ bool colour_voxel(const Geo &g, int colour, int &i, int &j, int &k, int &l)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int kl = blockIdx.z;
-    k = 1 + kl % g.nz;
-    l = 1 + kl / g.nz;
-    i = 1 + 2 * t + ((colour + j + k + l + 1) & 1);
-    return i <= g.nx && j <= g.ny;
-}
-
-__device__ __forceinline__ ff sum8(const float2 *v, long long o, const Geo &g)
-{
-    ff s = ff_add(ld_ff2(v, o + 1), ld_ff2(v, o - 1));
-    s = ff_add(s, ld_ff2(v, o - g.sy));
-    s = ff_add(s, ld_ff2(v, o + g.sy));
-    s = ff_add(s, ld_ff2(v, o - g.sz));
-    s = ff_add(s, ld_ff2(v, o + g.sz));
-    s = ff_add(s, ld_ff2(v, o - g.sw));
-    return ff_add(s, ld_ff2(v, o + g.sw));
-}
-
-__global__ void k_to_ff(long long n, const double *__restrict__ a, float2 *__restrict__ out)
-{
-    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < n; o += (long long)gridDim.x * blockDim.x)
-        st_ff2(out, o, ff_from_d(a[o]));
-}
-
-__global__ void k_from_ff(Geo g, const float2 *__restrict__ v, double *__restrict__ out)
-{
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = 1 + blockIdx.z % g.nz, l = 1 + blockIdx.z / g.nz;
-    if (i > g.nx || j > g.ny)
-        return;
-    const long long o = nat_index(g, i, j, k, l);
-    out[o] = ff_to_d(ld_ff2(v, o));
-}
-
-// gs = (prev + c sum_8 v_nb) / (1 + 8c), v += omega (gs - v); inv_d = 1/(1 + 8c)
-__global__ void k_presmooth_half_ff(Geo g, float2 *v, const float2 *__restrict__ prev, FFc c, FFc inv_d, FFc omega,
-                                    int colour)
-{
-    int i, j, k, l;
-    if (!colour_voxel(g, colour, i, j, k, l))
-        return;
-    const long long o = nat_index(g, i, j, k, l);
-    const ff gs = ff_mul(ff_add(ld_ff2(prev, o), ff_mul(ffc(c), sum8(v, o, g))), ffc(inv_d));
-    const ff vo = ld_ff2(v, o);
-    st_ff2(v, o, ff_add(vo, ff_mul(ffc(omega), ff_add(gs, ff_neg(vo)))));
-}
-
-#define FRONT_RESID_K 4
-
-// r = v (1 + 8c) - c sum_8 v_nb - prev; a thread sums r^2 over FRONT_RESID_K
-// planes (FP32: the sum decides the stop test only), the block in FP64
-__global__ void k_presmooth_resid_ff(Geo g, const float2 *__restrict__ v, const float2 *__restrict__ prev, FFc c,
-                                     FFc d, double h4, double *partial)
-{
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int nkb = (g.nz + FRONT_RESID_K - 1) / FRONT_RESID_K;
-    const int k0 = 1 + (blockIdx.z % nkb) * FRONT_RESID_K, l = 1 + blockIdx.z / nkb;
-    float acc = 0.f;
-    if (i <= g.nx && j <= g.ny) {
-        for (int k = k0; k < k0 + FRONT_RESID_K && k <= g.nz; ++k) {
-            const long long o = nat_index(g, i, j, k, l);
-            const ff r = ff_add(ff_add(ff_mul(ld_ff2(v, o), ffc(d)), ff_neg(ff_mul(ffc(c), sum8(v, o, g)))),
-                                ff_neg(ld_ff2(prev, o)));
-            acc = fmaf(r.h, r.h, acc);
+    static __device__ __forceinline__ Acc zero()
+    {
+        return Acc{both(0.f), both(0.f)};
+    }
+    template <int COL>
+    static __device__ __forceinline__ double total(const FrontArgs &f, Acc a)
+    {
+        const double k = COL == 0 ? f.d : (1.0 - f.omega) * f.d;
+        return k * k * ( ((double)lo2(a.s) + (double)hi2(a.s)) + ((double)lo2(a.e) + (double)hi2(a.e)));
+    }
+    static __device__ __forceinline__ Q make(double x, double y)
+    {
+        const ff a = ff_from_d(x), b = ff_from_d(y);
+        return make_float4(a.h, b.h, a.l, b.l);
+    }
+    static __device__ __forceinline__ void get(Q v, double *w)
+    {
+        w[0] = ff_to_d(ff_make(v.x, v.z));
+        w[1] = ff_to_d(ff_make(v.y, v.w));
+    }
+    static __device__ __forceinline__ Q live(const Q *p)
+    {
+        Q v;
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+        return v;
+    }
+    static __device__ __forceinline__ ff first(const Q *p)
+    {
+        return ff_make(ld_oth<true>(&p->x), ld_oth<true>(&p->z));
+    }
+    static __device__ __forceinline__ ff second(const Q *p)
+    {
+        return ff_make(ld_oth<true>(&p->y), ld_oth<true>(&p->w));
+    }
+    static __device__ __forceinline__ Q up(Q v, ff e)
+    {
+        return make_float4(v.y, e.h, v.w, e.l);
+    }
+    static __device__ __forceinline__ Q down(ff e, Q v)
+    {
+        return make_float4(e.h, v.x, e.l, v.z);
+    }
+    static __device__ __forceinline__ Q with_first(Q v, Q w)
+    {
+        return make_float4(w.x, v.y, w.z, v.w);
+    }
+    static __device__ __forceinline__ Q with_second(Q v, Q w)
+    {
+        return make_float4(v.x, w.y, v.z, w.w);
+    }
+    // gs = (prev + c sum_8 v_nb) / (1 + 8c), v = u + omega (gs - u).  The
+    // residual u (1 + 8c) - c sum - prev is (1 + 8c) (u - gs), and after a
+    // target's own update (1 - omega) of that (its neighbours do not move):
+    // the squares of gs - u are summed and scaled once.  The neighbours are
+    // added in pairs without renormalising (positive terms): against 64 bits an
+    // update's error is 3.0e-15 where renormalising after every operation of
+    // the reference's order left 3.3e-15, with two thirds of the instructions.
+    template <int COL>
+    static __device__ __forceinline__ Q update(const Const &C, Q u4, Q pv4, Q xr, Q xl, Q ym, Q yp, Q zm, Q zp, Q wm,
+                                               Q wp, bool two, Acc &acc)
+    {
+        const ff2 x = ff_add_nr2(unpack4(xr), unpack4(xl)), y = ff_add_nr2(unpack4(ym), unpack4(yp));
+        const ff2 z = ff_add_nr2(unpack4(zm), unpack4(zp)), w = ff_add_nr2(unpack4(wm), unpack4(wp));
+        const ff2 s = ff_norm2(ff_add_nr2(ff_add_nr2(x, y), ff_add_nr2(z, w)));
+        const ff2 u = unpack4(u4);
+        const ff2 gs = ff_mul2(C.inv_d, ff_norm2(ff_add_nr2(unpack4(pv4), ff_mul_nr2(C.c, s))));
+        const ff2 r = ff_sub2(gs, u);
+        const ff2 v = ff_add2(u, ff_mul_nr2(C.omega, r));
+        f2 rh = r.h;
+        if (!two)
+            rh = mk2(lo2(rh), 0.f);
+        const ff2 q = two_sum2(acc.s, mul2(rh, rh));
+        acc.s = q.h;
+        acc.e = add2(acc.e, q.l);
+        return pack4(v);
+    }
+    // the smoothed image folded in k for the g faces: the result inside, the
+    // reflected initial image (at its clamped coordinates) on the ghosts
+    static __device__ __forceinline__ ff value(const FrontArgs &a, const Q *red, int i, int j, int k, int l)
+    {
+        const Geo &g = a.g;
+        const int ic = min(max(i, 1), g.nx), jc = min(max(j, 1), g.ny), kc = min(max(k, 1), g.nz),
+                  lc = min(max(l, 1), g.nt);
+        const int col = (ic + jc + kc + lc) & 1;
+        const bool in = ic == i && jc == j && kc == k && lc == l;
+        const float *v = static_cast<const float *>(in ? (col ? a.B : (const void *)red) : a.P[col]);
+        const unsigned s = (((unsigned)lc * g.kM + kc) * g.jM + jc) * a.F.Hs + ((ic + 1) >> 1) + a.F.A - 1;
+        const size_t e = 4 * (size_t)(s >> 1) + (s & 1);
+        return ff_make(ld_oth<true>(v + e), ld_oth<true>(v + e + 2));
+    }
+    static __device__ __forceinline__ void fold(const FrontArgs &a, const Q *red, unsigned t0, unsigned dt)
+    {
+        if (!a.fold)
+            return;
+        const Geo &g = a.g;
+        const unsigned planes = (unsigned)a.Hk + 2, rows = (unsigned)g.lM * planes * g.jM;
+        // a warp per row
+        for (unsigned r = t0 >> 5; r < rows; r += dt >> 5) {
+            const unsigned rk = fdiv(r, g.fjM), l = rk / planes;
+            const int j = (int)(r - rk * g.fjM.d), m = (int)(rk - l * planes);
+            for (int i = (int)(t0 & 31); i < g.iM; i += 32) {
+                const ff x = value(a, red, i, j, m, (int)l), y = value(a, red, i, j, m + a.Hk, (int)l);
+                const float S = a.fold_scale;
+                __stcs(static_cast<float4 *>(a.fold) + ((size_t)r * g.iM + i),
+                       make_float4(x.h * S, y.h * S, x.l * S, y.l * S));
+            }
         }
     }
-    const double tot = block_sum_flat((double)acc * h4);
-    if (threadIdx.x == 0 && threadIdx.y == 0)
-        partial[(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = tot;
-}
-
-// face_sq of the face between o and o + st[D] (the reference's face formula)
-template <int D>
-__device__ __forceinline__ ff face_sq_ff(const float2 *v, long long o, const long long st[4], ff ih, ff iq)
-{
-    const long long nb = o + st[D];
-    ff s = ff_make(0.f, 0.f);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        ff comp;
-        if (a == D) {
-            comp = ff_mul(ff_add(ld_ff2(v, nb), ff_neg(ld_ff2(v, o))), ih);
-        } else {
-            const ff plus = ff_add(ld_ff2(v, nb + st[a]), ld_ff2(v, o + st[a]));
-            const ff minus = ff_add(ld_ff2(v, nb - st[a]), ld_ff2(v, o - st[a]));
-            comp = ff_mul(ff_add(plus, ff_neg(minus)), iq);
-        }
-        s = ff_add_nr(s, ff_sqr(comp)); // positive terms
-    }
-    return ff_norm(s);
-}
-
-struct FaceConst {
-    FFc ih, iq, K, theta, rho;
 };
 
-// each face shared by two voxels once, as k_gfaces: the thread at o (every
-// coordinate 0..n) computes the + face along D when o's other coordinates
-// are interior and stores it as g[2D][o] and g[2D+1][o + st[D]]
+// 62 registers, two blocks of 512 per SM: at 256^2 x 128 x 20 an image takes
+// 12.4 ms (10 iterations at 1.1 ms, the copies 1.6), at three blocks of 256 14.0, at
+// four of them 12.8, at five (48 registers) 13.6.  A half-sweep moves 2.7 GB
+// (0.40 ms at the copy rate) and keeps the FP32 pipe half busy; the kernels it
+// replaces (one thread per target, a residual pass) took 28 ms per image.
+__global__ void __launch_bounds__(FRONT_FF_THREADS, 2) k_presmooth_ff(const __grid_constant__ FrontArgs a)
+{
+    presmooth_body<PairFF>(a);
+}
+
+// a double image, ghosts included, folded in k
+__global__ void k_to_fold(Geo g, int Hk, float S, const double *__restrict__ img, float4 *__restrict__ out)
+{
+    const unsigned planes = (unsigned)Hk + 2, rows = (unsigned)g.lM * planes * g.jM;
+    const int lane = threadIdx.x & 31;
+    for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += (gridDim.x * blockDim.x) >> 5) {
+        const unsigned rk = fdiv(r, g.fjM), l = rk / planes;
+        const int j = (int)(r - rk * g.fjM.d), m = (int)(rk - l * planes);
+        const double *a = img + nat_index(g, 0, j, min(m, g.kM - 1), (int)l);
+        const double *b = img + nat_index(g, 0, j, min(m + Hk, g.kM - 1), (int)l);
+        for (int i = lane; i < g.iM; i += 32) {
+            const ff x = ff_from_d(__ldg(a + i)), y = ff_from_d(__ldg(b + i));
+            out[(size_t)r * g.iM + i] = make_float4(x.h * S, y.h * S, x.l * S, y.l * S);
+        }
+    }
+}
+
+// --- g faces ----------------------------------------------------------------
+
+struct FaceConst {
+    FFc n[2], t[2]; // per image: K weight / (h S)^2 (normal) and K weight / (4 h S)^2 (tangential)
+};
+
+__device__ __forceinline__ ff2 ldv(const float4 *__restrict__ v, unsigned x)
+{
+    return unpack4(__ldg(v + x));
+}
+// central difference along a stride
+__device__ __forceinline__ ff2 cdiff2(const float4 *__restrict__ v, unsigned x, unsigned sa)
+{
+    return ff_sub_nr2(ldv(v, x + sa), ldv(v, x - sa));
+}
+__device__ __forceinline__ ff2 konst(FFc c)
+{
+    return both(ff_make(c.h, c.l));
+}
+
+// K weight |grad v|^2 at the face between x and x + st[D] from the central
+// differences own[] at x: the reference's face formula with its tangential
+// pairs exchanged, (v[nb+a] + v[o+a]) - (v[nb-a] + v[o-a]) = D_a(nb) + D_a(o),
+// so that D_a(o) serves three faces
 template <int D>
-__device__ __forceinline__ void gface_plus_ff(const int c[4], const int n[4], long long o, const long long st[4],
-                                              const float2 *i0, const float2 *ithr, GPtrs8 &gout, const FaceConst &F)
+__device__ __forceinline__ ff2 face_term(const float4 *__restrict__ v, unsigned x, const unsigned st[4],
+                                         const ff2 own[4], ff2 vx, ff2 kn, ff2 kt)
 {
+    const unsigned nb = x + st[D];
+    ff2 tt;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-        if (a != D && c[a] < 1)
-            return;
-    const ff ih = ffc(F.ih), iq = ffc(F.iq);
-    ff s = ff_mul(ffc(F.theta), face_sq_ff<D>(i0, o, st, ih, iq));
-    if (ithr)
-        s = ff_add(s, ff_mul(ffc(F.rho), face_sq_ff<D>(ithr, o, st, ih, iq)));
-    const double gv = ff_to_d(ff_rcp(ff_add(ff_make(1.f, 0.f), ff_mul(ffc(F.K), s))));
-    if (c[D] >= 1)
-        gout.p[2 * D][o] = gv;
-    if (c[D] < n[D])
-        gout.p[2 * D + 1][o + st[D]] = gv;
+    for (int a = 0; a < 4; ++a) {
+        if (a == D)
+            continue;
+        const ff2 q = ff_sqr_nr2(ff_add_nr2(cdiff2(v, nb, st[a]), own[a]));
+        tt = a == (D == 0 ? 1 : 0) ? q : ff_add_nr2(tt, q);
+    }
+    const ff2 nn = ff_sqr_nr2(ff_sub_nr2(ldv(v, nb), vx));
+    return ff_add_nr2(ff_mul_nr2(kt, tt), ff_mul_nr2(kn, nn));
 }
 
-// 6 blocks per SM (40 registers) rather than 4 (56): the mixed edge
-// detector at 256^2 x 128 x 20 went from 71.5 to 70.6 ms (8 blocks spilled
-// and gained less)
-__global__ void __launch_bounds__(256, 6) k_gfaces_ff(Geo g, const float2 *__restrict__ i0, const float2 *__restrict__ ithr, GPtrs8 gout,
-                            FaceConst F)
+// g = 1/(1 + s): FP32 seeds, one Newton step (ff_rcp)
+__device__ __forceinline__ void g_of(ff2 s, double out[2])
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int kl = blockIdx.z;
-    const int k = kl % (g.nz + 1), l = kl / (g.nz + 1);
-    if (i > g.nx || j > g.ny)
+    const ff2 x = ff_add2(both(ff_make(1.f, 0.f)), ff_norm2(s));
+    const f2 y0 = mk2(__frcp_rn(lo2(x.h)), __frcp_rn(hi2(x.h)));
+    const f2 q = mul2(x.h, y0);
+    const f2 qe = fma2(x.l, y0, fma2(x.h, y0, neg2(q)));
+    const f2 r = sub2(sub2(both(1.f), q), qe);
+    const f2 c = mul2(y0, r), ce = fma2(y0, r, neg2(c));
+    ff2 y = fast_two_sum2(y0, c);
+    y.l = add2(y.l, ce);
+    out[0] = ff_to_d(ff_make(lo2(y.h), lo2(y.l)));
+    out[1] = ff_to_d(ff_make(hi2(y.h), hi2(y.l)));
+}
+
+// Face between o (coordinate cD along D) and o + st[D]: g[2D] at o where o
+// is interior along D, g[2D+1] at o + st[D] where that is.
+__device__ __forceinline__ void put_face(double *__restrict__ lo, double *__restrict__ hi, size_t o, size_t sd, int cD,
+                                         int nD, double gv)
+{
+    if (cD >= 1)
+        __stcs(lo + o, gv);
+    if (cD < nD)
+        __stcs(hi + o + sd, gv);
+}
+
+template <int D, bool TWO>
+__device__ __forceinline__ void boundary_gface(const float4 *__restrict__ v0, const float4 *__restrict__ v1, unsigned x,
+                                               const unsigned st[4], const FaceConst &F, double out[2])
+{
+    ff2 s;
+#pragma unroll
+    for (int im = 0; im < (TWO ? 2 : 1); ++im) {
+        const float4 *__restrict__ v = im ? v1 : v0;
+        ff2 own[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+            own[a] = a == D ? ff2{both(0.f), both(0.f)} : cdiff2(v, x, st[a]);
+        const ff2 t = face_term<D>(v, x, st, own, ldv(v, x), konst(F.n[im]), konst(F.t[im]));
+        s = im ? ff_add_nr2(s, t) : t;
+    }
+    g_of(s, out);
+}
+
+// One folded voxel per thread (voxels (i, j, m, l) and (i, j, m + Hk, l)):
+// the faces towards +x, +y, +z, +t of both, and at the volume's lower
+// boundaries also the face towards the ghost.  The flat index has i fastest,
+// m slowest: blocks at work together cover a few planes of all frames, whose
+// neighbouring frames and planes are then read from L2.
+// Bound by issue and the FP32 pipe (about 950 instructions per voxel with two
+// images).  At 256^2 x 128 x 20: two images 9.5 ms at five blocks of 128
+// threads (96 registers), 10.4 at 128 registers, 11.0 at 80; one image 5.1 ms at
+// 80 registers, 5.5 at 96.  The kernel it replaces (scalar float-float, every
+// difference formed at each of its faces) took 14.5 ms for two.
+constexpr int GFACES_THREADS = 128;
+template <bool TWO>
+__global__ void __launch_bounds__(GFACES_THREADS, TWO ? 5 : 6)
+    k_gfaces_ff(Geo g, int Hk, FastDiv dnx, FastDiv dny, FastDiv dnt, unsigned n, const float4 *__restrict__ v0,
+                const float4 *__restrict__ v1, GPtrs8 gout, const __grid_constant__ FaceConst F)
+{
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n)
         return;
-    const int c[4] = {i, j, k, l};
-    const int n[4] = {g.nx, g.ny, g.nz, g.nt};
-    const long long o = nat_index(g, i, j, k, l);
-    const long long st[4] = {1, g.sy, g.sz, g.sw};
-    gface_plus_ff<0>(c, n, o, st, i0, ithr, gout, F);
-    gface_plus_ff<1>(c, n, o, st, i0, ithr, gout, F);
-    gface_plus_ff<2>(c, n, o, st, i0, ithr, gout, F);
-    gface_plus_ff<3>(c, n, o, st, i0, ithr, gout, F);
+    unsigned h = fdiv(q, dnx);
+    const int i = 1 + (int)(q - h * dnx.d);
+    unsigned r = h;
+    h = fdiv(r, dny);
+    const int j = 1 + (int)(r - h * dny.d);
+    r = h;
+    h = fdiv(r, dnt);
+    const int l = 1 + (int)(r - h * dnt.d);
+    const int m = 1 + (int)h;
+    const unsigned st[4] = {1u, (unsigned)g.iM, (unsigned)(g.iM * g.jM), (unsigned)(g.iM * g.jM) * (Hk + 2)};
+    const unsigned x = fold_index(g, Hk, i, j, m, l);
+    ff2 s[4];
+#pragma unroll
+    for (int im = 0; im < (TWO ? 2 : 1); ++im) {
+        const float4 *__restrict__ v = im ? v1 : v0;
+        const ff2 kn = konst(F.n[im]), kt = konst(F.t[im]);
+        ff2 own[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+            own[a] = cdiff2(v, x, st[a]);
+        const ff2 vx = ldv(v, x);
+        ff2 t = face_term<0>(v, x, st, own, vx, kn, kt);
+        s[0] = im ? ff_add_nr2(s[0], t) : t;
+        t = face_term<1>(v, x, st, own, vx, kn, kt);
+        s[1] = im ? ff_add_nr2(s[1], t) : t;
+        t = face_term<2>(v, x, st, own, vx, kn, kt);
+        s[2] = im ? ff_add_nr2(s[2], t) : t;
+        t = face_term<3>(v, x, st, own, vx, kn, kt);
+        s[3] = im ? ff_add_nr2(s[3], t) : t;
+    }
+    const bool b1 = m + Hk <= g.nz; // the second voxel exists
+    const size_t oa = (size_t)nat_index(g, i, j, m, l), ob = oa + (size_t)Hk * g.sz;
+    const int c[4] = {i, j, m, l}, nn[4] = {g.nx, g.ny, g.nz, g.nt};
+    const size_t sd[4] = {1, (size_t)g.sy, (size_t)g.sz, (size_t)g.sw};
+    double gv[2];
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        g_of(s[d], gv);
+        put_face(gout.p[2 * d], gout.p[2 * d + 1], oa, sd[d], c[d], nn[d], gv[0]);
+        if (b1)
+            put_face(gout.p[2 * d], gout.p[2 * d + 1], ob, sd[d], d == 2 ? m + Hk : c[d], nn[d], gv[1]);
+    }
+    // the faces between a ghost and the first voxel along an axis
+    if (i == 1) {
+        boundary_gface<0, TWO>(v0, v1, x - st[0], st, F, gv);
+        __stcs(gout.p[1] + oa, gv[0]);
+        if (b1)
+            __stcs(gout.p[1] + ob, gv[1]);
+    }
+    if (j == 1) {
+        boundary_gface<1, TWO>(v0, v1, x - st[1], st, F, gv);
+        __stcs(gout.p[3] + oa, gv[0]);
+        if (b1)
+            __stcs(gout.p[3] + ob, gv[1]);
+    }
+    if (m == 1) { // k = 0 | 1; the second half's lower face is the first half's upper one
+        boundary_gface<2, TWO>(v0, v1, x - st[2], st, F, gv);
+        __stcs(gout.p[5] + oa, gv[0]);
+    }
+    if (l == 1) {
+        boundary_gface<3, TWO>(v0, v1, x - st[3], st, F, gv);
+        __stcs(gout.p[7] + oa, gv[0]);
+        if (b1)
+            __stcs(gout.p[7] + ob, gv[1]);
+    }
 }
-
-dim3 row_block(int nx)
-{
-    const int bx = nx >= 128 ? 128 : (nx >= 64 ? 64 : 32);
-    return dim3(bx, 256 / bx, 1);
-}
-
-} // namespace
 
 FFc split_ff(double v)
 {
@@ -206,55 +363,65 @@ FFc split_ff(double v)
     return c;
 }
 
-void launch_to_ff(const Geo &g, const double *a, float2 *out, cudaStream_t st)
+} // namespace
+
+int fold_of(const Geo &g)
 {
-    k_to_ff<<<2048, 256, 0, st>>>(g.n, a, out);
+    return (g.nz + 1) / 2;
 }
 
-void launch_from_ff(const Geo &g, const float2 *v, double *out, cudaStream_t st)
+size_t fold_units(const Geo &g)
 {
-    const dim3 bl = row_block(g.nx);
-    k_from_ff<<<dim3((g.nx + bl.x - 1) / bl.x, (g.ny + bl.y - 1) / bl.y, g.nz * g.nt), bl, 0, st>>>(g, v, out);
+    return (size_t)g.lM * (fold_of(g) + 2) * g.jM * g.iM;
 }
 
-void launch_presmooth_half_ff(const Geo &g, float2 *v, const float2 *prev, double c, double omega, int colour,
-                              cudaStream_t st)
+int presmooth_ff_grid(int sm_count)
 {
-    const int nxh = (g.nx + 1) / 2;
-    const dim3 bl = row_block(nxh);
-    const dim3 gr((nxh + bl.x - 1) / bl.x, (g.ny + bl.y - 1) / bl.y, g.nz * g.nt);
-    k_presmooth_half_ff<<<gr, bl, 0, st>>>(g, v, prev, split_ff(c), split_ff(1.0 / (1 + c * 8)), split_ff(omega),
-                                           colour);
+    int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_presmooth_ff, FRONT_FF_THREADS, 0);
+    return per * sm_count;
 }
 
-long long front_resid_blocks(const Geo &g)
+cudaError_t launch_presmooth_ff(const FrontArgs &a, int grid, cudaStream_t st)
 {
-    const dim3 bl = row_block(g.nx);
-    return (long long)((g.nx + bl.x - 1) / bl.x) * ((g.ny + bl.y - 1) / bl.y) *
-           ((g.nz + FRONT_RESID_K - 1) / FRONT_RESID_K) * g.nt;
+    void *args[] = {(void *)&a};
+    return cudaLaunchCooperativeKernel((const void *)k_presmooth_ff, dim3(grid), dim3(FRONT_FF_THREADS), args, 0, st);
 }
 
-void launch_presmooth_resid_ff(const Geo &g, const float2 *v, const float2 *prev, double c, double h4,
-                               double *partial, cudaStream_t st)
+// The folded image is scaled by the power of two nearest above 1/h, exactly,
+// so that its differences are of the gradient's size whatever h is: their
+// squares then stay in FP32's range as long as the gradient's do.
+float fold_scale(double h)
 {
-    const dim3 bl = row_block(g.nx);
-    const dim3 gr((g.nx + bl.x - 1) / bl.x, (g.ny + bl.y - 1) / bl.y,
-                  ((g.nz + FRONT_RESID_K - 1) / FRONT_RESID_K) * g.nt);
-    k_presmooth_resid_ff<<<gr, bl, 0, st>>>(g, v, prev, split_ff(c), split_ff(1 + c * 8), h4, partial);
+    int e = 0;
+    frexp(h, &e);
+    e = e < -100 ? -100 : (e > 100 ? 100 : e);
+    return (float)ldexp(1.0, 1 - e);
 }
 
-void launch_gfaces_ff(const Geo &g, const float2 *i0, const float2 *ithr, GPtrs8 gout, double h, double K,
+void launch_to_fold(const Geo &g, const double *img, float4 *out, double h, cudaStream_t st)
+{
+    k_to_fold<<<2432, 256, 0, st>>>(g, fold_of(g), fold_scale(h), img, out);
+}
+
+void launch_gfaces_ff(const Geo &g, const float4 *i0, const float4 *ithr, GPtrs8 gout, double h, double K,
                       double theta, double rho, cudaStream_t st)
 {
-    const dim3 bl = row_block(g.nx + 1);
-    const dim3 gr((g.nx + 1 + bl.x - 1) / bl.x, (g.ny + 1 + bl.y - 1) / bl.y, (g.nz + 1) * (g.nt + 1));
+    const int Hk = fold_of(g);
     FaceConst F;
-    F.ih = split_ff(1.0 / h);
-    F.iq = split_ff(1.0 / (4.0 * h));
-    F.K = split_ff(K);
-    F.theta = split_ff(theta);
-    F.rho = split_ff(rho);
-    k_gfaces_ff<<<gr, bl, 0, st>>>(g, i0, ithr, gout, F);
+    const double w[2] = {theta, rho};
+    const double hs = h * fold_scale(h), hs2 = hs * hs;
+    for (int im = 0; im < 2; ++im) {
+        F.n[im] = split_ff(K * w[im] / hs2);
+        F.t[im] = split_ff(K * w[im] / (16.0 * hs2));
+    }
+    const unsigned n = (unsigned)g.nx * g.ny * g.nt * Hk;
+    const unsigned nb = (n + GFACES_THREADS - 1) / GFACES_THREADS;
+    const FastDiv dx = make_fastdiv((unsigned)g.nx), dy = make_fastdiv((unsigned)g.ny), dt = make_fastdiv((unsigned)g.nt);
+    if (ithr)
+        k_gfaces_ff<true><<<nb, GFACES_THREADS, 0, st>>>(g, Hk, dx, dy, dt, n, i0, ithr, gout, F);
+    else
+        k_gfaces_ff<false><<<nb, GFACES_THREADS, 0, st>>>(g, Hk, dx, dy, dt, n, i0, i0, gout, F);
 }
 
 } // namespace ss4d

@@ -17,8 +17,6 @@ struct CPtrs8 {
 long long interior_blocks(const Geo &g);
 long long resid_blocks(const Geo &g); // partials of the residual passes
 void launch_reflect(const Geo &g, double *u, cudaStream_t st);
-void launch_presmooth_half(const Geo &g, double *v, const double *prev, double c, double omega, int colour,
-                           cudaStream_t st);
 void launch_presmooth_explicit(const Geo &g, double *v, const double *prev, double coeff, cudaStream_t st);
 // normalised Gaussian taps w[0..R] of one axis (ss4d_gaussian_smooth)
 struct GaussWeights {
@@ -27,8 +25,6 @@ struct GaussWeights {
 };
 void launch_gauss_axis(const Geo &g, int axis, const double *in, double *out, const GaussWeights &W,
                        cudaStream_t st);
-void launch_presmooth_resid(const Geo &g, const double *v, const double *prev, double c, double h4, double *partial,
-                            cudaStream_t st);
 void launch_gfaces(const Geo &g, const double *i0, const double *ithr, GPtrs8 gout, double h, double K, double theta,
                    double rho, cudaStream_t st);
 void launch_coef_ref(const Geo &g, const double *u, CPtrs8 gin, int has_g, GPtrs8 coef, double h, double eps2,
@@ -200,20 +196,16 @@ void launch_rescale_balls_range(const Geo &g, double *v, const int *frame_first,
                                 const double *bx, const double *by, const double *bz, double R, int l0, int l1,
                                 cudaStream_t st);
 
-// the mixed form's edge detector in float-float arithmetic (ss4d_front_ff.cu);
-// float2 arrays hold (high, low) pairs in the natural layout
+// the mixed form's edge detector in float-float arithmetic (ss4d_front_ff.cu):
+// images folded in k, fold_units() 16-byte units each
 struct FFc {
     float h, l; // a constant split on the host
 };
-FFc split_ff(double v);
-void launch_to_ff(const Geo &g, const double *a, float2 *out, cudaStream_t st);
-void launch_from_ff(const Geo &g, const float2 *v, double *out, cudaStream_t st); // interior only
-void launch_presmooth_half_ff(const Geo &g, float2 *v, const float2 *prev, double c, double omega, int colour,
-                              cudaStream_t st);
-long long front_resid_blocks(const Geo &g); // partials of launch_presmooth_resid_ff
-void launch_presmooth_resid_ff(const Geo &g, const float2 *v, const float2 *prev, double c, double h4,
-                               double *partial, cudaStream_t st);
-void launch_gfaces_ff(const Geo &g, const float2 *i0, const float2 *ithr, GPtrs8 gout, double h, double K,
+int fold_of(const Geo &g);
+size_t fold_units(const Geo &g);
+float fold_scale(double h);
+void launch_to_fold(const Geo &g, const double *img, float4 *out, double h, cudaStream_t st);
+void launch_gfaces_ff(const Geo &g, const float4 *i0, const float4 *ithr, GPtrs8 gout, double h, double K,
                       double theta, double rho, cudaStream_t st);
 void launch_pack_coef(const Geo &g, const Split &s, CPtrs8 a, const ss4d_params &p, SplitBufs b, int want32,
                       cudaStream_t st);

@@ -9,6 +9,7 @@
 // serial sum).  They serve the SS4D_ARITH_REFERENCE form, the edge detector of
 // every form (run once per segmentation), the MCF boundary and exact
 // solution, the rescale, the mask and the norms.
+#include "ss4d_exact.cuh"
 #include "ss4d_kernels.cuh"
 
 namespace ss4d {
@@ -73,85 +74,32 @@ __device__ inline double block_sum2d(double v)
 }
 
 // ---------------------------------------------------------------------------
-// Neumann reflection, one axis per launch (segmentation4D.c:826-864 runs the
-// axes in x, y, z, w order over full padded ranges).
+// Neumann reflection (segmentation4D.c:826-864) in one launch: the
+// reference's copies, axis by axis over full padded ranges, leave every ghost
+// (edges and corners included) with the value of the nearest interior voxel,
+// so a ghost reads it at its clamped coordinates.  A warp per padded row.
 
-__global__ void k_reflect_axis(Geo g, double *u, int axis)
+__global__ void k_reflect(Geo g, double *u)
 {
-    // enumerate the padded cross-section orthogonal to `axis`
-    long long cnt;
-    int e[3];
-    long long st[3], sa;
-    int Ma;
-    if (axis == 0) { e[0] = g.jM; e[1] = g.kM; e[2] = g.lM; st[0] = g.sy; st[1] = g.sz; st[2] = g.sw; sa = 1; Ma = g.iM; }
-    else if (axis == 1) { e[0] = g.iM; e[1] = g.kM; e[2] = g.lM; st[0] = 1; st[1] = g.sz; st[2] = g.sw; sa = g.sy; Ma = g.jM; }
-    else if (axis == 2) { e[0] = g.iM; e[1] = g.jM; e[2] = g.lM; st[0] = 1; st[1] = g.sy; st[2] = g.sw; sa = g.sz; Ma = g.kM; }
-    else { e[0] = g.iM; e[1] = g.jM; e[2] = g.kM; st[0] = 1; st[1] = g.sy; st[2] = g.sz; sa = g.sw; Ma = g.lM; }
-    cnt = (long long)e[0] * e[1] * e[2];
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cnt; t += (long long)gridDim.x * blockDim.x) {
-        long long r = t;
-        int a0 = (int)(r % e[0]); r /= e[0];
-        int a1 = (int)(r % e[1]);
-        int a2 = (int)(r / e[1]);
-        long long base = a0 * st[0] + a1 * st[1] + a2 * st[2];
-        u[base] = u[base + sa];
-        u[base + (Ma - 1) * sa] = u[base + (Ma - 2) * sa];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// x / d, rounded to nearest, for a divisor d > 0 known in advance with
-// y = 1/d rounded to nearest (y == 0: no fast path).  A quotient from the
-// reciprocal and one remainder correction (Markstein's iteration), then an
-// exact acceptance test: the remainder x - q d (one FMA, correctly rounded) must
-// be below d times half the spacing from q to its nearer neighbour; since
-// that bound is a power-of-two multiple of d, hence exact, and rounding is
-// monotonic, passing it proves q is the double nearest to x / d.  Otherwise
-// (near a tie, zero, q outside [2^-400, 2^601)) the IEEE division decides.
-__device__ inline double div_by_const(double x, double d, double y)
-{
-    if (y != 0.0) {
-        const double q0 = x * y;
-        const double q = fma(fma(-q0, d, x), y, q0);
-        const long long b = __double_as_longlong(q);
-        const int E = (int)((b >> 52) & 0x7ff) - 1023;
-        if (E >= -400 && E <= 600) {
-            const int e = E - 53 - ((b & 0xfffffffffffffLL) == 0 ? 1 : 0); // half spacing 2^e
-            // d 2^e (a normal number: d in [2^-300, 2^300]) by adding e to d's
-            // exponent, and |r| < d 2^e compared as the bit patterns of two
-            // non-negative doubles: integer work only
-            const long long lim = __double_as_longlong(d) + ((long long)e << 52);
-            if ((__double_as_longlong(fma(-q, d, x)) & 0x7fffffffffffffffLL) < lim)
-                return q;
+    const unsigned rows = (unsigned)(g.jM * g.kM * g.lM), step = (gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += step) {
+        const unsigned rk = fdiv(r, g.fjM), l = fdiv(rk, g.fkM);
+        const int j = (int)(r - rk * g.fjM.d), k = (int)(rk - l * g.fkM.d);
+        const int jc = min(max(j, 1), g.ny), kc = min(max(k, 1), g.nz), lc = min(max((int)l, 1), g.nt);
+        double *row = u + (size_t)r * g.iM;
+        if (jc == j && kc == k && lc == (int)l) {
+            if (lane < 2)
+                row[lane ? g.iM - 1 : 0] = row[lane ? g.nx : 1];
+        } else {
+            const double *src = u + nat_index(g, 0, jc, kc, lc);
+            for (int i = lane; i < g.iM; i += 32)
+                row[i] = src[min(max(i, 1), g.nx)];
         }
     }
-    return x / d;
-}
-
-// reciprocal for div_by_const, or 0 where the divisor is outside the range
-// its test needs (d in [2^-300, 2^300])
-static inline double div_const_recip(double d)
-{
-    return (d >= 0x1p-300 && d <= 0x1p300) ? 1.0 / d : 0.0;
 }
 
 // ---------------------------------------------------------------------------
-// presmoothing (segmentation4D.c:352-404); d = 1 + 8c (the same rounding on
-// the host), y its reciprocal for div_by_const
-
-__global__ void k_presmooth_half(Geo g, double *v, const double *prev, double c, double d, double y, double omega,
-                                 int colour)
-{
-    int i, j, k, l;
-    if (!colour_ijkl(g, colour, i, j, k, l))
-        return;
-    const long long o = nat_index(g, i, j, k, l);
-    double gs = div_by_const(prev[o] + c * (v[o + 1] + v[o - 1] + v[o - g.sy] + v[o + g.sy] + v[o - g.sz]
-                                            + v[o + g.sz] + v[o - g.sw] + v[o + g.sw]),
-                             d, y);
-    v[o] = v[o] + omega * (gs - v[o]);
-}
-
 // residual passes: a thread sums RESID_K k-planes before the block reduction
 #define RESID_K 4
 
@@ -163,26 +111,6 @@ __device__ inline bool resid_ijl(const Geo &g, int &i, int &j, int &k0, int &l)
     k0 = 1 + (blockIdx.z % nkb) * RESID_K;
     l = 1 + blockIdx.z / nkb;
     return i <= g.nx && j <= g.ny;
-}
-
-__global__ void k_presmooth_resid(Geo g, const double *v, const double *prev, double c, double d, double h4,
-                                  double *partial)
-{
-    int i, j, k0, l;
-    double acc = 0.0;
-    if (resid_ijl(g, i, j, k0, l)) {
-        for (int k = k0; k < k0 + RESID_K && k <= g.nz; ++k) {
-            const long long o = nat_index(g, i, j, k, l);
-            double r = v[o] * d
-                       - c * (v[o + 1] + v[o - 1] + v[o - g.sy] + v[o + g.sy] + v[o - g.sz] + v[o + g.sz]
-                              + v[o - g.sw] + v[o + g.sw])
-                       - prev[o];
-            acc += (r * r) * h4;
-        }
-    }
-    acc = block_sum2d(acc);
-    if (flat_tid() == 0)
-        partial[block_linear()] = acc;
 }
 
 // explicit smoother (segmentation4D.c:422-441): one Jacobi-style step from
@@ -815,8 +743,8 @@ long long interior_blocks(const Geo &g)
 
 void launch_reflect(const Geo &g, double *u, cudaStream_t st)
 {
-    for (int a = 0; a < 4; ++a)
-        k_reflect_axis<<<256, 256, 0, st>>>(g, u, a);
+    const long long warps = (long long)g.jM * g.kM * g.lM;
+    k_reflect<<<(unsigned)(warps < 8 * 1216 ? (warps + 7) / 8 : 1216), 256, 0, st>>>(g, u);
 }
 
 // one colour: ceil(nx/2) threads along a row
@@ -827,15 +755,6 @@ static inline void colour_cfg(const Geo &g, dim3 &grid, dim3 &block)
     const int by = 256 / bx;
     block = dim3(bx, by, 1);
     grid = dim3((nxh + bx - 1) / bx, (g.ny + by - 1) / by, g.nz * g.nt);
-}
-
-void launch_presmooth_half(const Geo &g, double *v, const double *prev, double c, double omega, int colour,
-                           cudaStream_t st)
-{
-    dim3 gr, bl;
-    colour_cfg(g, gr, bl);
-    const double d = 1 + c * 8;
-    k_presmooth_half<<<gr, bl, 0, st>>>(g, v, prev, c, d, div_const_recip(d), omega, colour);
 }
 
 static inline void resid_cfg(const Geo &g, dim3 &grid, dim3 &block)
@@ -849,14 +768,6 @@ long long resid_blocks(const Geo &g)
     dim3 gr, bl;
     resid_cfg(g, gr, bl);
     return (long long)gr.x * gr.y * gr.z;
-}
-
-void launch_presmooth_resid(const Geo &g, const double *v, const double *prev, double c, double h4, double *partial,
-                            cudaStream_t st)
-{
-    dim3 gr, bl;
-    resid_cfg(g, gr, bl);
-    k_presmooth_resid<<<gr, bl, 0, st>>>(g, v, prev, c, 1 + c * 8, h4, partial);
 }
 
 void launch_gauss_axis(const Geo &g, int axis, const double *in, double *out, const GaussWeights &W,

@@ -25,36 +25,6 @@ namespace {
 
 constexpr int LOOP_MAX_THREADS = 512;
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Barrier of a group, thread 0 of each block, between two block barriers:
-// arrive once the block's writes are made, then wait until `target` arrivals
-// were.  The release and the acquire order the blocks' writes and reads (the
-// block barriers carry the order to their other threads).  A wait is bounded
-// (about a second); one that runs out marks the group.
-__device__ __forceinline__ void group_arrive(LoopGroup *gr)
-{
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gr->count) : "memory");
-}
-__device__ __forceinline__ bool group_wait(LoopGroup *gr, unsigned target)
-{
-    if ((int)(ld_acquire(&gr->count) - target) < 0) {
-        const long long t0 = clock64();
-        while ((int)(ld_acquire(&gr->count) - target) < 0) {
-            if (clock64() - t0 > (1LL << 31)) {
-                atomicExch(&gr->err, 1);
-                return false;
-            }
-        }
-    }
-    return *(volatile int *)&gr->err == 0;
-}
-
 template <int COL>
 __device__ __forceinline__ double phase_sweep64(const LoopVol &V, int z, unsigned q0, unsigned dq)
 {

@@ -1,5 +1,6 @@
 // ss4d_loop.cuh — the persistent SOR loop (ss4d_loop.cu), used by the
-// single-volume handle and the batch.
+// single-volume handle and the batch, and the group barrier it shares with
+// the persistent presmoothing (ss4d_front.cuh).
 #pragma once
 
 #include <string.h>
@@ -21,6 +22,36 @@ struct LoopGroup {
     int err;
     int pad_[30]; // one 128-byte line per group
 };
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Barrier of a group, thread 0 of each block, between two block barriers:
+// arrive once the block's writes are made, then wait until `target` arrivals
+// were.  The release and the acquire order the blocks' writes and reads (the
+// block barriers carry the order to their other threads).  A wait is bounded
+// (about a second); one that runs out marks the group.
+__device__ __forceinline__ void group_arrive(LoopGroup *gr)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gr->count) : "memory");
+}
+__device__ __forceinline__ bool group_wait(LoopGroup *gr, unsigned target)
+{
+    if ((int)(ld_acquire(&gr->count) - target) < 0) {
+        const long long t0 = clock64();
+        while ((int)(ld_acquire(&gr->count) - target) < 0) {
+            if (clock64() - t0 > (1LL << 31)) {
+                atomicExch(&gr->err, 1);
+                return false;
+            }
+        }
+    }
+    return *(volatile int *)&gr->err == 0;
+}
 
 LoopVol make_loop_vol(const Geo &g, const Split &sp, const SplitBufs &b);
 // co-resident blocks of k_loop with that many threads on the device (0: unknown)

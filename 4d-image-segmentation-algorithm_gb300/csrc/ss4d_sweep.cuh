@@ -184,22 +184,29 @@ struct Place {
 
 // the target at (or the pair's first target at) flat index q of colour col
 template <int W>
-__device__ __forceinline__ Place place(const FlatIndex &F, const FastDiv &dx, int col, unsigned q)
+__device__ __forceinline__ Place place(const FlatIndex &F, const FastDiv &dx, int col, unsigned q, int &j, int &k,
+                                       int &l)
 {
     unsigned r = fdiv(q, dx);
     const unsigned x = W * (q - r * dx.d);
     unsigned h = fdiv(r, F.dJ);
-    const unsigned j = 1 + (r - h * F.dJ.d);
+    j = (int)(1 + (r - h * F.dJ.d));
     r = h;
     h = fdiv(r, F.dL);
-    const unsigned l = 1 + (r - h * F.dL.d);
-    const unsigned k = 1 + h;
+    l = (int)(1 + (r - h * F.dL.d));
+    k = (int)(1 + h);
     Place a;
     a.p = (col + j + k + l) & 1;
     a.i = 2 * (int)x + 2 - a.p;
-    a.s = ((l * F.kM + k) * F.jM + j) * F.Hs + x + F.A;
-    a.t = (((l - 1) * F.nz + (k - 1)) * F.ny + (j - 1)) * F.nxh + x;
+    a.s = (((unsigned)l * F.kM + k) * F.jM + j) * F.Hs + x + F.A;
+    a.t = ((((unsigned)l - 1) * F.nz + (k - 1)) * F.ny + (j - 1)) * F.nxh + x;
     return a;
+}
+template <int W>
+__device__ __forceinline__ Place place(const FlatIndex &F, const FastDiv &dx, int col, unsigned q)
+{
+    int j, k, l;
+    return place<W>(F, dx, col, q, j, k, l);
 }
 
 // compact per-colour interior index of voxel (i, j, k, l)

@@ -38,6 +38,7 @@ CUDA_UNITS = {
     "ss4d_ws.cu": [],
     "ss4d_nn.cu": [],
     "ss4d_conv_tc.cu": [],
+    "ss4d_wgrad_tc.cu": [],
     "ss4d_assemble_ff.cu": [],
     "ss4d_front_ff.cu": [],
     "ss4d_front64.cu": ["--fmad=false"],

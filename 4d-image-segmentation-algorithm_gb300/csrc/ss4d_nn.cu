@@ -8,8 +8,8 @@
 // (ss4d_conv_tc.cu): an implicit GEMM per frame, M = voxels, N = output
 // channels, K = 27 taps x input channels.  The data gradient of a layer is
 // the same convolution with the taps reversed and the channel roles swapped;
-// the weight gradient is an FP32 reduction over voxels with a fixed
-// summation order (this file).
+// the weight gradient is a product over the voxels on the tensor cores too
+// (ss4d_wgrad_tc.cu).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -19,111 +19,6 @@
 
 namespace ss4d {
 namespace nn {
-
-constexpr int TX = 8, TY = 8, TZ = 4;
-constexpr int HX = TX + 2, HY = TY + 2, HZ = TZ + 2;
-constexpr int TV = TX * TY * TZ; // 256 output voxels per tile
-constexpr int HV = HX * HY * HZ; // 600 input voxels per tile
-
-// dW[tap][co][ci] and db[co] summed over the voxels of each block's tiles
-// (FP32); X: planar, CIN channels (the layer input), dY: planar, YS channels
-// of which COUT are used.  Each block writes its partial sums; k_reduce_cols adds them in
-// block order.
-__host__ __device__ constexpr int wgrad_smem_bytes(int cin, int cout)
-{
-    return (HV * cin + TV * cout) * 4;
-}
-
-template <int CIN, int COUT, int YS>
-__global__ void __launch_bounds__(256) k_wgrad(const __nv_bfloat16 *__restrict__ x,
-                                               const __nv_bfloat16 *__restrict__ dy, int nx, int ny, int nz, int nf,
-                                               float *partial)
-{
-    constexpr int NOUT = 27 * COUT * CIN;
-    constexpr int NP = (COUT * CIN + 255) / 256; // (co, ci) pairs per thread
-    extern __shared__ float wsm[];
-    float *sx = wsm;
-    float *sd = wsm + HV * CIN;
-    float acc[NP][27], bacc = 0.f;
-#pragma unroll
-    for (int p = 0; p < NP; ++p)
-#pragma unroll
-        for (int t = 0; t < 27; ++t)
-            acc[p][t] = 0.f;
-    const int tid = threadIdx.x;
-    const int ntx = (nx + TX - 1) / TX, nty = (ny + TY - 1) / TY, ntz = (nz + TZ - 1) / TZ;
-    const long long ntiles = (long long)ntx * nty * ntz * nf;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        long long r = tile;
-        const int tx0 = (int)(r % ntx) * TX;
-        r /= ntx;
-        const int ty0 = (int)(r % nty) * TY;
-        r /= nty;
-        const int tz0 = (int)(r % ntz) * TZ;
-        const int f = (int)(r / ntz);
-        __syncthreads();
-        for (int q = tid; q < HV * CIN; q += blockDim.x) {
-            const int v = q / CIN, c = q % CIN;
-            const int gx = tx0 + v % HX - 1, gy = ty0 + (v / HX) % HY - 1, gz = tz0 + v / (HX * HY) - 1;
-            float val = 0.f;
-            if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && gz >= 0 && gz < nz)
-                val = __bfloat162float(
-                    x[tc::planar_off(f, c, CIN / 8, (long long)nx * ny * nz, ((long long)gz * ny + gy) * nx + gx)]);
-            sx[q] = val;
-        }
-        for (int q = tid; q < TV * COUT; q += blockDim.x) {
-            const int m = q / COUT, c = q % COUT;
-            const int ox = tx0 + m % TX, oy = ty0 + (m / TX) % TY, oz = tz0 + m / (TX * TY);
-            float val = 0.f;
-            if (ox < nx && oy < ny && oz < nz)
-                val = __bfloat162float(
-                    dy[tc::planar_off(f, c, YS / 8, (long long)nx * ny * nz, ((long long)oz * ny + oy) * nx + ox)]);
-            sd[q] = val;
-        }
-        __syncthreads();
-        for (int m = 0; m < TV; ++m) {
-            const int hbase = ((m / (TX * TY) + 1) * HY + ((m / TX) % TY) + 1) * HX + (m % TX) + 1;
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                const int q = tid + 256 * p;
-                if (q < COUT * CIN) {
-                    const int co = q / CIN, ci = q % CIN;
-                    const float d = sd[m * COUT + co];
-                    const float *xb = sx + hbase * CIN + ci;
-#pragma unroll
-                    for (int t = 0; t < 27; ++t)
-                        acc[p][t] = fmaf(xb[(((t / 9 - 1) * HY + ((t / 3) % 3 - 1)) * HX + (t % 3 - 1)) * CIN], d,
-                                         acc[p][t]);
-                }
-            }
-            if (tid < COUT)
-                bacc += sd[m * COUT + tid];
-        }
-    }
-    // partial row of this block: [27][COUT][CIN] then [COUT]
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const int q = tid + 256 * p;
-        if (q < COUT * CIN)
-#pragma unroll
-            for (int t = 0; t < 27; ++t)
-                partial[(size_t)blockIdx.x * (NOUT + COUT) + (size_t)t * COUT * CIN + q] = acc[p][t];
-    }
-    if (tid < COUT)
-        partial[(size_t)blockIdx.x * (NOUT + COUT) + NOUT + tid] = bacc;
-}
-
-// out[c] = sum over rows r of in[r][c], rows in order
-__global__ void k_reduce_cols(const float *__restrict__ in, int rows, int cols, float *out)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols)
-        return;
-    float s = 0.f;
-    for (int r = 0; r < rows; ++r)
-        s += in[(size_t)r * cols + c];
-    out[c] = s;
-}
 
 // squared error over the voxels at least `margin` from the crop border;
 // dy (channel 0 of 16, planar) = d(mean squared error)/d out
@@ -176,19 +71,6 @@ __global__ void k_adam(float *p, const float *__restrict__ g, float *m, float *v
     m[i] = mi;
     v[i] = vi;
     p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-}
-
-// gradient rows of the weight partials -> master layout [27][cout][cin_real] + bias
-__global__ void k_unpack_grad(const float *__restrict__ gsum, int cout, int cinp, int cin, float *gw, float *gb)
-{
-    const int n = 27 * cout * cin;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) {
-        const int tap = q / (cout * cin), r = q % (cout * cin), co = r / cin, ci = r % cin;
-        gw[q] = gsum[((size_t)tap * cout + co) * cinp + ci];
-    } else if (q < n + cout) {
-        gb[q - n] = gsum[27 * cout * cinp + (q - n)];
-    }
 }
 
 } // namespace nn
@@ -262,7 +144,6 @@ struct ss4d_wsnet {
     float *y;
     float *partial;                // weight-gradient partials
     size_t partial_cap;
-    float *gsum;                   // reduced weight gradient of one layer
     float *loss_part;
     float h_loss;
     long long step;
@@ -293,7 +174,7 @@ extern "C" ss4d_status ss4d_wsnet_destroy(ss4d_wsnet *n)
         return SS4D_OK;
     cudaStreamSynchronize(n->stream);
     void *ptrs[] = {n->p, n->g, n->m, n->v, n->a[0], n->a[1], n->a[2], n->dz16, n->dz32[0], n->dz32[1], n->y,
-                    n->partial, n->gsum, n->loss_part, n->err};
+                    n->partial, n->loss_part, n->err};
     for (void *q : ptrs)
         if (q)
             cudaFree(q);
@@ -305,17 +186,6 @@ extern "C" ss4d_status ss4d_wsnet_destroy(ss4d_wsnet *n)
     }
     free(n);
     return SS4D_OK;
-}
-
-static void set_conv_attrs()
-{
-    static bool done = false;
-    if (done)
-        return;
-    cudaFuncSetAttribute(k_wgrad<16, 24, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem_bytes(16, 24));
-    cudaFuncSetAttribute(k_wgrad<32, 24, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem_bytes(32, 24));
-    cudaFuncSetAttribute(k_wgrad<32, 1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem_bytes(32, 1));
-    done = true;
 }
 
 extern "C" ss4d_status ss4d_wsnet_create(void *stream, ss4d_wsnet **out)
@@ -348,8 +218,6 @@ extern "C" ss4d_status ss4d_wsnet_create(void *stream, ss4d_wsnet **out)
     if (e == cudaSuccess)
         e = cudaMalloc((void **)&n->err, sizeof(int));
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&n->gsum, (size_t)(27 * 24 * 32 + 24) * 4);
-    if (e == cudaSuccess)
         e = cudaMalloc((void **)&n->loss_part, 4096 * 4);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -359,7 +227,6 @@ extern "C" ss4d_status ss4d_wsnet_create(void *stream, ss4d_wsnet **out)
     cudaMemsetAsync(n->m, 0, n->nparam * 4, n->stream);
     cudaMemsetAsync(n->v, 0, n->nparam * 4, n->stream);
     cudaMemsetAsync(n->err, 0, sizeof(int), n->stream);
-    set_conv_attrs();
     *out = n;
     return SS4D_OK;
 }
@@ -482,13 +349,6 @@ static ss4d_status ensure_act(ss4d_wsnet *n, size_t vox, bool train)
     return SS4D_OK;
 }
 
-static int conv_grid(const ss4d_wsnet *n, int nx, int ny, int nz, int nf)
-{
-    const long long tiles = (long long)((nx + TX - 1) / TX) * ((ny + TY - 1) / TY) * ((nz + TZ - 1) / TZ) * nf;
-    const long long g = (long long)n->sm * 2;
-    return (int)(tiles < g ? tiles : g);
-}
-
 // one convolution on the tensor cores: cin input channels (16 or 32), nout
 // computed output channels (32, or 16 for the output layer), cout of them real
 static void conv(ss4d_wsnet *n, int cin, int nout, int cout, const __nv_bfloat16 *x, const __nv_bfloat16 *w,
@@ -545,24 +405,23 @@ extern "C" ss4d_status ss4d_wsnet_forward(ss4d_wsnet *n, const void *d_x0, int n
     return forward(n, (const __nv_bfloat16 *)d_x0, nx, ny, nz, nf, false, d_out);
 }
 
-template <int CIN, int COUT, int YS>
-static ss4d_status wgrad(ss4d_wsnet *n, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, int nx, int ny, int nz,
-                         int nf, int cin_real, float *gw, float *gb)
+// the weight and bias gradient of layer L from its input x and output gradient dy
+static ss4d_status wgrad(ss4d_wsnet *n, int L, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, int nx, int ny, int nz,
+                         int nf, float *gw, float *gb)
 {
-    const int grid = conv_grid(n, nx, ny, nz, nf);
-    const size_t cols = (size_t)27 * COUT * CIN + COUT;
-    if (n->partial_cap < cols * grid) {
+    const Layer &l = kLayers[L];
+    const size_t need = (size_t)tc::wgrad_ctas(nx, ny, nz, nf, n->sm) * (27 * 24 * 32 + 24); // the largest layer's
+    if (n->partial_cap < need) {
         if (n->partial)
             cudaFree(n->partial);
         n->partial = nullptr;
-        NCK(cudaMalloc((void **)&n->partial, cols * grid * 4));
-        n->partial_cap = cols * grid;
+        n->partial_cap = 0;
+        NCK(cudaMalloc((void **)&n->partial, need * 4));
+        n->partial_cap = need;
     }
-    k_wgrad<CIN, COUT, YS><<<grid, 256, wgrad_smem_bytes(CIN, COUT), n->stream>>>(x, dy, nx, ny, nz, nf, n->partial);
-    k_reduce_cols<<<(int)((cols + 255) / 256), 256, 0, n->stream>>>(n->partial, grid, (int)cols, n->gsum);
-    const int nmaster = 27 * COUT * cin_real + COUT;
-    k_unpack_grad<<<(nmaster + 255) / 256, 256, 0, n->stream>>>(n->gsum, COUT, CIN, cin_real, gw, gb);
-    NCK(cudaGetLastError());
+    if (tc::wgrad_tc(l.cinp, l.coutp_t, l.cout, l.cin, x, dy, nx, ny, nz, nf, n->partial, gw, gb, n->err, n->sm,
+                     n->stream) != cudaSuccess)
+        n->launch_failed = 1;
     return SS4D_OK;
 }
 
@@ -585,19 +444,19 @@ extern "C" ss4d_status ss4d_wsnet_train_step(ss4d_wsnet *n, const void *d_x0, co
     k_mse<<<lb, 256, 0, n->stream>>>(n->y, d_target, nx, ny, nz, nf, margin, 1.f / (float)inner, n->dz16,
                                      n->loss_part);
     // layer 4 (3 -> out): weights and data gradient (masked by a3 > 0)
-    if (wgrad<32, 1, 16>(n, n->a[2], n->dz16, nx, ny, nz, nf, 24, n->g + woff[3], n->g + boff[3]) != SS4D_OK)
+    if (wgrad(n, 3, n->a[2], n->dz16, nx, ny, nz, nf, n->g + woff[3], n->g + boff[3]) != SS4D_OK)
         return SS4D_ERR_CUDA;
     conv(n, 16, 32, 24, n->dz16, n->wt[3], nullptr, n->a[2], n->dz32[0], nullptr, nx, ny, nz, nf, 0);
     // layer 3
-    if (wgrad<32, 24, 32>(n, n->a[1], n->dz32[0], nx, ny, nz, nf, 24, n->g + woff[2], n->g + boff[2]) != SS4D_OK)
+    if (wgrad(n, 2, n->a[1], n->dz32[0], nx, ny, nz, nf, n->g + woff[2], n->g + boff[2]) != SS4D_OK)
         return SS4D_ERR_CUDA;
     conv(n, 32, 32, 24, n->dz32[0], n->wt[2], nullptr, n->a[1], n->dz32[1], nullptr, nx, ny, nz, nf, 0);
     // layer 2
-    if (wgrad<32, 24, 32>(n, n->a[0], n->dz32[1], nx, ny, nz, nf, 24, n->g + woff[1], n->g + boff[1]) != SS4D_OK)
+    if (wgrad(n, 1, n->a[0], n->dz32[1], nx, ny, nz, nf, n->g + woff[1], n->g + boff[1]) != SS4D_OK)
         return SS4D_ERR_CUDA;
     conv(n, 32, 32, 24, n->dz32[1], n->wt[1], nullptr, n->a[0], n->dz32[0], nullptr, nx, ny, nz, nf, 0);
     // layer 1
-    if (wgrad<16, 24, 32>(n, x0, n->dz32[0], nx, ny, nz, nf, 16, n->g + woff[0], n->g + boff[0]) != SS4D_OK)
+    if (wgrad(n, 0, x0, n->dz32[0], nx, ny, nz, nf, n->g + woff[0], n->g + boff[0]) != SS4D_OK)
         return SS4D_ERR_CUDA;
     if (n->launch_failed)
         return nfail(SS4D_ERR_CUDA, "a tensor-core convolution could not be launched (tensor map or launch)");

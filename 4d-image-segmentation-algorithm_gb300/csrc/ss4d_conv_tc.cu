@@ -32,8 +32,8 @@
 // per MMA, not per column, so a first MMA of A = 0 clears all TZ
 // accumulators and every MMA after it accumulates.
 //
-// Per CTA: one thread of a fifth warp issues the TMA loads and the MMAs, four
-// warps drain the accumulators (TMEM -> registers -> bias, ReLU, mask ->
+// Per CTA: one thread of the last warp issues the TMA loads and the MMAs, four
+// or eight warps drain the accumulators (TMEM -> registers -> bias, ReLU, mask ->
 // global); STAGES halo tiles and two accumulator buffers are in flight and
 // the roles meet only at mbarriers, so the loads of the next tiles and the
 // epilogue of tile i-1 run while the tensor core works on tile i.  Every wait on an
@@ -54,16 +54,20 @@ namespace tc {
 
 // ---- the kernel ---------------------------------------------------------------
 
-// warp roles: warps 0-3 read the accumulators (a warp reaches only its own 32
-// lanes of tensor memory) and store; lane 0 of warp 4 issues the loads and
-// the MMAs.  Barriers, one phase per use: full[s] (the loads of the tile in
+// warp roles: warps 0-3 (or 0-7: warps w and w + 4 reach the same 32 lanes
+// of tensor memory and take half of the planes each) read the accumulators
+// and store; lane 0 of the last warp issues the loads and the MMAs.  Barriers, one phase per use: full[s] (the loads of the tile in
 // halo stage s landed), done[b] (the MMAs of the tile in accumulator buffer
-// b completed: tcgen05.commit), free[b] (the four epilogue warps have read
+// b completed: tcgen05.commit), free[b] (the epilogue warps have read
 // buffer b).  Tile it uses stage it % STAGES and buffer it % 2.
-constexpr int EPI_WARPS = 4, THREADS = 32 * (EPI_WARPS + 1);
-
-template <int CIN, int N>
-__global__ void __launch_bounds__(THREADS, 1) k_conv_tc(const __grid_constant__ CUtensorMap tmap, TcArgs a)
+// A data gradient's epilogue loads its masks, 64 bytes a voxel: with eight
+// warps and the masks loaded ahead 51 -> 30 us per hidden layer at 8 crops of
+// 40x40x20 (four tiles per CTA).  Without masks, or over many tiles, the
+// tensor core's operand reads set the pace and four warps, whose tensor-memory
+// reads are spread out, disturb them less (a forward of 12 frames of
+// 128x128x64 3.64 ms against 3.73).
+template <int CIN, int N, int EPI_WARPS>
+__global__ void __launch_bounds__(32 * (EPI_WARPS + 1), 1) k_conv_tc(const __grid_constant__ CUtensorMap tmap, TcArgs a)
 {
     using C = TcCfg<CIN, N>;
     extern __shared__ unsigned char smem_raw[];
@@ -205,9 +209,26 @@ __global__ void __launch_bounds__(THREADS, 1) k_conv_tc(const __grid_constant__ 
         }
     } else {
         // ---- epilogue warps: accumulators -> bias, ReLU, mask -> global ----
-        const int m = warp * 32 + lane;
+        const int quad = warp & 3, m = quad * 32 + lane;
+        constexpr int PL = TZ / (EPI_WARPS / 4); // planes per warp
+        const int p0 = (warp >> 2) * PL;
+        const long long vol = (long long)a.nx * a.ny * a.nz;
         for (int it = 0; it < my_n; ++it) {
             const int b = it & 1;
+            int x0, y0, z0, f;
+            tile_xyzf(it, x0, y0, z0, f);
+            const int ox = x0 + (m & 7), oy = y0 + (m >> 3);
+            MaskRegs<N> mask[EPI_WARPS == 8 ? PL : 1];
+            auto masks = [&](int p) {
+                const int oz = z0 + p0 + p;
+                if (a.mask && ox < a.nx && oy < a.ny && oz < a.nz)
+                    load_masks<N>(a, mask[EPI_WARPS == 8 ? p : 0], f, ((long long)oz * a.ny + oy) * a.nx + ox, vol);
+            };
+            if (EPI_WARPS == 8) { // the masks come while the tensor core works on the tile
+#pragma unroll
+                for (int p = 0; p < PL; ++p)
+                    masks(p);
+            }
             // one lane waits, so that the warp stays converged for the
             // .sync.aligned tensor-memory loads
             int ok = 0;
@@ -220,13 +241,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_conv_tc(const __grid_constant__ 
                 break;
             }
             tc_fence_after();
-            int x0, y0, z0, f;
-            tile_xyzf(it, x0, y0, z0, f);
-            const int ox = x0 + (m & 7), oy = y0 + (m >> 3);
-            const long long vol = (long long)a.nx * a.ny * a.nz;
-#pragma unroll 1
-            for (int p = 0; p < TZ; ++p) {
-                const uint32_t col = tmem + (uint32_t)(b * TZ * N + (TZ - 1 - p) * N) + ((uint32_t)(warp * 32) << 16);
+            auto plane = [&](int p) {
+                const uint32_t col =
+                    tmem + (uint32_t)(b * TZ * N + (TZ - 1 - p0 - p) * N) + ((uint32_t)(quad * 32) << 16);
                 float v[N];
 #pragma unroll
                 for (int h = 0; h < N / 16; ++h) {
@@ -237,9 +254,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_conv_tc(const __grid_constant__ 
                     for (int e = 0; e < 16; ++e)
                         v[16 * h + e] = __uint_as_float(r[e]);
                 }
-                const int oz = z0 + p;
+                const int oz = z0 + p0 + p;
                 if (ox < a.nx && oy < a.ny && oz < a.nz)
-                    epilogue_store<N>(a, v, f, ((long long)oz * a.ny + oy) * a.nx + ox, vol);
+                    epilogue_store<N, EPI_WARPS == 8>(a, v, mask[EPI_WARPS == 8 ? p : 0], f,
+                                                      ((long long)oz * a.ny + oy) * a.nx + ox, vol);
+            };
+            if (EPI_WARPS == 8) {
+#pragma unroll
+                for (int p = 0; p < PL; ++p)
+                    plane(p);
+            } else {
+#pragma unroll 1
+                for (int p = 0; p < PL; ++p)
+                    plane(p);
             }
             // this warp is done with the buffer's tensor memory
             tc_fence_before();
@@ -274,13 +301,21 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 }
 
 namespace {
-template <int CIN, int N> void set_attr_once()
+template <int CIN, int N, int W>
+cudaError_t launch_warps(const CUtensorMap &m, const TcArgs &a, long long tiles, int sm_count, cudaStream_t st)
 {
-    static bool done = false;
-    if (!done) {
-        cudaFuncSetAttribute(k_conv_tc<CIN, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<CIN, N>::SMEM);
-        done = true;
+    constexpr int threads = 32 * (W + 1);
+    static int per_sm = 0;
+    if (!per_sm) {
+        cudaFuncSetAttribute(k_conv_tc<CIN, N, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<CIN, N>::SMEM);
+        int p = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k_conv_tc<CIN, N, W>, threads, TcCfg<CIN, N>::SMEM);
+        per_sm = p < 1 ? 1 : (p > 2 ? 2 : p); // tensor memory: 2 x TCOLS <= 512 columns
     }
+    const long long cap = (long long)sm_count * per_sm;
+    const int grid = (int)(tiles < cap ? tiles : cap);
+    k_conv_tc<CIN, N, W><<<grid, threads, TcCfg<CIN, N>::SMEM, st>>>(m, a);
+    return cudaGetLastError();
 }
 } // namespace
 
@@ -307,17 +342,9 @@ static cudaError_t launch(const void *x, const TcArgs &a, int sm_count, cudaStre
     CUtensorMap m;
     if (!make_map(&m, x, CIN, a.nx, a.ny, a.nz, a.nf))
         return cudaErrorInvalidValue;
-    set_attr_once<CIN, N>();
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv_tc<CIN, N>, THREADS, TcCfg<CIN, N>::SMEM);
-        per_sm = per_sm < 1 ? 1 : (per_sm > 2 ? 2 : per_sm); // tensor memory: 2 x TCOLS <= 512 columns
-    }
     const long long tiles = tc_tiles(a.nx, a.ny, a.nz, a.nf);
-    const long long cap = (long long)sm_count * per_sm;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    k_conv_tc<CIN, N><<<grid, THREADS, TcCfg<CIN, N>::SMEM, st>>>(m, a);
-    return cudaGetLastError();
+    return a.mask && tiles <= 16LL * sm_count ? launch_warps<CIN, N, 8>(m, a, tiles, sm_count, st)
+                                              : launch_warps<CIN, N, 4>(m, a, tiles, sm_count, st);
 }
 
 cudaError_t conv_tc(int cin, int n, const void *x, const TcArgs &a, int sm_count, cudaStream_t st)

@@ -75,10 +75,24 @@ __host__ __device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t l
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
-// one voxel's N accumulated channels -> bias, ReLU, mask -> global; voxel vf
-// of frame f, vol voxels per frame
+// the masks of one voxel's channels (16 bytes per 8 of them)
+template <int N> struct MaskRegs {
+    uint4 q[N / 8];
+};
 template <int N>
-__device__ __forceinline__ void epilogue_store(const TcArgs &a, float (&v)[N], int f, long long vf, long long vol)
+__device__ __forceinline__ void load_masks(const TcArgs &a, MaskRegs<N> &m, int f, long long vf, long long vol)
+{
+#pragma unroll
+    for (int c = 0; c < N; c += 8)
+        if (c < a.mstride)
+            m.q[c / 8] = __ldg(reinterpret_cast<const uint4 *>(a.mask + planar_off(f, c, a.mstride / 8, vol, vf)));
+}
+
+// one voxel's N accumulated channels -> bias, ReLU, mask (loaded AHEAD, or
+// here) -> global; voxel vf of frame f, vol voxels per frame
+template <int N, bool AHEAD>
+__device__ __forceinline__ void epilogue_store(const TcArgs &a, float (&v)[N], MaskRegs<N> &mask, int f, long long vf,
+                                               long long vol)
 {
 #pragma unroll
     for (int c = 0; c < N; ++c) {
@@ -90,12 +104,13 @@ __device__ __forceinline__ void epilogue_store(const TcArgs &a, float (&v)[N], i
         v[c] = x;
     }
     if (a.mask) {
+        if (!AHEAD)
+            load_masks<N>(a, mask, f, vf, vol);
 #pragma unroll
         for (int c = 0; c < N; c += 8) {
             if (c >= a.mstride)
                 break;
-            const uint4 q = *reinterpret_cast<const uint4 *>(a.mask + planar_off(f, c, a.mstride / 8, vol, vf));
-            const __nv_bfloat162 *m2 = reinterpret_cast<const __nv_bfloat162 *>(&q);
+            const __nv_bfloat162 *m2 = reinterpret_cast<const __nv_bfloat162 *>(&mask.q[c / 8]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 if (!(__low2float(m2[e]) > 0.f))

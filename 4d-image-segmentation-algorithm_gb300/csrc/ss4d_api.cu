@@ -145,7 +145,7 @@ struct ss4d_solver {
     int pre_next;    // the next mixed loop's first refinement pass was formed by the assembly
     float *hist[4];  // earlier steps' changes (split layout): h1 red, h1 black, h2 red, h2 black
     int proj;        // start the first round from the projection onto the earlier changes (ss4d_project.cu)
-    double *d_proj;  // its per-block sums (18 * n_partial / 2 doubles) and coefficients (3 floats after them)
+    double *d_proj;  // its per-block sums (18 * n_partial / 2 doubles), coefficients (3 floats after them) and block count
     double inner_omega; // mixed form: relaxation factor of the FP32 sweeps (0: omega_c)
     // per-kernel timing (ss4d_solver_set_timing)
     int timing;
@@ -884,13 +884,15 @@ static ss4d_status project_start(ss4d_solver *s, int pre, LoopState *d_state)
     if (!s->d_proj) {
         const size_t nd = 9 * (size_t)s->n_partial; // 18 * grid with n_partial >= 2 * grid
         CKS(dmalloc(s, (void **)&s->d_proj, sizeof(double) * nd + 4 * sizeof(float)));
+        CK(cudaMemsetAsync(s->d_proj + nd, 0, 4 * sizeof(float), s->stream)); // the count of finished blocks
     }
     float *c = reinterpret_cast<float *>(s->d_proj + 9 * (size_t)s->n_partial);
     const int m = s->have_dprev >= 3 ? 3 : 2;
     timed(s, SS4D_K_PROJECT, true, [&] {
-        launch_projection(s->geo, s->sp, s->cfg, s->sb, s->hist, m, s->d_proj, c, d_state, s->sm_count, s->stream);
+        launch_projection(s->geo, s->sp, s->cfg, s->sb, s->hist, m, s->d_proj, c,
+                          reinterpret_cast<unsigned *>(c + 3), d_state, s->sm_count, s->stream);
     });
-    s->launches += 4;
+    s->launches += 2;
     return SS4D_OK;
 }
 

@@ -252,9 +252,10 @@ struct SolverView {
 };
 // the first round's start from the previous steps' changes (ss4d_project.cu):
 // hist = the extrapolation history arrays (h1 red, h1 black, h2 red, h2 black),
-// m = 2 or 3 vectors, part = 18 * cfg.grid doubles, c = 3 floats
+// m = 2 or 3 vectors, part = 18 * cfg.grid doubles, c = 3 floats, done a zero
+// that is zero again afterwards
 void launch_projection(const Geo &g, const Split &sp, const SweepCfg &cfg, SplitBufs b, float *const *hist, int m,
-                       double *part, float *c, LoopState *st, int sm_count, cudaStream_t s);
+                       double *part, float *c, unsigned *done, LoopState *st, int sm_count, cudaStream_t s);
 SweepCfg make_sweep_cfg_xt(const Geo &g, const Split &s, int sm_count, int kb, int xt);
 // tiles of the kernels that give each thread two adjacent targets of a row
 // (the FP32 sweep, the projection's products): cfg's row chunks of cfg.XT

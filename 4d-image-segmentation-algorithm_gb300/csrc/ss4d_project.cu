@@ -20,16 +20,16 @@
 // the round measures the exact FP64 residual as always, so the stop rule and
 // the tolerance do not depend on the start.
 //
-//   k_proj_dots<COL>: per block the nine sums H_00 H_01 H_02 H_11 H_12 H_22
-//                     g_0 g_1 g_2 over a sample of the targets of colour
-//                     COL (every PROJ_STRIDE-th tile);
-//   k_proj_solve:     one block sums the partials of both colours in a fixed
-//                     order and solves H c = g (Cholesky, FP64); a system that
-//                     is not positive definite, or sums that are not finite,
-//                     leave the start at zero;
-//   k_proj_start:     d0 into the round's correction arrays (red: dR[dsrc],
-//                     black: dB) and LoopState.keep, so that the round's start
-//                     keeps it (k_zero_delta).
+//   k_proj_dots:  per block the nine sums H_00 H_01 H_02 H_11 H_12 H_22
+//                 g_0 g_1 g_2 over a sample of the targets of one colour
+//                 (every PROJ_STRIDE-th tile), one half of the grid for each
+//                 colour; the last block to finish adds the partials in a
+//                 fixed order and solves H c = g (Cholesky, FP64); a system
+//                 that is not positive definite, or sums that are not finite,
+//                 leave the start at zero;
+//   k_proj_start: d0 into the round's correction arrays (red: dR[dsrc],
+//                 black: dB) and LoopState.keep, so that the round's start
+//                 keeps it (k_zero_delta).
 #include "ss4d_sweep.cuh"
 
 namespace ss4d {
@@ -104,22 +104,21 @@ __device__ __forceinline__ float2 av_pair(const float *__restrict__ own, const f
 // since the FP64 refinement judges the result.
 constexpr int PROJ_STRIDE = 9;
 
-// two adjacent targets per thread (pc: make_pair_cfg), 64 registers (four
-// blocks per SM); every block of the launch writes its nine partials
+// the nine sums of a block's share of colour COL, block `block` of `half`,
+// per thread
 template <int COL>
-__global__ void __launch_bounds__(256, 4) k_proj_dots(Geo g, Split sp, SweepCfg pc, SplitBufs b, ProjVecs V, int m,
-                                                      double *part)
+__device__ __forceinline__ void proj_sums(const Geo &g, const Split &sp, const SweepCfg &pc, const SplitBufs &b,
+                                          const ProjVecs &V, int m, unsigned block, unsigned half, float acc[9])
 {
     const unsigned Hy = (unsigned)sp.Hs, Hz = Hy * (unsigned)g.jM, Hw = Hz * (unsigned)g.kM;
     const uint4 *__restrict__ cq = b.coefq[COL];
     const float *__restrict__ cs = b.coefs[COL];
     const double *__restrict__ rp = b.rpre[COL];
     const int tx = threadIdx.x & (pc.XT - 1), ty = threadIdx.x / pc.XT;
-    float acc[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q)
         acc[q] = 0.f;
-    for (long long t = (long long)blockIdx.x * PROJ_STRIDE; t < pc.ntiles; t += (long long)gridDim.x * PROJ_STRIDE) {
+    for (long long t = (long long)block * PROJ_STRIDE; t < pc.ntiles; t += (long long)half * PROJ_STRIDE) {
         const TileCoord tc = tile_coord(g, pc, t, tx, ty);
         if (!tc.ok)
             continue;
@@ -160,77 +159,136 @@ __global__ void __launch_bounds__(256, 4) k_proj_dots(Geo g, Split sp, SweepCfg 
         acc[7] = fmaf(rh0, Av[1].x, fmaf(rh1, Av[1].y, acc[7]));
         acc[8] = fmaf(rh0, Av[2].x, fmaf(rh1, Av[2].y, acc[8]));
     }
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        const double tot = block_sum((double)acc[q]);
-        if (threadIdx.x == 0)
-            part[(size_t)(COL * 9 + q) * gridDim.x + blockIdx.x] = tot;
-    }
 }
 
-// c[0..2] for the start; st->keep = 1 when the start is used
-__global__ void k_proj_solve(const double *__restrict__ part, int grid, int m, LoopState *st, float *c)
+// c[0..2] for the start from the nine sums; st->keep = 1 when it is used.
+// Loops of constant length, so that the little system stays in registers.
+__device__ __forceinline__ void proj_solve(const double *sum, int m, LoopState *st, float *c)
 {
-    __shared__ double sum[9];
-    if (st->stop)
-        return;
-    for (int q = 0; q < 9; ++q) {
-        double a = 0.0;
-        for (int t = threadIdx.x; t < grid; t += blockDim.x)
-            a += part[(size_t)q * grid + t] + part[(size_t)(9 + q) * grid + t];
-        a = block_sum(a);
-        if (threadIdx.x == 0)
-            sum[q] = a;
-        __syncthreads();
-    }
-    if (threadIdx.x != 0)
-        return;
     const int iu[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-    double H[3][3], x[3], L[3][3] = {{0.0}};
+    double x[3], L[3][3];
     bool ok = m >= 1;
-    for (int i = 0; i < m; ++i) {
-        x[i] = sum[6 + i];
-        for (int j = 0; j < m; ++j)
-            H[i][j] = sum[iu[i][j]];
-    }
     // Cholesky H = L L^T; a pivot below 1e-12 of its diagonal entry (or not
     // finite) rejects the system
-    for (int j = 0; j < m && ok; ++j) {
-        double d = H[j][j];
-        for (int k = 0; k < j; ++k)
-            d -= L[j][k] * L[j][k];
-        if (!(d > 1e-12 * H[j][j]) || !isfinite(d)) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        if (j >= m || !ok)
+            continue;
+        x[j] = sum[6 + j];
+        double d = sum[iu[j][j]];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (k < j)
+                d -= L[j][k] * L[j][k];
+        if (!(d > 1e-12 * sum[iu[j][j]]) || !isfinite(d)) {
             ok = false;
-            break;
+            continue;
         }
         L[j][j] = sqrt(d);
-        for (int i = j + 1; i < m; ++i) {
-            double e = H[i][j];
-            for (int k = 0; k < j; ++k)
-                e -= L[i][k] * L[j][k];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (i <= j || i >= m)
+                continue;
+            double e = sum[iu[i][j]];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k < j)
+                    e -= L[i][k] * L[j][k];
             L[i][j] = e / L[j][j];
         }
     }
     if (ok) {
-        for (int i = 0; i < m; ++i) { // L y = g
-            for (int k = 0; k < i; ++k)
-                x[i] -= L[i][k] * x[k];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) { // L y = g
+            if (i >= m)
+                continue;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k < i)
+                    x[i] -= L[i][k] * x[k];
             x[i] /= L[i][i];
         }
-        for (int i = m - 1; i >= 0; --i) { // L^T c = y
-            for (int k = i + 1; k < m; ++k)
-                x[i] -= L[k][i] * x[k];
+#pragma unroll
+        for (int i = 2; i >= 0; --i) { // L^T c = y
+            if (i >= m)
+                continue;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k > i && k < m)
+                    x[i] -= L[k][i] * x[k];
             x[i] /= L[i][i];
-        }
-        for (int i = 0; i < m; ++i)
             ok = ok && isfinite(x[i]);
+        }
     }
+#pragma unroll
     for (int i = 0; i < 3; ++i)
         c[i] = ok && i < m ? (float)x[i] : 0.f;
     st->keep = ok ? 1 : 0;
     st->proj = ok ? 1 : 0;
 }
 
+// Two adjacent targets per thread (pc: make_pair_cfg), 64 registers (four
+// blocks per SM); blocks 0 .. half - 1 take the red targets, the others the
+// black ones.  A block's sums are added quantity by quantity, one warp each:
+// each lane first adds eight threads' values, since five FP64 shuffle steps in
+// every warp for each of nine quantities (2,880 FP64 instructions a block)
+// took longer than a small volume's products.  At 45x37x29x7 the projection's
+// kernels took 78 us per step (two product launches of 19, the solve 31, the
+// start 6), now 22.
+__global__ void __launch_bounds__(256, 4) k_proj_dots(Geo g, Split sp, SweepCfg pc, SplitBufs b, ProjVecs V, int m,
+                                                      double *part, unsigned *done, LoopState *st, float *c)
+{
+    __shared__ float vals[9][256];
+    __shared__ double sum[9];
+    __shared__ int last;
+    const unsigned half = gridDim.x / 2;
+    const int colour = blockIdx.x >= half;
+    const unsigned block = blockIdx.x - (colour ? half : 0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float acc[9];
+    if (colour == 0)
+        proj_sums<0>(g, sp, pc, b, V, m, block, half, acc);
+    else
+        proj_sums<1>(g, sp, pc, b, V, m, block, half, acc);
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+        vals[q][threadIdx.x] = acc[q];
+    __syncthreads();
+    for (int q = warp; q < 9; q += 8) {
+        double a = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+            a += (double)vals[q][32 * w + lane];
+        a = warp_sum(a);
+        if (lane == 0)
+            part[(size_t)q * gridDim.x + blockIdx.x] = a;
+    }
+    // the last block to finish has every partial
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last)
+        return;
+    __threadfence();
+    for (int q = warp; q < 9; q += 8) {
+        double a = 0.0;
+        for (unsigned t = lane; t < gridDim.x; t += 32)
+            a += __ldcg(part + (size_t)q * gridDim.x + t);
+        a = warp_sum(a);
+        if (lane == 0)
+            sum[q] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *done = 0; // for the next step
+        if (!st->stop)
+            proj_solve(sum, m, st, c);
+    }
+}
+
+// four columns per thread (cs is a multiple of 8)
 __global__ void __launch_bounds__(256) k_proj_start(Split sp, SplitBufs b, ProjVecs V, int m,
                                                     const float *__restrict__ c, const LoopState *__restrict__ st)
 {
@@ -238,22 +296,27 @@ __global__ void __launch_bounds__(256) k_proj_start(Split sp, SplitBufs b, ProjV
         return;
     const float c0 = c[0], c1 = c[1], c2 = c[2];
     float *red = pick(b.dR, st->dsrc);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < sp.cs;
-         t += (long long)gridDim.x * blockDim.x) {
+    const long long n = sp.cs >> 2;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int col = 0; col < 2; ++col) {
-            float d = c0 * V.v[0][col][t];
-            if (m >= 2)
-                d = fmaf(c1, V.v[1][col][t], d);
-            if (m >= 3)
-                d = fmaf(c2, V.v[2][col][t], d);
-            (col == 0 ? red : b.dB)[t] = d;
+            const float4 a = reinterpret_cast<const float4 *>(V.v[0][col])[t];
+            float4 d = make_float4(c0 * a.x, c0 * a.y, c0 * a.z, c0 * a.w);
+            if (m >= 2) {
+                const float4 e = reinterpret_cast<const float4 *>(V.v[1][col])[t];
+                d = make_float4(fmaf(c1, e.x, d.x), fmaf(c1, e.y, d.y), fmaf(c1, e.z, d.z), fmaf(c1, e.w, d.w));
+            }
+            if (m >= 3) {
+                const float4 e = reinterpret_cast<const float4 *>(V.v[2][col])[t];
+                d = make_float4(fmaf(c2, e.x, d.x), fmaf(c2, e.y, d.y), fmaf(c2, e.z, d.z), fmaf(c2, e.w, d.w));
+            }
+            reinterpret_cast<float4 *>(col == 0 ? red : b.dB)[t] = d;
         }
     }
 }
 
 void launch_projection(const Geo &g, const Split &sp, const SweepCfg &cfg, SplitBufs b, float *const *hist, int m,
-                       double *part, float *c, LoopState *st, int sm_count, cudaStream_t s)
+                       double *part, float *c, unsigned *done, LoopState *st, int sm_count, cudaStream_t s)
 {
     ProjVecs V;
     for (int col = 0; col < 2; ++col) {
@@ -267,20 +330,20 @@ void launch_projection(const Geo &g, const Split &sp, const SweepCfg &cfg, Split
     // buffer part is sized for)
     static int per_sm = 0;
     if (!per_sm) {
-        int a = 0, b1 = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_proj_dots<0>, 256, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_proj_dots<1>, 256, 0);
-        per_sm = a < b1 ? a : b1;
-        if (per_sm < 1)
-            per_sm = 1;
+        int a = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_proj_dots, 256, 0);
+        per_sm = a < 1 ? 1 : a;
     }
+    // per colour: blocks beyond the sampled tiles would add zeros
+    const long long tiles = (pc.ntiles + PROJ_STRIDE - 1) / PROJ_STRIDE;
     int grid = sm_count * per_sm;
     if (grid > cfg.grid)
         grid = cfg.grid;
-    k_proj_dots<0><<<grid, 256, 0, s>>>(g, sp, pc, b, V, m, part);
-    k_proj_dots<1><<<grid, 256, 0, s>>>(g, sp, pc, b, V, m, part);
-    k_proj_solve<<<1, 256, 0, s>>>(part, grid, m, st, c);
-    k_proj_start<<<sm_count * 8, 256, 0, s>>>(sp, b, V, m, c, st);
+    if (grid > tiles)
+        grid = (int)tiles;
+    k_proj_dots<<<2 * grid, 256, 0, s>>>(g, sp, pc, b, V, m, part, done, st, c);
+    const long long need = (sp.cs / 4 + 255) / 256;
+    k_proj_start<<<(int)(need < sm_count * 8 ? need : sm_count * 8), 256, 0, s>>>(sp, b, V, m, c, st);
 }
 
 } // namespace ss4d

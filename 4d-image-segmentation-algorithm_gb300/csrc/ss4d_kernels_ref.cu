@@ -9,6 +9,10 @@
 // serial sum).  They serve the SS4D_ARITH_REFERENCE form, the edge detector of
 // every form (run once per segmentation), the MCF boundary and exact
 // solution, the rescale, the mask and the norms.
+#include <cooperative_groups.h>
+#include <float.h>
+#include <math.h>
+
 #include "ss4d_exact.cuh"
 #include "ss4d_kernels.cuh"
 
@@ -396,41 +400,60 @@ __device__ inline double mcf_coord(int i, double h)
     return ((i - 1) * h) + (h / 2.) - 1.25;
 }
 
-__device__ inline double mcf_value(double x, double y, double z, double w, double t)
+// (x^2 + y^2 + z^2 + w^2 - 1) / 6 + t in the reference's order
+__device__ __forceinline__ double mcf_value(double x, double y2, double z2, double w2, double t)
 {
-    return ((x * x + y * y + z * z + w * w - 1.0) / 6.0) + t;
+    return div_by_const(x * x + y2 + z2 + w2 - 1.0, 6.0, 1.0 / 6.0) + t;
 }
 
+// the coordinate of index q of an axis of M, on a face if asked for
+__device__ __forceinline__ double mcf_axis(int q, int M, double h, bool face)
+{
+    return face ? (q == M - 1 ? (h / 2.) + 1.25 : -(h / 2.) - 1.25) : mcf_coord(q, h);
+}
+
+// On a ghost the reference's eight passes run x-lo, x-hi, ..., w-hi over full
+// ranges: the last pass touching it decides its value, and it uses the special
+// face coordinate on its own axis only: the last axis the voxel is a ghost on.
+// With ghosts_only a thread per x ghost of the interior rows, then (as for
+// the whole field) a warp per padded row that is all ghosts, y, z and w formed
+// once per row.  A value costs tens of FP64 instructions, which a warp pays in
+// full for one lane: walking every voxel, or a warp per interior row for its
+// two ghosts, took 191-197 us at 40^4, every ghost with its own four coordinates 90.
 __global__ void k_mcf_field(Geo g, double *u, double h, double t, int ghosts_only)
 {
-    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < g.n; o += (long long)gridDim.x * blockDim.x) {
-        long long r = o;
-        const int i = (int)(r % g.iM); r /= g.iM;
-        const int j = (int)(r % g.jM); r /= g.jM;
-        const int k = (int)(r % g.kM);
-        const int l = (int)(r / g.kM);
-        const int idx[4] = {i, j, k, l};
-        const int M[4] = {g.iM, g.jM, g.kM, g.lM};
-        double x[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-            x[a] = mcf_coord(idx[a], h);
-        if (ghosts_only) {
-            // the reference's eight passes run x-lo, x-hi, ..., w-hi over full
-            // ranges: the last pass touching a ghost decides its value, and it
-            // uses the special face coordinate on its own axis only.
-            int last = -1;
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-                if (idx[a] == 0 || idx[a] == M[a] - 1)
-                    last = a;
-            if (last < 0)
-                continue;
-            x[last] = idx[last] == M[last] - 1 ? (h / 2.) + 1.25 : -(h / 2.) - 1.25;
-            if (M[last] == 1)
-                x[last] = (h / 2.) + 1.25;
+    const unsigned rows = (unsigned)(g.jM * g.kM * g.lM), threads = gridDim.x * blockDim.x;
+    const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    auto coords = [&](unsigned r, int &j, int &k, int &l) {
+        const unsigned rk = fdiv(r, g.fjM), q = fdiv(rk, g.fkM);
+        j = (int)(r - rk * g.fjM.d);
+        k = (int)(rk - q * g.fkM.d);
+        l = (int)q;
+        return j >= 1 && j <= g.ny && k >= 1 && k <= g.nz && l >= 1 && l <= g.nt;
+    };
+    auto square = [&](int q, int M, bool face) {
+        const double c = mcf_axis(q, M, h, face);
+        return c * c;
+    };
+    int j, k, l;
+    if (ghosts_only)
+        for (unsigned q = tid; q < 2 * rows; q += threads) {
+            const unsigned r = q >> 1;
+            const int i = (q & 1) ? g.iM - 1 : 0;
+            if (coords(r, j, k, l))
+                u[(size_t)r * g.iM + i] = mcf_value(mcf_axis(i, g.iM, h, true), square(j, g.jM, false),
+                                                    square(k, g.kM, false), square(l, g.lM, false), t);
         }
-        u[o] = mcf_value(x[0], x[1], x[2], x[3], t);
+    for (unsigned r = tid >> 5; r < rows; r += threads >> 5) {
+        const bool inner = coords(r, j, k, l);
+        if (inner && ghosts_only)
+            continue;
+        const bool fl = ghosts_only && (l == 0 || l == g.lM - 1), fk = ghosts_only && !fl && (k == 0 || k == g.kM - 1),
+                   fj = ghosts_only && !fl && !fk;
+        const double y2 = square(j, g.jM, fj), z2 = square(k, g.kM, fk), w2 = square(l, g.lM, fl);
+        for (int i = lane; i < g.iM; i += 32)
+            u[(size_t)r * g.iM + i] = mcf_value(mcf_coord(i, h), y2, z2, w2, t);
     }
 }
 
@@ -439,52 +462,125 @@ __global__ void k_mcf_field(Geo g, double *u, double h, double t, int ghosts_onl
 // frame; the balls of a frame are processed in their order because each
 // ball's min/max sees the values the earlier balls rescaled.
 
-__global__ void k_rescale_balls(Geo g, double *v, const int *frame_first, const int *frame_count, const double *bx,
-                                const double *by, const double *bz, double R, int l0)
+// The test sqrt(dx^2 + dy^2 + dz^2) <= R is made on the squares: t2 is the
+// largest double whose square root, correctly rounded, is at most R (found on
+// the host), and the square root is monotonic; the squares per axis come from
+// tables of the box, and what only compares runs on the integer pipe.  A
+// frame's balls are a serial chain, and on one SM the FP64 pipe set its pace
+// (414 us for five balls of radius 8 per frame with a square root per voxel and
+// pass): a cluster of RESCALE_CTAS blocks shares a frame's rows and exchanges
+// the extrema through distributed shared memory.
+
+// tables of one ball's box; an axis longer than the table is formed in place
+constexpr int BALL_TABLE = 256;
+constexpr int RESCALE_CTAS = 8;
+
+__device__ __forceinline__ double sq_at(const double *tab, int q, int i0, double c)
 {
-    const int l = l0 + blockIdx.x;
+    if (q < BALL_TABLE)
+        return tab[q];
+    const double d = (i0 + q) - c;
+    return d * d;
+}
+
+// a signed comparison of two keys compares the numbers (-0 below +0); its own inverse
+__device__ inline long long dkey(long long b)
+{
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+
+// minimum of a and maximum of b over the block, in every thread
+__device__ __forceinline__ void block_minmax_keys(long long &a, long long &b)
+{
+    __shared__ long long sa[32], sb[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long x = __shfl_xor_sync(0xffffffffu, a, o), y = __shfl_xor_sync(0xffffffffu, b, o);
+        a = x < a ? x : a;
+        b = y > b ? y : b;
+    }
+    __syncthreads();
+    if (lane == 0) {
+        sa[warp] = a;
+        sb[warp] = b;
+    }
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) {
+        a = sa[w] < a ? sa[w] : a;
+        b = sb[w] > b ? sb[w] : b;
+    }
+}
+
+__global__ void __cluster_dims__(RESCALE_CTAS, 1, 1) __launch_bounds__(256)
+    k_rescale_balls(Geo g, double *v, const int *frame_first, const int *frame_count, const double *bx,
+                    const double *by, const double *bz, double R, double t2, int l0)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ double tx[BALL_TABLE], ty[BALL_TABLE], tz[BALL_TABLE];
+    __shared__ long long ext[2][RESCALE_CTAS][2]; // per parity of the ball: every block's extrema
+    const int l = l0 + blockIdx.x / RESCALE_CTAS, rank = (int)cluster.block_rank();
     const int first = frame_first[l], count = frame_count[l];
+    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) * RESCALE_CTAS;
+    const int warp = (threadIdx.x >> 5) * RESCALE_CTAS + rank;
+    const long long t2b = __double_as_longlong(t2);
     for (int c = 0; c < count; ++c) {
         const double cx = bx[first + c], cy = by[first + c], cz = bz[first + c];
-        const int k0 = (int)(cz - R - 0.5), k1 = (int)(cz + R + 0.5);
-        const int j0 = (int)(cy - R - 0.5), j1 = (int)(cy + R + 0.5);
-        const int i0 = (int)(cx - R - 0.5), i1 = (int)(cx + R + 0.5);
-        const int ni = i1 - i0 + 1, nj = j1 - j0 + 1, nk = k1 - k0 + 1;
-        const long long cnt = (long long)ni * nj * nk;
-        double mn = 100000, mx = 0;
-        for (long long t = threadIdx.x; t < cnt; t += blockDim.x) {
-            const int i = i0 + (int)(t % ni), j = j0 + (int)((t / ni) % nj), k = k0 + (int)(t / ((long long)ni * nj));
-            const double dx = i - cx, dy = j - cy, dz = k - cz;
-            if (sqrt((dx * dx) + (dy * dy) + (dz * dz)) <= R) {
-                const double val = v[nat_index(g, i, j, k, l)];
-                mn = val < mn ? val : mn;
-                mx = val > mx ? val : mx;
-            }
-        }
-        mn = block_min(mn);
-        mx = block_max(mx);
-        __shared__ double qo[2];
-        if (threadIdx.x == 0) {
-            // ball values never exceed the reference's starting bounds in a
-            // meaningful run; keep its initial values 100000 / 0 exactly
-            const double lo = mn < 100000 ? mn : 100000, hi = mx > 0 ? mx : 0;
-            const double quot = 1. / (hi - lo);
-            qo[0] = quot;
-            qo[1] = lo * quot;
+        const int k0 = (int)(cz - R - 0.5), j0 = (int)(cy - R - 0.5), i0 = (int)(cx - R - 0.5);
+        const int nk = (int)(cz + R + 0.5) - k0 + 1, nj = (int)(cy + R + 0.5) - j0 + 1,
+                  ni = (int)(cx + R + 0.5) - i0 + 1;
+        const int most = max(ni, max(nj, nk)) < BALL_TABLE ? max(ni, max(nj, nk)) : BALL_TABLE;
+        for (int q = threadIdx.x; q < most; q += blockDim.x) {
+            const double dx = (i0 + q) - cx, dy = (j0 + q) - cy, dz = (k0 + q) - cz;
+            tx[q] = dx * dx;
+            ty[q] = dy * dy;
+            tz[q] = dz * dz;
         }
         __syncthreads();
-        const double quot = qo[0], off = qo[1];
-        for (long long t = threadIdx.x; t < cnt; t += blockDim.x) {
-            const int i = i0 + (int)(t % ni), j = j0 + (int)((t / ni) % nj), k = k0 + (int)(t / ((long long)ni * nj));
-            const double dx = i - cx, dy = j - cy, dz = k - cz;
-            if (sqrt((dx * dx) + (dy * dy) + (dz * dz)) <= R) {
-                const long long o = nat_index(g, i, j, k, l);
-                const double nv = (quot * v[o]) - off;
-                if (c == 0 || v[o] < nv)
-                    v[o] = nv;
+        // a warp of the cluster per row of the box; d2 <= t2 as a comparison of
+        // bit patterns (d2 >= +0 or NaN; a negative or NaN t2 admits nothing)
+        auto rows = [&](auto &&body) {
+            if (!(t2 >= 0.0))
+                return;
+            for (int r = warp; r < nj * nk; r += nw) {
+                const int kk = r / nj, jj = r - kk * nj;
+                const double y2 = sq_at(ty, jj, j0, cy), z2 = sq_at(tz, kk, k0, cz);
+                double *row = v + nat_index(g, i0, j0 + jj, k0 + kk, l);
+                for (int ii = lane; ii < ni; ii += 32)
+                    if (__double_as_longlong((sq_at(tx, ii, i0, cx) + y2) + z2) <= t2b)
+                        body(row + ii);
             }
+        };
+        // the reference's starting bounds 100000 and 0; a NaN changes neither
+        long long mn = dkey(__double_as_longlong(100000.0)), mx = dkey(__double_as_longlong(0.0));
+        rows([&](double *p) {
+            const long long b = __double_as_longlong(__ldcg(p));
+            if ((b & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL) {
+                const long long k = dkey(b);
+                mn = k < mn ? k : mn;
+                mx = k > mx ? k : mx;
+            }
+        });
+        block_minmax_keys(mn, mx);
+        if (threadIdx.x < RESCALE_CTAS) {
+            long long(*to)[2] = cluster.map_shared_rank(ext[c & 1], threadIdx.x);
+            to[rank][0] = mn;
+            to[rank][1] = mx;
         }
-        __syncthreads();
+        cluster.sync();
+        for (int q = 0; q < RESCALE_CTAS; ++q) {
+            mn = ext[c & 1][q][0] < mn ? ext[c & 1][q][0] : mn;
+            mx = ext[c & 1][q][1] > mx ? ext[c & 1][q][1] : mx;
+        }
+        const double lo = __longlong_as_double(dkey(mn)), hi = __longlong_as_double(dkey(mx));
+        const double quot = 1. / (hi - lo), off = lo * quot;
+        rows([&](double *p) {
+            const double val = __ldcg(p), nv = (quot * val) - off;
+            if (c == 0 || val < nv)
+                *p = nv;
+        });
+        cluster.sync(); // the next ball may cover the same voxels
     }
 }
 
@@ -655,13 +751,6 @@ __global__ void k_mask_zero(Geo g, double *v, const double *Mmask, int l_off)
 
 // ---------------------------------------------------------------------------
 // threshold to mask (segmentation4D_mpi.c:1470-1478)
-
-// ordered 64-bit keys of doubles: a signed comparison of two keys compares the
-// numbers (-0 below +0); the map is its own inverse.  NaN is skipped.
-__device__ inline long long dkey(long long b)
-{
-    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
 
 #define MINMAX_BLOCKS 2048
 // interior min and max of u per block, as (min, max) pairs in partial; a
@@ -872,7 +961,8 @@ void launch_mass(const Geo &g, const double *a, double h4, double *partial, int 
 
 void launch_mcf_field(const Geo &g, double *u, double h, double t, int ghosts_only, cudaStream_t st)
 {
-    k_mcf_field<<<1024, 256, 0, st>>>(g, u, h, t, ghosts_only);
+    const long long warps = (long long)g.jM * g.kM * g.lM;
+    k_mcf_field<<<(unsigned)(warps < 8 * 1216 ? (warps + 7) / 8 : 1216), 256, 0, st>>>(g, u, h, t, ghosts_only);
 }
 
 void launch_rescale_balls(const Geo &g, double *v, const int *frame_first, const int *frame_count, const double *bx,
@@ -881,11 +971,28 @@ void launch_rescale_balls(const Geo &g, double *v, const int *frame_first, const
     launch_rescale_balls_range(g, v, frame_first, frame_count, bx, by, bz, R, 1, g.lM - 1, st);
 }
 
+// the largest double t with sqrt(t) <= R (both rounded to nearest); negative
+// or NaN where there is none, which no square is at most
+static double largest_square(double R)
+{
+    if (!(R >= 0.0) || isinf(R))
+        return R;
+    double t = R * R;
+    if (isinf(t))
+        t = DBL_MAX;
+    while (sqrt(t) > R)
+        t = nextafter(t, -1.0);
+    while (t < DBL_MAX && sqrt(nextafter(t, HUGE_VAL)) <= R)
+        t = nextafter(t, HUGE_VAL);
+    return t;
+}
+
 void launch_rescale_balls_range(const Geo &g, double *v, const int *frame_first, const int *frame_count,
                                 const double *bx, const double *by, const double *bz, double R, int l0, int l1,
                                 cudaStream_t st)
 {
-    k_rescale_balls<<<l1 - l0, 256, 0, st>>>(g, v, frame_first, frame_count, bx, by, bz, R, l0);
+    k_rescale_balls<<<(l1 - l0) * RESCALE_CTAS, 256, 0, st>>>(g, v, frame_first, frame_count, bx, by, bz, R,
+                                                              largest_square(R), l0);
 }
 
 void launch_mask_zero(const Geo &g, double *v, const double *Mmask, cudaStream_t st)

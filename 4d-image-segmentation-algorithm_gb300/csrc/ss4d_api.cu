@@ -506,10 +506,11 @@ static ss4d_status ensure_split(ss4d_solver *s, int mixed)
         s->sb.dB = d3 + 2 * cs;
         s->sb.r32[0] = r2;
         s->sb.r32[1] = r2 + cs;
-        double *fd = nullptr; // float-float forward differences, 4 axes, natural layout
-        CKS(dmalloc(s, (void **)&fd, sizeof(double) * 4 * (size_t)s->geo.n));
+        double *fd = nullptr; // float-float forward differences, 4 axes, folded in k
+        const size_t fold = 2 * fold_units(s->geo);
+        CKS(dmalloc(s, (void **)&fd, sizeof(double) * 4 * fold));
         for (int d = 0; d < 4; ++d)
-            s->sb.fd[d] = fd + (size_t)d * s->geo.n;
+            s->sb.fd[d] = fd + (size_t)d * fold;
         double *rp = nullptr; // the first refinement pass's residual, per colour (split layout)
         CKS(dmalloc(s, (void **)&rp, sizeof(double) * 2 * cs));
         CK(cudaMemsetAsync(rp, 0, sizeof(double) * 2 * cs, s->stream));

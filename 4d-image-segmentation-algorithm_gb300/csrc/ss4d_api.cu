@@ -708,7 +708,7 @@ static void assemble(ss4d_solver *s, const ss4d_params *p, const double *d_u, CP
         launch_assemble_ff(s->geo, s->sp, d_u, gi, has_g, *p, s->sb, pack, s->sm_count, s->stream, pre, s->asm_kblock);
         s->launches += 3;
     } else {
-        launch_assemble(s->geo, s->sp, d_u, gi, has_g, *p, s->sb, 0, s->stream);
+        launch_assemble(s->geo, s->sp, d_u, gi, has_g, *p, s->sb, 0, s->sm_count, s->stream);
         s->launches += 2;
     }
 }
@@ -1679,7 +1679,7 @@ extern "C" ss4d_status ss4d_seg_time_step_host(ss4d_solver *s, const ss4d_params
         }
     }
     if (!mixed) {
-        launch_assemble(g, s->sp, d_u, gi, 1, *p, s->sb, 0, s->stream);
+        launch_assemble(g, s->sp, d_u, gi, 1, *p, s->sb, 0, s->sm_count, s->stream);
         s->launches += 2;
     }
     CKS(last_launch());

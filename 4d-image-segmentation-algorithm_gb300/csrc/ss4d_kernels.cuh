@@ -148,7 +148,7 @@ struct SweepCfg {
 SweepCfg make_sweep_cfg(const Geo &g, const Split &s, int sm_count, int kb);
 
 void launch_assemble(const Geo &g, const Split &s, const double *u, CPtrs8 gin, int has_g, const ss4d_params &p,
-                     SplitBufs b, int want32, cudaStream_t st);
+                     SplitBufs b, int want32, int sm_count, cudaStream_t st);
 void launch_pack(const Geo &g, const Split &s, const double *u, const double *prev, SplitBufs b, cudaStream_t st);
 // mixed form: the same coefficient records from float-float arithmetic (3
 // kernels); with pack the first of them also makes launch_pack's copies of u

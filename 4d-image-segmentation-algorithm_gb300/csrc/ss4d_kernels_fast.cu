@@ -42,12 +42,13 @@ namespace ss4d {
 // FP64 runs at 1/68 of the FP32 rate on GB300, so these passes are bounded
 // by the FP64 pipe, not by HBM.
 
-// 1/sqrt(x), x > 0: FP32 seed + one Newton step
+// 1/sqrt(x), x > 0: FP32 seed + one Newton step (y0 / 2 is exact in FP32 too)
 __device__ __forceinline__ double rsqrt_nr(double x)
 {
-    const double y0 = f2d_bits(rsqrtf(d2f_bits(x)));
+    const float f0 = rsqrtf(d2f_bits(x));
+    const double y0 = f2d_bits(f0);
     const double e = fma(-x * y0, y0, 1.0); // 1 - x y0^2
-    return fma(0.5 * y0, e, y0);
+    return fma(f2d_bits(0.5f * f0), e, y0);
 }
 
 // 1/x, x >= 1: FP32 seed + one Newton step
@@ -78,84 +79,214 @@ __device__ __forceinline__ void store_coef(double *cf, uint4 *cq, float *cs, lon
     }
 }
 
-// Threads cover voxels v with every index in [0, n_a]; face d of v (between
-// v and v + e_d) is evaluated when v is interior on the other three axes, so
-// index 0 on axis d yields the face the interior voxel 1 sees backwards.
-__global__ void __launch_bounds__(256) k_faces(Geo g, const double *__restrict__ u, CPtrs8 gin, int has_g, double ih,
-                                               double iq2, double eps2, SplitBufs b)
+// The face between v and v + e_d from its normal difference n = u(v + e_d) -
+// u(v) and its three tangential terms t (the sum of the central differences
+// at v and v + e_d along the other axes): |grad u|_eps and g / |grad u|_eps.
+struct FaceK {
+    double ih, iq2, eps2; // 1/h, 1/(4h)^2
+};
+template <bool UNIT>
+__device__ __forceinline__ void face64(const FaceK &K, double n, double t0, double t1, double t2, double gv,
+                                       double *fn, double *fq)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z % (g.nz + 1), l = blockIdx.z / (g.nz + 1);
-    if (i > g.nx || j > g.ny)
-        return;
-    const int idx[4] = {i, j, k, l};
-    const long long o = nat_index(g, i, j, k, l);
+    const double cn = UNIT ? n : n * K.ih; // h == 1: the product is n itself
+    const double tt = fma(t2, t2, fma(t1, t1, t0 * t0));
+    const double s2 = fma(tt, K.iq2, fma(cn, cn, K.eps2));
+    const double y = rsqrt_nr(s2);
+    __stcs(fn, s2 * y);
+    __stcs(fq, gv * y);
+}
+
+// Tile and march of k_faces (make_face_plan).
+struct FacePlan {
+    int TX, KC;           // tile width (TX x 256/TX voxels), planes per block
+    int nti, ntj, nkc;    // tiles along i and j, chunks of planes
+    unsigned main, edge;  // blocks of interior voxels; the rest take boundary faces
+    unsigned nb[4];       // boundary faces per axis
+};
+
+// central difference of u at v along a stride
+__device__ __forceinline__ double cd64(const double *__restrict__ u, long long v, long long sa)
+{
+    return __ldg(u + v + sa) - __ldg(u + v - sa);
+}
+
+// the face between the ghost v and v + e_D, everything from u
+template <int D, bool UNIT>
+__device__ __forceinline__ void edge_face64(const Geo &g, const double *__restrict__ u, const CPtrs8 &gin, int has_g,
+                                            const FaceK &K, const SplitBufs &b, long long v)
+{
     const long long st[4] = {1, g.sy, g.sz, g.sw};
-    const double uc = u[o];
-    // central differences at v along each axis where v is interior
-    double D[4];
+    const long long nb = v + st[D];
+    double t[3];
+    int q = 0;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
-        D[a] = idx[a] >= 1 ? u[o + st[a]] - u[o - st[a]] : 0.0;
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        bool ok = true;
+        if (a != D)
+            t[q++] = cd64(u, nb, st[a]) + cd64(u, v, st[a]);
+    face64<UNIT>(K, __ldg(u + nb) - __ldg(u + v), t[0], t[1], t[2], has_g ? __ldg(gin.p[2 * D + 1] + nb) : 1.0,
+                 b.fn[D] + v, b.fq[D] + v);
+}
+
+// fn, fq of every face between v and v + e_d, v with index >= 0 along d and
+// interior along the others.  Main blocks take the faces of interior voxels:
+// a tile of TX x TY voxels (i, j) marches over KC planes, so that each
+// voxel's four central differences are formed once (its neighbours' towards
+// +i and +j come through shared memory, plus a halo column and row, those
+// towards +k one plane ahead, those at +l directly).  The other blocks take
+// the faces between a ghost and the first voxel, one per thread.
+//
+// Bound by the FP64 pipe (2 lanes per clock and SM): about 66 FP64
+// instructions per voxel instead of 84 with every difference formed at each
+// of its faces, no lanes spent on ghosts (a row of 129 took five warps) and no rows
+// padded to a power of two: 6.4 -> 4.0 ms at 128^3 x 16, 93 -> 39 us at 32^3 x 8.
+template <bool UNIT>
+__global__ void __launch_bounds__(256, 3) k_faces(Geo g, const double *__restrict__ u, CPtrs8 gin, int has_g, FaceK K,
+                                                  FacePlan P, SplitBufs b)
+{
+    if (blockIdx.x >= P.main) {
+        // boundary faces, all lanes busy: flat over the four sets
+        for (unsigned q = (blockIdx.x - P.main) * blockDim.x + threadIdx.x;; q += P.edge * blockDim.x) {
+            unsigned r = q;
+            if (r < P.nb[0]) { // i = 0: (j, k, l)
+                const int j = 1 + (int)(r % g.ny);
+                r /= g.ny;
+                edge_face64<0, UNIT>(g, u, gin, has_g, K, b, nat_index(g, 0, j, 1 + (int)(r % g.nz), 1 + (int)(r / g.nz)));
+                continue;
+            }
+            if ((r -= P.nb[0]) < P.nb[1]) { // j = 0: (i, k, l)
+                const int i = 1 + (int)(r % g.nx);
+                r /= g.nx;
+                edge_face64<1, UNIT>(g, u, gin, has_g, K, b, nat_index(g, i, 0, 1 + (int)(r % g.nz), 1 + (int)(r / g.nz)));
+                continue;
+            }
+            if ((r -= P.nb[1]) < P.nb[2]) { // k = 0: (i, j, l)
+                const int i = 1 + (int)(r % g.nx);
+                r /= g.nx;
+                edge_face64<2, UNIT>(g, u, gin, has_g, K, b, nat_index(g, i, 1 + (int)(r % g.ny), 0, 1 + (int)(r / g.ny)));
+                continue;
+            }
+            if ((r -= P.nb[2]) < P.nb[3]) { // l = 0: (i, j, k)
+                const int i = 1 + (int)(r % g.nx);
+                r /= g.nx;
+                edge_face64<3, UNIT>(g, u, gin, has_g, K, b, nat_index(g, i, 1 + (int)(r % g.ny), 1 + (int)(r / g.ny), 0));
+                continue;
+            }
+            return;
+        }
+    }
+    // tiles fastest, then frames, chunks of planes slowest
+    unsigned r = blockIdx.x;
+    const int ti = (int)(r % P.nti);
+    r /= P.nti;
+    const int tj = (int)(r % P.ntj);
+    r /= P.ntj;
+    const int l = 1 + (int)(r % g.nt), kc = (int)(r / g.nt);
+    const int TX = P.TX, TY = 256 / TX, pitch = TX + 1;
+    const int tx = threadIdx.x & (TX - 1), ty = threadIdx.x / TX;
+    const int i0 = 1 + ti * TX, j0 = 1 + tj * TY, i = i0 + tx, j = j0 + ty;
+    const int k0 = 1 + kc * P.KC, k1 = min(k0 + P.KC - 1, g.nz);
+    __shared__ double sD[4][33 * 9]; // (TY + 1) x (TX + 1) at most 33 x 9 = 9 x 33
+    const bool in = i <= g.nx && j <= g.ny;
+    // ghosts inside the tile: the differences their interior neighbours read
+    const bool gcol = i == g.nx + 1 && j <= g.ny, grow = j == g.ny + 1 && i <= g.nx;
+    const long long st[4] = {1, g.sy, g.sz, g.sw};
+    long long v = nat_index(g, i, j, k0, l);
+    double uc = 0.0, D[4] = {0.0, 0.0, 0.0, 0.0};
+    if (in) {
+        uc = __ldg(u + v);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
-            if (a != d && idx[a] < 1)
-                ok = false;
-        if (!ok)
-            continue;
-        const long long nb = o + st[d];
-        const double cn = (u[nb] - uc) * ih;
-        double tt = 0.0;
+            D[a] = cd64(u, v, st[a]);
+    }
+    const int here = ty * pitch + tx;
+    // the halo's voxels: the column i0 + TX by the threads 32 .. 32 + TY - 1,
+    // the row j0 + TY by the threads 0 .. TX - 1 (both in one warp each, which
+    // TX and TY allow: 8 .. 32)
+    const int hc = (int)threadIdx.x - 32;
+    const bool col = hc >= 0 && hc < TY && i0 + TX <= g.nx + 1 && j0 + hc <= g.ny;
+    const bool row = (int)threadIdx.x < TX && j0 + TY <= g.ny + 1 && i0 + (int)threadIdx.x <= g.nx;
+    long long vh = col ? nat_index(g, i0 + TX, j0 + hc, k0, l) : row ? nat_index(g, i0 + (int)threadIdx.x, j0 + TY, k0, l) : 0;
+    const int hslot = col ? hc * pitch + TX : TY * pitch + (int)threadIdx.x;
+    for (int k = k0; k <= k1; ++k, v += g.sz, vh += g.sz) {
+        __syncthreads();
+        if (in) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            if (a == d)
-                continue;
-            const double t = (u[nb + st[a]] - u[nb - st[a]]) + D[a];
-            tt = fma(t, t, tt);
+            for (int a = 0; a < 4; ++a)
+                sD[a][here] = D[a];
+        } else if (gcol || grow) {
+            sD[gcol ? 1 : 0][here] = cd64(u, v, gcol ? st[1] : st[0]);
+            sD[2][here] = cd64(u, v, st[2]);
+            sD[3][here] = cd64(u, v, st[3]);
         }
-        const double s2 = fma(tt, iq2, fma(cn, cn, eps2));
-        const double y = rsqrt_nr(s2);
-        double gv = 1.0;
-        if (has_g)
-            gv = idx[d] >= 1 ? __ldg(gin.p[2 * d] + o) : __ldg(gin.p[2 * d + 1] + nb);
-        __stcs(b.fn[d] + o, s2 * y);
-        __stcs(b.fq[d] + o, gv * y);
+        if (col || row) {
+            sD[col ? 1 : 0][hslot] = cd64(u, vh, col ? st[1] : st[0]);
+            sD[2][hslot] = cd64(u, vh, st[2]);
+            sD[3][hslot] = cd64(u, vh, st[3]);
+        }
+        __syncthreads();
+        if (!in)
+            continue;
+        const int e = here + 1, n = here + pitch; // v + e_i, v + e_j
+        const double ge = has_g ? __ldg(gin.p[0] + v) : 1.0, gn = has_g ? __ldg(gin.p[2] + v) : 1.0,
+                     gt = has_g ? __ldg(gin.p[4] + v) : 1.0, gf = has_g ? __ldg(gin.p[6] + v) : 1.0;
+        face64<UNIT>(K, __ldg(u + v + st[0]) - uc, sD[1][e] + D[1], sD[2][e] + D[2], sD[3][e] + D[3], ge, b.fn[0] + v,
+                     b.fq[0] + v);
+        face64<UNIT>(K, __ldg(u + v + st[1]) - uc, sD[0][n] + D[0], sD[2][n] + D[2], sD[3][n] + D[3], gn, b.fn[1] + v,
+                     b.fq[1] + v);
+        {
+            const long long w = v + st[3];
+            face64<UNIT>(K, __ldg(u + w) - uc, cd64(u, w, st[0]) + D[0], cd64(u, w, st[1]) + D[1],
+                         cd64(u, w, st[2]) + D[2], gf, b.fn[3] + v, b.fq[3] + v);
+        }
+        const long long w = v + st[2]; // the plane ahead (a ghost plane at k = nz: no D_k there)
+        const double un = __ldg(u + w);
+        const double n0 = cd64(u, w, st[0]), n1 = cd64(u, w, st[1]), n3 = cd64(u, w, st[3]);
+        face64<UNIT>(K, un - uc, n0 + D[0], n1 + D[1], n3 + D[3], gt, b.fn[2] + v, b.fq[2] + v);
+        uc = un;
+        D[0] = n0;
+        D[1] = n1;
+        D[2] = k < k1 ? cd64(u, w, st[2]) : 0.0;
+        D[3] = n3;
     }
 }
 
-__global__ void __launch_bounds__(256) k_voxel_coef(Geo g, Split sp, double eps2, double c, double omega, SplitBufs b,
-                                                    int want32)
+// flat over the interior voxels: no lane of this FP64-bound kernel is lost to
+// the ends of rows
+__global__ void __launch_bounds__(256) k_voxel_coef(Geo g, Split sp, FastDiv dx, FastDiv dy, FastDiv dz, double eps2,
+                                                    double c, double omega, SplitBufs b, int want32)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = 1 + blockIdx.z % g.nz, l = 1 + blockIdx.z / g.nz;
-    if (i > g.nx || j > g.ny)
-        return;
-    const long long o = nat_index(g, i, j, k, l);
-    const long long st[4] = {1, g.sy, g.sz, g.sw};
-    double q[8], sum = 0.0;
+    const unsigned n = (unsigned)g.nint;
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) {
+        unsigned r = fdiv(w, dx);
+        const int i = 1 + (int)(w - r * dx.d);
+        unsigned h = fdiv(r, dy);
+        const int j = 1 + (int)(r - h * dy.d);
+        r = h;
+        h = fdiv(r, dz);
+        const int k = 1 + (int)(r - h * dz.d), l = 1 + (int)h;
+        const long long o = nat_index(g, i, j, k, l);
+        const long long st[4] = {1, g.sy, g.sz, g.sw};
+        double q[8], sum = 0.0;
 #pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        sum += __ldg(b.fn[d] + o) + __ldg(b.fn[d] + o - st[d]);
-        q[2 * d] = __ldg(b.fq[d] + o);
-        q[2 * d + 1] = __ldg(b.fq[d] + o - st[d]);
-    }
-    const double x = fma(sum * sum, 1.0 / 64.0, eps2); // mean^2 + eps2
-    const double cv = c * (x * rsqrt_nr(x));           // c * vc
-    const int col = (i + j + k + l) & 1;
-    double *cf = pick(b.coef, col);
-    double ac[8], diag = 1.0;
+        for (int d = 0; d < 4; ++d) {
+            sum += __ldg(b.fn[d] + o) + __ldg(b.fn[d] + o - st[d]);
+            q[2 * d] = __ldg(b.fq[d] + o);
+            q[2 * d + 1] = __ldg(b.fq[d] + o - st[d]);
+        }
+        const double x = fma(sum * sum, 1.0 / 64.0, eps2); // mean^2 + eps2
+        const double cv = c * (x * rsqrt_nr(x));           // c * vc
+        const int col = (i + j + k + l) & 1;
+        double *cf = pick(b.coef, col);
+        double ac[8], diag = 1.0;
 #pragma unroll
-    for (int f = 0; f < 8; ++f) {
-        ac[f] = cv * q[f];
-        diag += ac[f];
+        for (int f = 0; f < 8; ++f) {
+            ac[f] = cv * q[f];
+            diag += ac[f];
+        }
+        store_coef(cf, pick(b.coefq, col), pick(b.coefs, col), coef_index(g, sp, i, j, k, l), ac, diag,
+                   omega * rcp_nr(diag), want32);
     }
-    store_coef(cf, pick(b.coefq, col), pick(b.coefs, col), coef_index(g, sp, i, j, k, l), ac, diag,
-               omega * rcp_nr(diag), want32);
 }
 
 // given natural coefficient arrays e..bw (the reference's layout) -> split
@@ -595,18 +726,56 @@ static inline void interior_grid(const Geo &g, dim3 &grid, dim3 &block)
     grid = dim3((g.nx + bx - 1) / bx, (g.ny + by - 1) / by, g.nz * g.nt);
 }
 
-void launch_assemble(const Geo &g, const Split &s, const double *u, CPtrs8 gin, int has_g, const ss4d_params &p,
-                     SplitBufs b, int want32, cudaStream_t st)
+// The tile width that wastes the fewest warps on a row's end (a warp is TX
+// wide and 32/TX rows high; one wholly outside costs nothing), the wider
+// one of equals; planes per block so that eight blocks per SM are there to
+// share, at most 16 (a block's first plane costs its differences extra).
+static FacePlan make_face_plan(const Geo &g, int sm_count)
 {
-    const int bx = g.nx + 1 >= 128 ? 128 : (g.nx + 1 >= 64 ? 64 : 32);
-    const int by = 256 / bx;
-    dim3 fb(bx, by, 1), fg((g.nx + 1 + bx - 1) / bx, (g.ny + 1 + by - 1) / by, (g.nz + 1) * (g.nt + 1));
-    const double ih = 1.0 / p.h, iq = 1.0 / (4.0 * p.h);
-    k_faces<<<fg, fb, 0, st>>>(g, u, gin, has_g, ih, iq * iq, p.eps2, b);
-    dim3 gr, bl;
-    interior_grid(g, gr, bl);
+    FacePlan P;
+    long long best = 0;
+    P.TX = 0;
+    for (int tx = 32; tx >= 8; tx >>= 1) {
+        const int wr = 32 / tx;
+        const long long warps = (long long)((g.nx + tx - 1) / tx) * ((g.ny + wr - 1) / wr);
+        if (!P.TX || warps < best) {
+            P.TX = tx;
+            best = warps;
+        }
+    }
+    const int TY = 256 / P.TX;
+    P.nti = (g.nx + P.TX - 1) / P.TX;
+    P.ntj = (g.ny + TY - 1) / TY;
+    const long long cols = (long long)P.nti * P.ntj * g.nt;
+    long long kc = cols * g.nz / (8LL * sm_count);
+    P.KC = (int)(kc < 1 ? 1 : (kc > 16 ? 16 : kc));
+    P.nkc = (g.nz + P.KC - 1) / P.KC;
+    P.main = (unsigned)(cols * P.nkc);
+    P.nb[0] = (unsigned)(g.ny * g.nz * g.nt);
+    P.nb[1] = (unsigned)(g.nx * g.nz * g.nt);
+    P.nb[2] = (unsigned)(g.nx * g.ny * g.nt);
+    P.nb[3] = (unsigned)(g.nx * g.ny * g.nz);
+    const long long faces = (long long)P.nb[0] + P.nb[1] + P.nb[2] + P.nb[3];
+    const long long need = (faces + 255) / 256;
+    P.edge = (unsigned)(need < 4LL * sm_count ? need : 4LL * sm_count);
+    return P;
+}
+
+void launch_assemble(const Geo &g, const Split &s, const double *u, CPtrs8 gin, int has_g, const ss4d_params &p,
+                     SplitBufs b, int want32, int sm_count, cudaStream_t st)
+{
+    const double iq = 1.0 / (4.0 * p.h);
+    const FaceK K = {1.0 / p.h, iq * iq, p.eps2};
+    const FacePlan P = make_face_plan(g, sm_count);
+    if (p.h == 1.0)
+        k_faces<true><<<P.main + P.edge, 256, 0, st>>>(g, u, gin, has_g, K, P, b);
+    else
+        k_faces<false><<<P.main + P.edge, 256, 0, st>>>(g, u, gin, has_g, K, P, b);
     const double c = p.tau / (p.h * p.h);
-    k_voxel_coef<<<gr, bl, 0, st>>>(g, s, p.eps2, c, p.omega_c, b, want32);
+    const long long need = (g.nint + 255) / 256, most = 8LL * sm_count;
+    k_voxel_coef<<<(unsigned)(need < most ? need : most), 256, 0, st>>>(
+        g, s, make_fastdiv((unsigned)g.nx), make_fastdiv((unsigned)g.ny), make_fastdiv((unsigned)g.nz), p.eps2, c,
+        p.omega_c, b, want32);
 }
 
 void launch_pack(const Geo &g, const Split &s, const double *u, const double *prev, SplitBufs b, cudaStream_t st)

@@ -125,6 +125,7 @@ struct ss4d_solver {
     LoopGroup *d_group;
     double *d_loop_parts;
     int loop_blocks[2];  // its grid per form; 0: not known, -1: the graph's loop instead
+    bool loop_ahead[2];  // its form (loop_plan)
     // rescale balls
     int *d_frame_first, *d_frame_count;
     double *d_bx, *d_by, *d_bz;
@@ -931,10 +932,10 @@ static ss4d_status run_split_loop(ss4d_solver *s, const ss4d_params *p, int mixe
 // The loop as one persistent cooperative launch (ss4d_loop.cu) rather than
 // the graph's while loop?  The plain form always: its flat walk of the
 // targets and the missing launches win at every size (a step at 32^3 x 8
-// 886 -> 683 us, 161 x 143 x 61 x 9 15.4 -> 12.7 ms, 256 x 256 x 128 x 8
+// 886 -> 543 us, 161 x 143 x 61 x 9 15.4 -> 12.7 ms, 256 x 256 x 128 x 8
 // 61.0 -> 60.1 ms).  The mixed form up to 9e6 voxels: there the loop's data (about 30
 // bytes per voxel) stays in L2 or near it, and the graph's body costs seven
-// launches an iteration (32^3 x 8 850 -> 453 us, 64 x 64 x 64 x 10 1648 ->
+// launches an iteration (32^3 x 8 850 -> 391 us, 64 x 64 x 64 x 10 1648 ->
 // 1386 us, 131 x 129 x 65 x 8 3.94 -> 3.90 ms); beyond, the launches are lost
 // in the half-sweeps' time and the separate FP32 kernel, at 40 warps per SM
 // instead of 32, streams faster (161 x 143 x 61 x 9 5.53 against 5.58 ms,
@@ -950,15 +951,14 @@ static bool loop_persistent(const ss4d_solver *s, int mixed)
 static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixed, bool *done)
 {
     *done = false;
+    LoopVol V = make_loop_vol(s->geo, s->sp, s->sb);
     if (!s->loop_blocks[mixed]) {
-        const int g = loop_grid(mixed, 1, LOOP_THREADS, s->sm_count);
+        const int g = loop_plan(mixed, V.F, LOOP_THREADS, s->sm_count, &s->loop_ahead[mixed]);
         s->loop_blocks[mixed] = g > 0 ? g : -1;
     }
-    if (s->loop_blocks[mixed] < 0)
+    int grid = s->loop_blocks[mixed];
+    if (grid < 0)
         return SS4D_OK;
-    LoopVol V = make_loop_vol(s->geo, s->sp, s->sb);
-    const long long need = ((long long)(mixed ? V.F.npairs : V.F.ntargets) + LOOP_THREADS - 1) / LOOP_THREADS;
-    int grid = need < s->loop_blocks[mixed] ? (int)need : s->loop_blocks[mixed];
     if (s->max_grid > 0 && grid > s->max_grid)
         grid = s->max_grid;
     share_blocks(&V, 1, grid);
@@ -971,7 +971,7 @@ static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixe
     CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
     const int bodies = mixed ? 4 * (p->maxNoGSIteration + 4) + 16 : p->maxNoGSIteration + 8;
     cudaError_t e = launch_loop(mixed, &V, 1, grid, LOOP_THREADS, s->d_state, s->d_params, s->d_loop_parts,
-                                s->d_group, bodies, s->stream);
+                                s->d_group, bodies, s->loop_ahead[mixed], s->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         s->loop_blocks[mixed] = -1; // from now on the graph's loop

@@ -873,7 +873,7 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
             if (b->withhold_barrier) // arrival counts far below any target: no arrival completes a barrier
                 BCK(cudaMemset2DAsync(&b->d_groups->count, sizeof(LoopGroup), 0x80, sizeof(unsigned), b->n, b->stream));
             BCK(launch_loop(f, b->h_loop, b->n, b->pgrid[f], BLOOP_THREADS, b->d_st, b->d_par, b->d_loop_parts,
-                            b->d_groups, guard_max, b->stream));
+                            b->d_groups, guard_max, false, b->stream));
             persisted = true;
         }
     }

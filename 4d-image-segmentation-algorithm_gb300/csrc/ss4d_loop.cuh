@@ -56,12 +56,15 @@ __device__ __forceinline__ bool group_wait(LoopGroup *gr, unsigned target)
 LoopVol make_loop_vol(const Geo &g, const Split &sp, const SplitBufs &b);
 // co-resident blocks of k_loop with that many threads on the device (0: unknown)
 int loop_grid(int mixed, int nv, int threads, int sm_count);
+// the grid of one volume's k_loop, and whether it is the AHEAD form (0: unknown)
+int loop_plan(int mixed, const FlatIndex &F, int threads, int sm_count, bool *ahead);
 // deals `grid` blocks out to the volumes in proportion to their targets
 // (at least one each; nv <= grid)
 void share_blocks(LoopVol *vols, int nv, int grid);
 // vols (host memory), st, par, groups (zeroed by the caller) per volume;
 // parts 4 doubles per block
 cudaError_t launch_loop(int mixed, const LoopVol *vols, int nv, int grid, int threads, LoopState *st,
-                        const DevParams *par, double *parts, LoopGroup *groups, int max_bodies, cudaStream_t stream);
+                        const DevParams *par, double *parts, LoopGroup *groups, int max_bodies, bool ahead,
+                        cudaStream_t stream);
 
 } // namespace ss4d

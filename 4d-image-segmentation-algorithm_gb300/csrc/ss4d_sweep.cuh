@@ -223,11 +223,14 @@ __device__ __forceinline__ long long tile_coef_index(const Geo &g, const Split &
 
 // One FP64 update of the target at split index s (row phase p, record tq):
 //   r = diag*u - (prev + sum_f c a_f u_f),   dst = u - (omega/diag) r.
-// Returns the pre-update residual r.
+// sweep64_calc only forms it; sweep64_at stores it and returns r.
+struct Sweep64Out {
+    double r, u; // the residual before the update, the updated value
+};
 template <bool LIVE>
-__device__ __forceinline__ double sweep64_at(int p, long long s, long long tq, long long Hy, long long Hz,
-                                             long long Hw, const double *src, double *dst, const double *oth,
-                                             const double *__restrict__ cf, const double *__restrict__ pv)
+__device__ __forceinline__ Sweep64Out sweep64_calc(int p, long long s, long long tq, long long Hy, long long Hz,
+                                                   long long Hw, const double *src, const double *oth,
+                                                   const double *__restrict__ cf, const double *__restrict__ pv)
 {
     const double u0 = LIVE ? __ldcg(src + s) : src[s];
     const double *cv = cf + coef_at(tq, 0, 10); // component f at cv[32 f]
@@ -242,8 +245,16 @@ __device__ __forceinline__ double sweep64_at(int p, long long s, long long tq, l
     const double diag = ld_stream(cv + 256);
     const double winv = ld_stream(cv + 288);
     const double r = fma(diag, u0, -S); // S includes prev
-    dst[s] = fma(-winv, r, u0);
-    return r;
+    return Sweep64Out{r, fma(-winv, r, u0)};
+}
+template <bool LIVE>
+__device__ __forceinline__ double sweep64_at(int p, long long s, long long tq, long long Hy, long long Hz,
+                                             long long Hw, const double *src, double *dst, const double *oth,
+                                             const double *__restrict__ cf, const double *__restrict__ pv)
+{
+    const Sweep64Out o = sweep64_calc<LIVE>(p, s, tq, Hy, Hz, Hw, src, oth, cf, pv);
+    dst[s] = o.u;
+    return o.r;
 }
 
 __device__ __forceinline__ double sweep64_target(const Geo &g, const Split &sp, const TileCoord &tc, int p,
@@ -392,12 +403,14 @@ __device__ __forceinline__ Sweep32Out sweep32_target(const Geo &g, const Split &
 // (a colour array holds fewer than 2^31 elements).  The pair reads its own
 // values, right-hand sides and y/z/w neighbours as 8-byte pairs and shares
 // its index arithmetic; each target's arithmetic is sweep32_target's.
-// Returns acc plus the squared pre-update residuals (first target first).
+struct Pair32Out {
+    float o0, o1, r0, r1; // updated values, residuals before the update
+};
 template <bool LIVE>
-__device__ __forceinline__ float sweep32_pair(int p, unsigned s, unsigned tq, bool two, unsigned Hy, unsigned Hz,
-                                              unsigned Hw, const float *src, float *dst, const float *oth,
-                                              const uint4 *__restrict__ cq, const float *__restrict__ cs,
-                                              const float *__restrict__ rhs, float omega, float acc)
+__device__ __forceinline__ Pair32Out sweep32_pair_calc(int p, unsigned s, unsigned tq, bool two, unsigned Hy,
+                                                       unsigned Hz, unsigned Hw, const float *src, const float *oth,
+                                                       const uint4 *__restrict__ cq, const float *__restrict__ cs,
+                                                       const float *__restrict__ rhs, float omega)
 {
     const float2 u = LIVE ? __ldcg(reinterpret_cast<const float2 *>(src + s)) : *reinterpret_cast<const float2 *>(src + s);
     const float2 rh = __ldcs(reinterpret_cast<const float2 *>(rhs + s));
@@ -418,19 +431,38 @@ __device__ __forceinline__ float sweep32_pair(int p, unsigned s, unsigned tq, bo
     // record order: +x (column s_t - p + 1), -x (s_t - p), +y, -y, +z, -z, +w, -w
     const float nb0[8] = {p ? vx.x : vx.y, p ? ex : vx.x, yp.x, ym.x, zp.x, zm.x, wp.x, wm.x};
     float d0;
-    const float r0 = resid32(w0, sc0, nb0, u.x, rh.x, d0);
-    const float o0 = fmaf(-__fdividef(omega, d0), r0, u.x);
-    acc = fmaf(r0, r0, acc);
+    Pair32Out out;
+    out.r0 = resid32(w0, sc0, nb0, u.x, rh.x, d0);
+    out.o0 = fmaf(-__fdividef(omega, d0), out.r0, u.x);
+    out.r1 = out.o1 = 0.f;
     if (two) {
         const float nb1[8] = {p ? vx.y : ex, p ? vx.x : vx.y, yp.y, ym.y, zp.y, zm.y, wp.y, wm.y};
         float d1;
-        const float r1 = resid32(w1, sc1, nb1, u.y, rh.y, d1);
-        acc = fmaf(r1, r1, acc);
-        *reinterpret_cast<float2 *>(dst + s) = make_float2(o0, fmaf(-__fdividef(omega, d1), r1, u.y));
+        out.r1 = resid32(w1, sc1, nb1, u.y, rh.y, d1);
+        out.o1 = fmaf(-__fdividef(omega, d1), out.r1, u.y);
+    }
+    return out;
+}
+// stores a pair; acc plus its squared residuals, the first target's first
+__device__ __forceinline__ float sweep32_pair_put(const Pair32Out &o, unsigned s, bool two, float *dst, float acc)
+{
+    acc = fmaf(o.r0, o.r0, acc);
+    if (two) {
+        acc = fmaf(o.r1, o.r1, acc);
+        *reinterpret_cast<float2 *>(dst + s) = make_float2(o.o0, o.o1);
     } else {
-        dst[s] = o0;
+        dst[s] = o.o0;
     }
     return acc;
+}
+template <bool LIVE>
+__device__ __forceinline__ float sweep32_pair(int p, unsigned s, unsigned tq, bool two, unsigned Hy, unsigned Hz,
+                                              unsigned Hw, const float *src, float *dst, const float *oth,
+                                              const uint4 *__restrict__ cq, const float *__restrict__ cs,
+                                              const float *__restrict__ rhs, float omega, float acc)
+{
+    return sweep32_pair_put(sweep32_pair_calc<LIVE>(p, s, tq, two, Hy, Hz, Hw, src, oth, cq, cs, rhs, omega), s, two, dst,
+                            acc);
 }
 
 // ---------------------------------------------------------------------------

@@ -13,7 +13,10 @@ pytestmark = pytest.mark.gpu
 # two rounds of 304 blocks of 512 threads are 311,296 pairs (mixed) or
 # columns (FP64): the first of each couple fills them, the second goes on
 SIZES = [(1, 1, 1, 1), (2, 1, 3, 2), (3, 5, 1, 7), (33, 9, 14, 7), (47, 31, 23, 5), (64, 4, 4, 2),
-         (64, 32, 38, 16), (65, 32, 38, 16), (64, 32, 38, 8), (65, 32, 38, 8)]
+         (64, 32, 38, 16), (65, 32, 38, 16), (64, 32, 38, 8), (65, 32, 38, 8),
+         # one round and three rounds of the form whose last warp has no
+         # targets (304 blocks of 480 columns, 152 of 480 pairs), and just over
+         (64, 38, 12, 10), (65, 38, 12, 10), (64, 38, 36, 10), (65, 38, 36, 10)]
 
 
 def _volume(ss4d, torch, dims, seed, **over):

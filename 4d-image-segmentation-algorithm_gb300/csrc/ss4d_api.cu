@@ -2045,6 +2045,11 @@ int ss4d::solver_sm_count(const ss4d_solver *s)
     return s->sm_count;
 }
 
+void ss4d::solver_set_stream(ss4d_solver *s, cudaStream_t stream)
+{
+    s->stream = stream;
+}
+
 ss4d_status ss4d::solver_view(ss4d_solver *s, SolverView *out)
 {
     REQ(s && out, "NULL argument");

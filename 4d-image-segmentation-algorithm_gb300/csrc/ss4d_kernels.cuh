@@ -278,5 +278,8 @@ ss4d_status solver_project_start(ss4d_solver *s, int pre, LoopState *d_state);
 // device time of `iters` (black + red) FP64 sweep pairs with the current shape
 ss4d_status solver_time_sweeps(ss4d_solver *s, const ss4d_params *p, int iters, float *ms);
 int solver_sm_count(const ss4d_solver *s);
+// what the handle launches from now on goes to `stream` (the caller orders it
+// against what went before)
+void solver_set_stream(ss4d_solver *s, cudaStream_t stream);
 
 } // namespace ss4d

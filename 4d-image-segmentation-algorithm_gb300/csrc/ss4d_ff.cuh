@@ -114,9 +114,20 @@ __device__ __forceinline__ ff ff_from_pos_d(double d)
     return ff_make(h, l);
 }
 
+// h + l rounded to double.  An FP64 addition, of which an SM makes two a
+// clock, bounded the coefficient kernel (nine per voxel beside the residual's
+// nine multiply-adds); a positive h from 2^-75 up whose low part is at most
+// half a unit takes integer operations instead: h's bits as a double, whose
+// last 29 mantissa bits are zero, plus l in units of the last one, rounded to
+// an integer (to even, and h's part is even): the double the addition gives.
+// Below a power of two the units halve: that case is added in FP64.
 __device__ __forceinline__ double ff_to_d(ff a)
 {
-    return f2d_bits(a.h) + f2d_bits(a.l);
+    const unsigned h = __float_as_uint(a.h), e = h & 0x7F800000u;
+    const float l = a.l * __uint_as_float((306u << 23) - e); // l 2^(52 - exponent of h)
+    if (h - (52u << 23) >= (255u - 52u) << 23 || !(fabsf(l) <= 0x1p28f) || (h == e && l < 0.f))
+        return f2d_bits(a.h) + f2d_bits(a.l);
+    return __longlong_as_double((((long long)h << 29) + (896LL << 52)) + __float2int_rn(l));
 }
 
 // 1/sqrt(x), x > 0 and normal: FP32 seed y0 (relative error below 2^-21),

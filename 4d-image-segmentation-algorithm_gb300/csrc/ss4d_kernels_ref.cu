@@ -193,9 +193,10 @@ __device__ inline double face_sq(const double *v, long long c, long long nb, con
 }
 
 // face_sq of the face between o and o + st[d], in the reference's expression
-// order.  POW2: h is a power of two, so x / h == x * (1/h) and x / (4h) ==
-// x * (1/(4h)) exactly (one rounding of the same real number); otherwise the
-// divisions by h and 4h go through div_by_const (ih, iq: its reciprocals).
+// order: through div_by_const (ih, iq: the reciprocals of h and q = 4h), or,
+// POW2, times q^2 with h a power of two: the divisions then scale exactly, so
+// the squares and their sum are formed unscaled (the normal difference times
+// 4) and the caller scales once.
 template <bool POW2, int D>
 __device__ inline double face_sq_plus(const double *v, long long o, const long long st[4], double h, double q,
                                       double ih, double iq)
@@ -206,10 +207,10 @@ __device__ inline double face_sq_plus(const double *v, long long o, const long l
     for (int a = 0; a < 4; ++a) {
         if (a == D) {
             const double t = v[nb] - v[o];
-            comp[a] = POW2 ? t * ih : div_by_const(t, h, ih);
+            comp[a] = POW2 ? t * 4.0 : div_by_const(t, h, ih);
         } else {
             const double t = (v[nb + st[a]] + v[o + st[a]]) - (v[nb - st[a]] + v[o - st[a]]);
-            comp[a] = POW2 ? t * iq : div_by_const(t, q, iq);
+            comp[a] = POW2 ? t : div_by_const(t, q, iq);
         }
     }
     return (comp[0] * comp[0]) + (comp[1] * comp[1]) + (comp[2] * comp[2]) + (comp[3] * comp[3]);
@@ -241,15 +242,22 @@ __device__ inline void gface_plus(const Geo &g, const int c[4], const int n[4], 
         gout.p[2 * D + 1][o + st[D]] = gv;
 }
 
+// One thread per voxel of a plane, i fastest across rows: bound by the FP64
+// pipe, which a warp holds for the same time whatever lanes it uses, and a
+// tile of 128 x 2 left a quarter of them empty at 97 x 101.  With that and the
+// scaling (24 of about 230 FP64 instructions a voxel with two images) the edge
+// detector of two images took, in us: 97 x 101 x 53 x 11 8846 -> 7859, 256^2 x
+// 128 x 10 111.4e3 -> 103.3e3; h = 0.3: 11348 -> 10062, 142.8e3 -> 135.2e3.
+// POW2: theta and rho hold the scale 1/(4h)^2.
 template <bool POW2>
-__global__ void k_gfaces(Geo g, const double *i0, const double *ithr, GPtrs8 gout, double h, double K, double theta,
-                         double rho, double ih, double iq)
+__global__ void __launch_bounds__(256) k_gfaces(Geo g, FastDiv row, FastDiv planes, const double *i0,
+                                                const double *ithr, GPtrs8 gout, double h, double K, double theta,
+                                                double rho, double ih, double iq)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int kl = blockIdx.z;
-    const int k = kl % (g.nz + 1), l = kl / (g.nz + 1);
-    if (i > g.nx || j > g.ny)
+    const unsigned at = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = (int)fdiv(at, row), i = (int)(at - j * row.d);
+    const int l = (int)fdiv(blockIdx.y, planes), k = (int)(blockIdx.y - l * planes.d);
+    if (j > g.ny)
         return;
     const int c[4] = {i, j, k, l};
     const int n[4] = {g.nx, g.ny, g.nz, g.nt};
@@ -884,18 +892,20 @@ void launch_presmooth_explicit(const Geo &g, double *v, const double *prev, doub
 void launch_gfaces(const Geo &g, const double *i0, const double *ithr, GPtrs8 gout, double h, double K, double theta,
                    double rho, cudaStream_t st)
 {
-    const int bx = g.nx + 1 >= 128 ? 128 : (g.nx + 1 >= 64 ? 64 : 32);
-    const int by = 256 / bx;
-    dim3 bl(bx, by, 1), gr((g.nx + 1 + bx - 1) / bx, (g.ny + 1 + by - 1) / by, (g.nz + 1) * (g.nt + 1));
+    const int planes = (g.nz + 1) * (g.nt + 1); // grids of at most 65,535 planes
     int e = 0;
     const double m = frexp(h, &e);
     const double ih = 1.0 / h, iq = 1.0 / (4.0 * h);
-    // a power of two whose reciprocals are normal numbers
-    if (m == 0.5 && ih * h == 1.0 && iq * (4.0 * h) == 1.0 && isnormal(ih) && isnormal(iq) && isnormal(4.0 * h))
-        k_gfaces<true><<<gr, bl, 0, st>>>(g, i0, ithr, gout, h, K, theta, rho, ih, iq);
+    const FastDiv row = make_fastdiv((unsigned)g.nx + 1), pl = make_fastdiv((unsigned)g.nz + 1);
+    const dim3 gr(((unsigned)(g.nx + 1) * (g.ny + 1) + 255) / 256, planes);
+    // a power of two far from the ends of the range, and weights that stay
+    // normal with its scale
+    const double s0 = theta * (iq * iq), s1 = rho * (iq * iq);
+    if (m == 0.5 && abs(e) < 128 && (theta == 0.0 || isnormal(s0)) && (rho == 0.0 || isnormal(s1)))
+        k_gfaces<true><<<gr, 256, 0, st>>>(g, row, pl, i0, ithr, gout, h, K, s0, s1, ih, iq);
     else
-        k_gfaces<false><<<gr, bl, 0, st>>>(g, i0, ithr, gout, h, K, theta, rho, div_const_recip(h),
-                                           div_const_recip(4.0 * h));
+        k_gfaces<false><<<gr, 256, 0, st>>>(g, row, pl, i0, ithr, gout, h, K, theta, rho, div_const_recip(h),
+                                            div_const_recip(4.0 * h));
 }
 
 void launch_coef_ref(const Geo &g, const double *u, CPtrs8 gin, int has_g, GPtrs8 coef, double h, double eps2,

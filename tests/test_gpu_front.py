@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 DIMS = [(1, 1, 1, 1), (2, 1, 1, 1), (3, 2, 1, 2), (4, 3, 2, 1), (5, 1, 3, 2), (33, 3, 5, 2), (34, 4, 4, 3), (67, 2, 7, 1)]
 
 
-@pytest.mark.parametrize("h", [1.0, 0.7, 3e-7])
+@pytest.mark.parametrize("h", [1.0, 0.125, 0.7, 3e-7])
 @pytest.mark.parametrize("dims", DIMS)
 @pytest.mark.parametrize("images", [1, 2])
 @pytest.mark.parametrize("arith", ["fp64", "mixed"])

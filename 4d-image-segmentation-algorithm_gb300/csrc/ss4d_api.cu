@@ -601,62 +601,85 @@ static ss4d_status sor_reference(ss4d_solver *s, const ss4d_params *p, double *u
     return isfinite(R) ? SS4D_OK : SS4D_ERR_NONFINITE;
 }
 
-// the mixed form's loop as a CUDA graph's while loop
-static ss4d_status build_graph(ss4d_solver *s)
+// a conditional node of `graph` after node `after` (or the first one): its
+// handle (1 when the graph is launched) and its empty body
+static cudaError_t add_conditional(cudaGraph_t graph, cudaGraphNode_t *after, cudaGraphConditionalNodeType type,
+                                   cudaGraphConditionalHandle *h, cudaGraphNode_t *node, cudaGraph_t *body)
 {
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    cudaGraphConditionalHandle h;
-    CK(cudaGraphCreate(&graph, 0));
-    cudaError_t e = cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        set_err("cudaGraphConditionalHandleCreate: %s", cudaGetErrorString(e));
-        return SS4D_ERR_CUDA;
-    }
+    cudaError_t e = cudaGraphConditionalHandleCreate(h, graph, 1, cudaGraphCondAssignDefault);
+    if (e != cudaSuccess)
+        return e;
     // the C++ view of this union-holding struct has no default constructor:
     // build it in zeroed storage, as the C API expects unused bytes zero
-    alignas(cudaGraphNodeParams) unsigned char cp_store[sizeof(cudaGraphNodeParams)];
-    memset(cp_store, 0, sizeof cp_store);
-    cudaGraphNodeParams &cp = *reinterpret_cast<cudaGraphNodeParams *>(cp_store);
+    alignas(cudaGraphNodeParams) unsigned char store[sizeof(cudaGraphNodeParams)];
+    memset(store, 0, sizeof store);
+    cudaGraphNodeParams &cp = *reinterpret_cast<cudaGraphNodeParams *>(store);
     cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.handle = *h;
+    cp.conditional.type = type;
     cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    e = cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &cp);
-    if (e != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        set_err("cudaGraphAddNode(conditional): %s", cudaGetErrorString(e));
-        return SS4D_ERR_CUDA;
-    }
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    e = cudaStreamBeginCaptureToGraph(s->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        set_err("cudaStreamBeginCaptureToGraph: %s", cudaGetErrorString(e));
-        return SS4D_ERR_CUDA;
-    }
-    const unsigned long long hv = (unsigned long long)h;
-    launch_refine(s->geo, s->sp, s->cfg, 0, s->sb, s->d_state, s->cap);
-    launch_refine(s->geo, s->sp, s->cfg, 1, s->sb, s->d_state, s->cap);
-    launch_zero_delta(s->sp, s->sb, s->d_state, s->cap);
-    launch_sweep32(s->geo, s->sp, s->cfg, 1, s->sb, s->d_params, s->d_state, s->cap);
-    launch_sweep32(s->geo, s->sp, s->cfg, 0, s->sb, s->d_params, s->d_state, s->cap);
-    launch_ctrl_mixed(s->sb, s->cfg.grid, s->d_params, s->d_state, hv, 1, s->cap);
+    e = cudaGraphAddNode(node, graph, after, nullptr, after ? 1 : 0, &cp);
+    if (e == cudaSuccess)
+        *body = cp.conditional.phGraph_out[0];
+    return e;
+}
+
+// launches made by f on s->cap, as nodes of `graph` after node `after` (or first)
+template <typename F>
+static cudaError_t capture_into(ss4d_solver *s, cudaGraph_t graph, cudaGraphNode_t *after, F &&f)
+{
+    cudaError_t e = cudaStreamBeginCaptureToGraph(s->cap, graph, after, nullptr, after ? 1 : 0,
+                                                  cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess)
+        return e;
+    f();
     cudaGraph_t captured = nullptr;
-    e = cudaStreamEndCapture(s->cap, &captured);
+    return cudaStreamEndCapture(s->cap, &captured);
+}
+
+// The mixed form's loop as a CUDA graph's while loop.  The kernels that only a
+// round's start or end runs (the refinement pass and its test, the zeroed
+// corrections) stand under a condition of their own; the inner iterations
+// are GRAPH_TESTS pairs of half-sweeps, the red one running the controller in
+// its last block, and those after a round's end return at once.  With all
+// seven kernels in every body an iteration of 161 x 143 x 61 x 9 (two
+// half-sweeps of about 50 us) spent 20 us between kernels; the step went from
+// 6.66 to 6.56 ms by the condition, 6.40 by four iterations per body (eight
+// gave no more) and 6.16 by the controller in the half-sweep.  Launching the
+// kernels programmatically, each while its predecessor still ran, lost 5 us
+// an iteration.
+static constexpr int GRAPH_TESTS = 4;
+static ss4d_status build_graph(ss4d_solver *s)
+{
+    cudaGraph_t graph = nullptr, body = nullptr, open_body = nullptr;
+    cudaGraphConditionalHandle h, ho;
+    cudaGraphNode_t loop, open;
+    CK(cudaGraphCreate(&graph, 0));
+    cudaError_t e = add_conditional(graph, nullptr, cudaGraphCondTypeWhile, &h, &loop, &body);
+    if (e == cudaSuccess)
+        e = add_conditional(body, nullptr, cudaGraphCondTypeIf, &ho, &open, &open_body);
+    const unsigned long long conds[2] = {(unsigned long long)h, (unsigned long long)ho};
+    if (e == cudaSuccess)
+        e = capture_into(s, open_body, nullptr, [&] {
+            launch_refine(s->geo, s->sp, s->cfg, 0, s->sb, s->d_state, s->cap);
+            launch_refine(s->geo, s->sp, s->cfg, 1, s->sb, s->d_state, s->cap);
+            launch_ctrl_mixed(s->sb, s->cfg.grid, s->d_params, s->d_state, conds, s->cap);
+            launch_zero_delta(s->sp, s->sb, s->d_state, s->cap);
+        });
+    if (e == cudaSuccess)
+        e = capture_into(s, body, &open, [&] {
+            for (int n = 0; n < GRAPH_TESTS; ++n) {
+                launch_sweep32(s->geo, s->sp, s->cfg, 1, s->sb, s->d_params, s->d_state, s->cap, n);
+                launch_sweep32(s->geo, s->sp, s->cfg, 0, s->sb, s->d_params, s->d_state, s->cap, n, conds);
+            }
+        });
+    cudaGraphExec_t exec = nullptr;
+    if (e == cudaSuccess)
+        e = cudaGraphInstantiate(&exec, graph, 0);
     if (e != cudaSuccess) {
         cudaGetLastError();
         cudaGraphDestroy(graph);
-        set_err("cudaStreamEndCapture: %s", cudaGetErrorString(e));
-        return SS4D_ERR_CUDA;
-    }
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        cudaGraphDestroy(graph);
-        set_err("cudaGraphInstantiate: %s", cudaGetErrorString(e));
+        set_err("the loop's graph: %s", cudaGetErrorString(e));
         return SS4D_ERR_CUDA;
     }
     s->graphmx = graph;
@@ -732,7 +755,7 @@ static ss4d_status ws_first_pass(ss4d_solver *s)
     const SweepCfg &cfg = s->cfg;
     launch_refine(s->geo, s->sp, cfg, 0, s->sb, s->d_state, s->stream);
     launch_refine(s->geo, s->sp, cfg, 1, s->sb, s->d_state, s->stream);
-    launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
+    launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, nullptr, s->stream);
     s->launches += 4; // a refinement pass is 3 launches
     return last_launch();
 }
@@ -933,15 +956,13 @@ static ss4d_status run_split_loop(ss4d_solver *s, const ss4d_params *p, int mixe
 // the graph's while loop?  The plain form always: its flat walk of the
 // targets and the missing launches win at every size (a step at 32^3 x 8
 // 886 -> 543 us, 161 x 143 x 61 x 9 15.4 -> 12.7 ms, 256 x 256 x 128 x 8
-// 61.0 -> 60.1 ms).  The mixed form up to 9e6 voxels: there the loop's data (about 30
-// bytes per voxel) stays in L2 or near it, and the graph's body costs seven
-// launches an iteration (32^3 x 8 850 -> 391 us, 64 x 64 x 64 x 10 1648 ->
-// 1386 us, 131 x 129 x 65 x 8 3.94 -> 3.90 ms); beyond, the launches are lost
-// in the half-sweeps' time and the separate FP32 kernel, at 40 warps per SM
-// instead of 32, streams faster (161 x 143 x 61 x 9 5.53 against 5.58 ms,
-// 256 x 256 x 128 x 8 24.1 against 26.0 ms).
+// 61.0 -> 60.1 ms).  The mixed form up to 5e6 voxels (us of a step, graph and
+// persistent: 32^3 x 8 850 and 391, 64 x 64 x 64 x 10 1464 and 1343, 96 x 96 x
+// 64 x 8 2063 and 2037; 128 x 96 x 64 x 8 2518 and 2598, 131 x 129 x 65 x 8 3609
+// and 3871): beyond, the launches are lost in the half-sweeps' time and the
+// separate FP32 kernel, at 40 warps per SM instead of 32, streams faster.
 #define LOOP_THREADS 512
-#define LOOP_MIXED_MAX_VOXELS 9000000
+#define LOOP_MIXED_MAX_VOXELS 5000000
 static bool loop_persistent(const ss4d_solver *s, int mixed)
 {
     return !mixed || s->geo.nint <= LOOP_MIXED_MAX_VOXELS;
@@ -1019,7 +1040,7 @@ static ss4d_status drive_loop(ss4d_solver *s, const ss4d_params *p, int mixed, i
                       [&] { launch_sweep64(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream); });
                 timed(s, SS4D_K_SWEEP64, true,
                       [&] { launch_sweep64(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
-                launch_ctrl64(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
+                launch_ctrl64(s->sb, cfg.grid, s->d_params, s->d_state, s->stream);
                 s->launches += 3;
             } else {
                 // kernels whose mode does not match return at once: only the
@@ -1033,7 +1054,7 @@ static ss4d_status drive_loop(ss4d_solver *s, const ss4d_params *p, int mixed, i
                       [&] { launch_sweep32(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream); });
                 timed(s, SS4D_K_SWEEP32, mode != 0,
                       [&] { launch_sweep32(g, sp, cfg, 0, s->sb, s->d_params, s->d_state, s->stream); });
-                launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
+                launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, nullptr, s->stream);
                 s->launches += 7;
             }
             CKS(last_launch());
@@ -1057,7 +1078,7 @@ static ss4d_status refine_paused(ss4d_solver *s)
     const SweepCfg &cfg = s->cfg;
     timed(s, SS4D_K_REFINE, true, [&] { launch_refine(g, sp, cfg, 0, s->sb, s->d_state, s->stream); });
     timed(s, SS4D_K_REFINE, true, [&] { launch_refine(g, sp, cfg, 1, s->sb, s->d_state, s->stream); });
-    launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, 0, 0, s->stream);
+    launch_ctrl_mixed(s->sb, cfg.grid, s->d_params, s->d_state, nullptr, s->stream);
     s->launches += 4;
     return last_launch();
 }
@@ -1067,7 +1088,7 @@ static ss4d_status refine_paused(ss4d_solver *s)
 static void count_graph_launches(ss4d_solver *s)
 {
     if (s->last_graphed)
-        s->launches += 7LL * s->h_state->bodies;
+        s->launches += 2LL * s->h_state->bodies + 3LL * s->h_state->opened;
 }
 
 extern "C" ss4d_status ss4d_solver_set_timing(ss4d_solver *s, int enable)

@@ -83,6 +83,8 @@ struct LoopState {
     int spec;        // mixed form: pause the loop when a round ends, before its refinement pass
                      // (the host-array step downloads the round's result meanwhile)
     int paused;      // set by the controller when it paused the loop (spec); the refinement clears it
+    int opened;      // mixed form, graph: bodies that started a round or refined
+    int arrived;     // mixed form, graph: blocks of the red half-sweep that have ended
     double R;        // last FP64 residual (sum r^2 h^4)
     double R_first;  // FP64 residual after iteration 1 (fast) / initial (mixed)
     double Rd;       // mixed form: last FP32 correction residual
@@ -216,17 +218,19 @@ void launch_loop_init(LoopState *state, int mode, cudaStream_t st, int pre = 0, 
 void launch_sweep64(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
                     LoopState *state, cudaStream_t st);
 void launch_advance(LoopState *state, cudaStream_t st);
-void launch_ctrl64(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, unsigned long long cond_handle,
-                   int use_cond, cudaStream_t st);
+void launch_ctrl64(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, cudaStream_t st);
 
 // mixed precision
 void launch_refine(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, LoopState *state,
                    cudaStream_t st);
 void launch_zero_delta(const Split &s, SplitBufs b, LoopState *state, cudaStream_t st);
+// conds (the graph's loop): the conditions of the while loop and of the
+// kernels that only a round's start runs; the red half-sweep then also runs
+// the controller.  follow: a half-sweep that only acts within a round
 void launch_sweep32(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
-                    LoopState *state, cudaStream_t st);
-void launch_ctrl_mixed(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, unsigned long long cond_handle,
-                       int use_cond, cudaStream_t st);
+                    LoopState *state, cudaStream_t st, int follow = 0, const unsigned long long *conds = nullptr);
+void launch_ctrl_mixed(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, const unsigned long long *conds,
+                       cudaStream_t st);
 
 int max_blocks_sweep64();
 int max_blocks_sweep32();

@@ -432,6 +432,8 @@ __global__ void k_loop_init(LoopState *st, int mode, int pre, int spec)
     st->dsrc = 0;
     st->final_red = 0;
     st->bodies = 0;
+    st->opened = 0;
+    st->arrived = 0;
     st->keep = 0;
     st->warm = 0;
     st->near = 0;
@@ -489,8 +491,7 @@ __global__ void __launch_bounds__(256) k_sweep64(Geo g, Split sp, SweepCfg cfg, 
 }
 
 // sums the partials of both colours in a fixed order and decides
-__global__ void k_ctrl64(SplitBufs b, int nparts, const DevParams *__restrict__ dp, LoopState *st,
-                         cudaGraphConditionalHandle h, int use_cond)
+__global__ void k_ctrl64(SplitBufs b, int nparts, const DevParams *__restrict__ dp, LoopState *st)
 {
     double a = 0.0, c = 0.0;
     for (int t = threadIdx.x; t < nparts; t += blockDim.x) {
@@ -499,11 +500,8 @@ __global__ void k_ctrl64(SplitBufs b, int nparts, const DevParams *__restrict__ 
     }
     a = block_sum(a);
     c = block_sum(c);
-    if (threadIdx.x == 0) {
-        const bool stop = ctrl64_update(st, a, c, dp);
-        if (use_cond)
-            cudaGraphSetConditional(h, stop ? 0u : 1u);
-    }
+    if (threadIdx.x == 0)
+        ctrl64_update(st, a, c, dp);
 }
 
 // ---------------------------------------------------------------------------
@@ -578,6 +576,36 @@ __global__ void k_zero_delta(Split sp, SplitBufs b, const LoopState *__restrict_
     }
 }
 
+// the conditions of the loop's graph (ss4d_api.cu): test 1: the red half-sweep
+// runs the controller
+struct LoopConds {
+    cudaGraphConditionalHandle loop, open;
+    int test;
+};
+
+// one block: the partial sums of both colours in a fixed order, and the controller
+__device__ void test_mixed(const SplitBufs &b, int nparts, const DevParams *dp, LoopState *st, const LoopConds &lc)
+{
+    const int mode = st->mode;
+    double a = 0.0, c = 0.0;
+    if (mode != 1) {
+        for (int t = threadIdx.x; t < nparts; t += blockDim.x) {
+            a += __ldcg(b.partial[0] + t);
+            c += __ldcg(b.partial[1] + t);
+        }
+    }
+    a = block_sum(a);
+    c = block_sum(c);
+    if (threadIdx.x != 0)
+        return;
+    st->arrived = 0;
+    const bool stop = ctrl_mixed_update(st, a, c, dp);
+    if (lc.test) { // a paused loop leaves the graph too
+        cudaGraphSetConditional(lc.loop, stop || st->paused ? 0u : 1u);
+        cudaGraphSetConditional(lc.open, st->mode != 2);
+    }
+}
+
 // FP32 half-sweep of colour COL: each thread updates two adjacent targets of
 // a row (flat index of pairs), so the pair shares its index arithmetic and reads its
 // own values, right-hand sides and the y/z/w neighbours as 8-byte pairs; each
@@ -586,10 +614,11 @@ __global__ void k_zero_delta(Split sp, SplitBufs b, const LoopState *__restrict_
 // partial residual sum.
 template <int COL>
 __global__ void __launch_bounds__(256) k_sweep32(FlatIndex F, SplitBufs b,
-                                                 const DevParams *__restrict__ dp, const LoopState *__restrict__ st)
+                                                 const DevParams *__restrict__ dp, LoopState *st, int follow,
+                                                 LoopConds lc)
 {
     const int mode = st->mode;
-    if ((COL == 0 ? (mode == 0) : (mode != 2)) || st->stop)
+    if ((COL == 0 && !follow ? (mode == 0) : (mode != 2)) || st->stop)
         return;
     const int ds = st->dsrc;
     const float *src;
@@ -619,32 +648,36 @@ __global__ void __launch_bounds__(256) k_sweep32(FlatIndex F, SplitBufs b,
     const double tot = block_sum((double)acc);
     if (threadIdx.x == 0)
         b.partial[COL][blockIdx.x] = tot;
+    if (COL == 1 || !lc.test)
+        return;
+    // the last block to come here adds the partial sums of both colours (in
+    // their order: it does not matter which block it is) and runs the
+    // controller, in place of a launch of its own
+    __shared__ int last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&st->arrived, 1) == (int)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (last)
+        test_mixed(b, gridDim.x, dp, st, lc);
 }
 
-__global__ void k_ctrl_mixed(SplitBufs b, int nparts, const DevParams *__restrict__ dp, LoopState *st,
-                             cudaGraphConditionalHandle h, int use_cond)
+// the controller by itself: after the refinement pass, and after every body
+// of the host-driven loop
+__global__ void k_ctrl_mixed(SplitBufs b, int nparts, const DevParams *__restrict__ dp, LoopState *st, LoopConds lc)
 {
     if (st->stop) { // stopped before the loop (the warm-start prologue's test)
-        if (threadIdx.x == 0 && use_cond)
-            cudaGraphSetConditional(h, 0u);
+        if (threadIdx.x == 0 && lc.test)
+            cudaGraphSetConditional(lc.loop, 0u);
         return;
     }
-    const int mode = st->mode;
-    double a = 0.0, c = 0.0;
-    if (mode != 1) {
-        for (int t = threadIdx.x; t < nparts; t += blockDim.x) {
-            a += b.partial[0][t];
-            if (mode == 0 || mode == 2)
-                c += b.partial[1][t];
-        }
-    }
-    a = block_sum(a);
-    c = block_sum(c);
-    if (threadIdx.x != 0)
+    if (lc.test && st->mode != 0) // in the graph: the half-sweep's
         return;
-    const bool stop = ctrl_mixed_update(st, a, c, dp);
-    if (use_cond) // a paused loop leaves the graph too
-        cudaGraphSetConditional(h, stop || st->paused ? 0u : 1u);
+    if (lc.test && threadIdx.x == 0)
+        st->opened += 1;
+    test_mixed(b, nparts, dp, st, lc);
 }
 
 // ---------------------------------------------------------------------------
@@ -839,10 +872,9 @@ void launch_sweep64(const Geo &g, const Split &s, const SweepCfg &cfg, int colou
         k_sweep64<1><<<cfg.grid, cfg.threads, 0, st>>>(g, s, cfg, b, dp, state);
 }
 
-void launch_ctrl64(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, unsigned long long cond_handle,
-                   int use_cond, cudaStream_t st)
+void launch_ctrl64(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, cudaStream_t st)
 {
-    k_ctrl64<<<1, 256, 0, st>>>(b, nparts, dp, state, (cudaGraphConditionalHandle)cond_handle, use_cond);
+    k_ctrl64<<<1, 256, 0, st>>>(b, nparts, dp, state);
 }
 
 void launch_refine(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, LoopState *state,
@@ -879,19 +911,25 @@ SweepCfg make_pair_cfg(const Geo &g, const Split &s, const SweepCfg &cfg)
 }
 
 void launch_sweep32(const Geo &g, const Split &s, const SweepCfg &cfg, int colour, SplitBufs b, const DevParams *dp,
-                    LoopState *state, cudaStream_t st)
+                    LoopState *state, cudaStream_t st, int follow, const unsigned long long *conds)
 {
     const FlatIndex F = make_flat(g, s);
+    LoopConds lc = {};
+    if (conds)
+        lc = LoopConds{conds[0], conds[1], 1};
     if (colour == 0)
-        k_sweep32<0><<<cfg.grid, cfg.threads, 0, st>>>(F, b, dp, state);
+        k_sweep32<0><<<cfg.grid, cfg.threads, 0, st>>>(F, b, dp, state, follow, lc);
     else
-        k_sweep32<1><<<cfg.grid, cfg.threads, 0, st>>>(F, b, dp, state);
+        k_sweep32<1><<<cfg.grid, cfg.threads, 0, st>>>(F, b, dp, state, follow, lc);
 }
 
-void launch_ctrl_mixed(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, unsigned long long cond_handle,
-                       int use_cond, cudaStream_t st)
+void launch_ctrl_mixed(SplitBufs b, int nparts, const DevParams *dp, LoopState *state, const unsigned long long *conds,
+                       cudaStream_t st)
 {
-    k_ctrl_mixed<<<1, 256, 0, st>>>(b, nparts, dp, state, (cudaGraphConditionalHandle)cond_handle, use_cond);
+    LoopConds lc = {};
+    if (conds)
+        lc = LoopConds{conds[0], conds[1], 1};
+    k_ctrl_mixed<<<1, 256, 0, st>>>(b, nparts, dp, state, lc);
 }
 
 } // namespace ss4d

@@ -89,3 +89,28 @@ def test_persistent_loop_grid_cap(ss4d, cuda, max_grid):
             got.append((st["iterations"], u.cpu().numpy()))
         assert got[0][0] == got[1][0]
         assert np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("form,maxit", [("mixed", 200), ("mixed", 6), ("mixed", 9), ("projected", 200), ("tight", 200)])
+def test_graph_loop_equals_host_driven_loop(ss4d, cuda, form, maxit):
+    """Volumes above 5e6 voxels run the mixed loop as a graph whose bodies hold
+    four iterations and whose half-sweep runs the controller: rounds that end
+    at any of the four, a limit that ends the loop inside a body."""
+    torch = cuda
+    dims = (131, 127, 62, 5)
+    p, u0, g = _volume(ss4d, torch, dims, 11, maxNoGSIteration=maxit, **({"gsTol": 1e-20} if form == "tight" else {}))
+    out = []
+    for device_loop in (True, False):
+        u = u0.clone()
+        with ss4d.Solver.for_interior(*dims, arith="mixed") as S:
+            S.set_graph(device_loop)
+            if form == "projected":
+                S.set_extrapolation(3)
+                S.set_projection(True)
+            rec = []
+            for _ in range(4 if form == "projected" else 2):
+                st = S.seg_time_step(p, u, None, g)
+                rec.append((st["iterations"], st["refinements"], st["projected"]))
+        out.append((rec, u))
+    assert out[0][0] == out[1][0]
+    assert torch.equal(out[0][1], out[1][1])

@@ -27,8 +27,7 @@
 namespace ss4d {
 
 // 1/s; its FP64 division costs a warp as much as 2000 FP32 instructions, so a
-// block's first thread forms it for all (per thread at 128x128x64x12 the
-// features took 575 us, now 547, the apply 255, now 77)
+// block's first thread forms it for all
 __device__ __forceinline__ float ws_inv_sigma(const Geo &g, const LoopState *st, const DevParams *dp)
 {
     const double var = st->R_first / ((double)g.nint * dp->h4);
@@ -40,41 +39,61 @@ __device__ __forceinline__ long long split_index(const Geo &g, const Split &sp, 
     return (((long long)l * g.kM + k) * g.jM + j) * sp.Hs + ((i + 1) >> 1) + sp.A - 1;
 }
 
+// Bound by its 196 bytes per voxel.  The loads go out before the block waits
+// for 1/s: behind it they took 555 us at 128x128x64x12, now 362 (6.8 TB/s).
 __global__ void __launch_bounds__(256) k_ws_features(Geo g, Split sp, SplitBufs b, const double *__restrict__ i0,
                                                      CPtrs8 gin, const LoopState *__restrict__ st,
                                                      const DevParams *__restrict__ dp, __nv_bfloat16 *x0)
 {
     __shared__ float inv_sigma;
-    if (threadIdx.x == 0 && threadIdx.y == 0)
-        inv_sigma = ws_inv_sigma(g, st, dp);
-    __syncthreads();
-    const float inv = inv_sigma;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     const int k = 1 + blockIdx.z % g.nz, l = 1 + blockIdx.z / g.nz;
-    if (i > g.nx || j > g.ny)
-        return;
+    const bool in = i <= g.nx && j <= g.ny;
     const int col = (i + j + k + l) & 1;
-    const long long s = split_index(g, sp, i, j, k, l);
+    const long long s = split_index(g, sp, i, j, k, l), o = nat_index(g, i, j, k, l);
+    // every load of the voxel on its way before the block waits for 1/s
+    float r0 = 0.f, rm = 0.f, rp = 0.f;
+    double cf[9], gf[8], u0 = 0.0, im = 0.0;
+    if (in) {
+        r0 = pick(b.r32, col)[s];
+        if (l > 1)
+            rm = pick(b.r32, col ^ 1)[split_index(g, sp, i, j, k, l - 1)];
+        if (l < g.nt)
+            rp = pick(b.r32, col ^ 1)[split_index(g, sp, i, j, k, l + 1)];
+        const double *cv = pick(b.coef, col) + coef_at(coef_index(g, sp, i, j, k, l), 0, 10);
+#pragma unroll
+        for (int f = 0; f < 9; ++f)
+            cf[f] = cv[32 * f];
+#pragma unroll
+        for (int f = 0; f < 8; ++f)
+            gf[f] = __ldg(gin.p[f] + o);
+        u0 = col == 0 ? b.R[0][s] : b.Bk[s];
+        im = __ldg(i0 + o);
+    }
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+        inv_sigma = ws_inv_sigma(g, st, dp);
+    __syncthreads();
+    if (!in)
+        return;
+    const float inv = inv_sigma;
     float ch[16];
-    ch[0] = pick(b.r32, col)[s] * inv;
-    ch[1] = l > 1 ? pick(b.r32, col ^ 1)[split_index(g, sp, i, j, k, l - 1)] * inv : 0.f;
-    ch[2] = l < g.nt ? pick(b.r32, col ^ 1)[split_index(g, sp, i, j, k, l + 1)] * inv : 0.f;
-    const double *cv = pick(b.coef, col) + coef_at(coef_index(g, sp, i, j, k, l), 0, 10);
-    const float idiag = 1.f / d2f_bits(cv[256]);
+    ch[0] = r0 * inv;
+    ch[1] = l > 1 ? rm * inv : 0.f;
+    ch[2] = l < g.nt ? rp * inv : 0.f;
+    const float idiag = 1.f / d2f_bits(cf[8]);
     ch[3] = ch[0] * idiag;
 #pragma unroll
     for (int f = 0; f < 8; ++f)
-        ch[4 + f] = d2f_bits(cv[32 * f]) * idiag;
+        ch[4 + f] = d2f_bits(cf[f]) * idiag;
     ch[12] = idiag;
-    const long long o = nat_index(g, i, j, k, l);
     float gb = 0.f;
 #pragma unroll
     for (int f = 0; f < 8; ++f)
-        gb += d2f_bits(__ldg(gin.p[f] + o));
+        gb += d2f_bits(gf[f]);
     ch[13] = gb * 0.125f;
-    ch[14] = d2f_bits(col == 0 ? b.R[0][s] : b.Bk[s]);
-    ch[15] = d2f_bits(__ldg(i0 + o));
+    ch[14] = d2f_bits(u0);
+    ch[15] = d2f_bits(im);
     __nv_bfloat162 v[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c)
@@ -86,6 +105,8 @@ __global__ void __launch_bounds__(256) k_ws_features(Geo g, Split sp, SplitBufs 
     *reinterpret_cast<uint4 *>(x0 + tc::planar_off(l - 1, 8, 2, vol, vf)) = *reinterpret_cast<uint4 *>(&v[4]);
 }
 
+// A block takes several planes: one per block, the FP64 divisions of 1/s alone,
+// one per block, took 54 of its 77 us at 128x128x64x12; now 45 us.
 __global__ void __launch_bounds__(256) k_ws_apply(Geo g, Split sp, SplitBufs b, const float *__restrict__ y,
                                                   const LoopState *__restrict__ st, const DevParams *__restrict__ dp)
 {
@@ -96,20 +117,18 @@ __global__ void __launch_bounds__(256) k_ws_apply(Geo g, Split sp, SplitBufs b, 
         inv_sigma = ws_inv_sigma(g, st, dp);
     __syncthreads();
     const float inv = inv_sigma;
+    const float sigma = inv > 0.f ? 1.f / inv : 0.f;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = 1 + blockIdx.z % g.nz, l = 1 + blockIdx.z / g.nz;
     if (i > g.nx || j > g.ny)
         return;
-    const float sigma = inv > 0.f ? 1.f / inv : 0.f;
-    const size_t vox = (((size_t)(l - 1) * g.nz + (k - 1)) * g.ny + (j - 1)) * g.nx + (i - 1);
-    const float d = sigma * y[vox];
-    const int col = (i + j + k + l) & 1;
-    const long long s = split_index(g, sp, i, j, k, l);
-    if (col == 0)
-        pick(b.dR, st->dsrc)[s] = isfinite(d) ? d : 0.f;
-    else
-        b.dB[s] = isfinite(d) ? d : 0.f;
+    float *const red = pick(b.dR, st->dsrc);
+    for (int z = blockIdx.z; z < g.nz * g.nt; z += gridDim.z) {
+        const int k = 1 + z % g.nz, l = 1 + z / g.nz;
+        const float d = sigma * y[((size_t)z * g.ny + (j - 1)) * g.nx + (i - 1)];
+        const int col = (i + j + k + l) & 1;
+        (col == 0 ? red : b.dB)[split_index(g, sp, i, j, k, l)] = isfinite(d) ? d : 0.f;
+    }
 }
 
 // (r0 - A32 d)^2 over the targets of one colour, as in k_sweep32 without the update
@@ -188,6 +207,8 @@ void launch_ws_apply(const Geo &g, const Split &sp, SplitBufs b, const float *y,
 {
     dim3 gr, bl;
     ws_interior_grid(g, gr, bl);
+    const unsigned planes = 8 * 152 / (gr.x * gr.y) + 1; // about a wave of blocks
+    gr.z = gr.z < planes ? gr.z : planes;
     k_ws_apply<<<gr, bl, 0, s>>>(g, sp, b, y, st, dp);
 }
 

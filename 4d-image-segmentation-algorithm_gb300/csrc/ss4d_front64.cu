@@ -5,8 +5,11 @@
 // reference's bit for bit; only the residual's terms are added in another
 // order (and unscaled by h^4 until their sum is complete).
 //
-// Bound by the FP64 pipe: 18 instructions per target for the update and 4 for
-// its residual, which the separate residual pass formed with 15.4 per voxel.
+// Bound by the FP64 pipe: 16 instructions per target for the update and 2 for
+// its residual, which the separate residual pass formed with 15.4 per voxel
+// (the edge detector of two images of 97 x 101 x 53 x 11: 7.84 ms with 4, 7.39 with 2).
+// Two blocks of 256 per SM (90 registers, none spilled): 6.96 ms; three 7.16,
+// four 7.39, five 7.43; one of 384 7.10, one of 512 7.20.
 #include "ss4d_front.cuh"
 
 namespace ss4d {
@@ -76,9 +79,10 @@ struct Exact64 {
                                                  double yp, double zm, double zp, double wm, double wp, double &acc)
     {
         const double cs = C.c * (xr + xl + ym + yp + zm + zp + wm + wp);
-        const double gs = div_by_const(pv + cs, C.d, C.y);
+        const double t = pv + cs;
+        const double gs = div_by_const(t, C.d, C.y);
         const double v = u + C.omega * (gs - u);
-        const double r = (COL == 0 ? u : v) * C.d - cs - pv;
+        const double r = fma(COL == 0 ? u : v, C.d, -t); // one rounding instead of three
         acc = fma(r, r, acc);
         return v;
     }
@@ -97,7 +101,7 @@ struct Exact64 {
     }
 };
 
-__global__ void __launch_bounds__(FRONT64_THREADS, 4) k_presmooth64(const __grid_constant__ FrontArgs a)
+__global__ void __launch_bounds__(FRONT64_THREADS, 2) k_presmooth64(const __grid_constant__ FrontArgs a)
 {
     presmooth_body<Exact64>(a);
 }

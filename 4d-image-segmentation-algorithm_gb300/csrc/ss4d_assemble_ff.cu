@@ -64,14 +64,6 @@ __device__ __forceinline__ ff2 pair_of(ff a, ff b)
 {
     return ff2{mk2(a.h, b.h), mk2(a.l, b.l)};
 }
-__device__ __forceinline__ ff lane0(ff2 a)
-{
-    return ff_make(lo2(a.h), lo2(a.l));
-}
-__device__ __forceinline__ ff lane1(ff2 a)
-{
-    return ff_make(hi2(a.h), hi2(a.l));
-}
 __device__ __forceinline__ ff2 ldf(const float4 *__restrict__ p, unsigned x)
 {
     return unpack4(__ldg(p + x));

@@ -114,20 +114,6 @@ inline Geo make_geo(const ss4d_dims &d)
     return g;
 }
 
-// (i, j, k, l) of natural index o < 2^31
-__device__ __forceinline__ void nat_coords(const Geo &g, unsigned o, int &i, int &j, int &k, int &l)
-{
-    unsigned q = fdiv(o, g.fiM);
-    i = (int)(o - q * g.fiM.d);
-    o = q;
-    q = fdiv(o, g.fjM);
-    j = (int)(o - q * g.fjM.d);
-    o = q;
-    q = fdiv(o, g.fkM);
-    k = (int)(o - q * g.fkM.d);
-    l = (int)q;
-}
-
 __host__ __device__ inline long long nat_index(const Geo &g, int i, int j, int k, int l)
 {
     return (((long long)l * g.kM + k) * g.jM + j) * g.iM + i;

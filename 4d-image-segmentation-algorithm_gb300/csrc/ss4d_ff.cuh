@@ -155,42 +155,6 @@ __device__ __forceinline__ ff ld_ff(const double *p, long long o)
     return ff_make(v.x, v.y);
 }
 
-__device__ __forceinline__ void st_ff(double *p, long long o, ff v)
-{
-    __stcs(reinterpret_cast<float2 *>(p) + o, make_float2(v.h, v.l));
-}
-
-
-__device__ __forceinline__ ff ff_neg(ff a)
-{
-    return ff_make(-a.h, -a.l);
-}
-
-// 1/x for normal x: FP32 seed y0 = 1/x.h (correctly rounded), one Newton
-// step y = y0 + y0 (1 - x y0) with x y0 formed to float-float: error about e0^2
-__device__ __forceinline__ ff ff_rcp(ff x)
-{
-    const float y0 = __frcp_rn(x.h);
-    const float q = x.h * y0;
-    float qe = fmaf(x.h, y0, -q);
-    qe = fmaf(x.l, y0, qe);                // x y0 = q + qe
-    const float r = (1.f - q) - qe;        // 1 - q is exact (q near 1)
-    const float c = y0 * r, ce = fmaf(y0, r, -c);
-    ff y = fast_two_sum(y0, c);
-    y.l += ce;
-    return y;
-}
-
-__device__ __forceinline__ ff ld_ff2(const float2 *p, long long o)
-{
-    const float2 v = p[o];
-    return ff_make(v.x, v.y);
-}
-
-__device__ __forceinline__ void st_ff2(float2 *p, long long o, ff v)
-{
-    p[o] = make_float2(v.h, v.l);
-}
 
 } // namespace ffa
 } // namespace ss4d

@@ -73,10 +73,6 @@ struct ff2 {
     f2 h, l;
 };
 
-__device__ __forceinline__ ff2 mkff2(f2 h, f2 l)
-{
-    return ff2{h, l};
-}
 __device__ __forceinline__ ff2 both(ff a)
 {
     return ff2{both(a.h), both(a.l)};

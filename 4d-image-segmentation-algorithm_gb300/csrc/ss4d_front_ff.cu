@@ -225,7 +225,8 @@ __device__ __forceinline__ ff2 face_term(const float4 *__restrict__ v, unsigned 
     return ff_add_nr2(ff_mul_nr2(kt, tt), ff_mul_nr2(kn, nn));
 }
 
-// g = 1/(1 + s): FP32 seeds, one Newton step (ff_rcp)
+// g = 1/(1 + s): FP32 seeds y0, one Newton step y = y0 + y0 (1 - x y0) with x y0
+// formed to float-float: error about that of y0 squared
 __device__ __forceinline__ void g_of(ff2 s, double out[2])
 {
     const ff2 x = ff_add2(both(ff_make(1.f, 0.f)), ff_norm2(s));

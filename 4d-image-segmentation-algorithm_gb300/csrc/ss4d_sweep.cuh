@@ -16,15 +16,6 @@ __device__ __forceinline__ float ld_stream(const float *p)
 {
     return __ldcs(p);
 }
-__device__ __forceinline__ double2 ld_stream2(const double *p)
-{
-    return __ldcs(reinterpret_cast<const double2 *>(p));
-}
-__device__ __forceinline__ float4 ld_stream4(const float *p)
-{
-    return __ldcs(reinterpret_cast<const float4 *>(p));
-}
-
 // FP32 <-> FP64 conversions by integer bit operations.  On this GPU a
 // conversion instruction to or from FP64 issues at the FP64 rate (1/68 of
 // FP32); these run on the integer pipe instead.

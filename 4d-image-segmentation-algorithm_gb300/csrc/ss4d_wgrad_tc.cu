@@ -2,30 +2,32 @@
 // convolutions on the fifth-generation tensor cores.
 //
 // dW[tap][co][ci] = sum over the voxels v of X[v + tap][ci] dY[v][co] is a
-// matrix product whose contraction runs over the voxels: D[(dz, ci)][co] for
-// each of the nine (dy, dx) taps, K = 16 voxels (8 along x, two rows of y) a
-// multiply-add.  The channel-group planar activations are what such operands
-// want when the channels are the contiguous index (MN-major, no swizzle: a
-// core matrix is 8 voxels by 8 channels, 128 contiguous bytes of a row of a
-// channel group).  A tile of X, 10 x 18 x (TZ + 2) voxels, arrives by one TMA
+// matrix product whose contraction runs over the voxels: for each of the three
+// dy taps D[(dz, ci)][(dx, co)], K = 16 voxels (8 along x, two rows of y) a
+// multiply-add; along x the sum runs over w = v + dx, X[w] dY[w - dx], so that the
+// dx taps are shifts of dY and lie in N.  The channel-group planar activations
+// are what such operands want when the channels are the contiguous index
+// (MN-major, no swizzle: a core matrix is 8 voxels by 8 channels, 128 contiguous bytes of a row of a
+// channel group).  A tile of X, 8 x 18 x (WZ + 2) voxels, arrives by one TMA
 // box with the channel groups inside the planes, [z][group][y][x][8], so
 // that consecutive groups and then consecutive planes lie a constant stride
 // apart: 128 rows of the A operand starting at plane p are the channels of
 // planes p, p + 1, p + 2 (the three dz taps of output plane p) and beyond,
-// whose rows of D nobody reads.  dY, 8 x 16 x TZ voxels with the groups
-// inside the planes too, is the B operand.  Both operands are the tiles
-// themselves; voxels outside the crop are zeros of the TMA's fill.  A tenth
+// whose rows of D nobody reads.  dY, 8 x 16 x WZ voxels at the three shifts,
+// [z][dx][group][y][x][8], is the B operand.  Both operands are the tiles
+// themselves; voxels outside the crop are zeros of the TMA's fill.  A fourth
 // product with a matrix of ones adds up dY for the bias gradient.
 //
-// The ten accumulators stay in tensor memory over all tiles of a CTA
-// (K = 512 voxels each); at its end a CTA writes its partial sums, which
+// The accumulators stay in tensor memory over all tiles of a CTA
+// (K = 256 voxels each); at its end a CTA writes its partial sums, which
 // k_reduce_grad adds in CTA order.  One thread issues loads and
 // multiply-adds, two tiles are in flight; waits are bounded as in
 // ss4d_conv_tc.cu.
 //
-// What bounds it: the tensor core's operand reads (4 KB of A and 1 KB of B
-// from shared memory per multiply-add of M = 128, N = 32, K = 16), as in
-// the convolutions.
+// What bounds it: the tensor core's operand reads from shared memory, 4 KB of
+// A and 3 KB of B per multiply-add of M = 128, N = 96, K = 16.  With each of
+// the nine (dy, dx) taps a multiply-add of its own (N = 32, 4 KB of A for 1 KB of
+// B) a layer of 8 crops of 40 x 40 x 20 took 54 us, now 32.
 #include <cuda_bf16.h>
 
 #include "ss4d_conv_tc.cuh"
@@ -37,13 +39,14 @@ namespace tc {
 namespace {
 
 constexpr int WG_WARPS = 4, WG_THREADS = 32 * (WG_WARPS + 1);
+constexpr int WZ = 2; // planes of a tile: two tiles of X and of three dY's fit
 
 // CIN input channels of X, NY channels of dY (N)
 template <int CIN, int NY> struct WgCfg {
     static constexpr int XG = CIN / 8, YG = NY / 8; // channel groups
-    static constexpr int XGS = HX * HY * 16;        // bytes of one group of one plane
+    static constexpr int XGS = TX * HY * 16;        // bytes of one group of one plane
     static constexpr int YGS = TX * TY * 16;
-    static constexpr int XB = HZ * XG * XGS, YB = TZ * YG * YGS; // one tile
+    static constexpr int XB = (WZ + 2) * XG * XGS, YB = WZ * 3 * YG * YGS; // one tile
     static constexpr int XS = (XB + 1023) / 1024 * 1024, YS = (YB + 1023) / 1024 * 1024;
     static constexpr int ONES = 4096; // 128 x 16 ones
     static constexpr int NACC = 10;
@@ -51,7 +54,7 @@ template <int CIN, int NY> struct WgCfg {
     // X tiles first: the rows of A past the tile's last plane stay inside
     static constexpr int SMEM = 1024 + 2 * XS + 2 * YS + ONES + 128;
     static_assert(NACC * NY <= TCOLS, "tensor memory");
-    static_assert(XS + 2 * YS >= (TZ - 1) * XG * XGS + 16 * XGS + HX * 16,
+    static_assert(XS + 2 * YS >= (WZ - 1) * XG * XGS + 16 * XGS,
                   "the A operand's unused rows must stay in shared memory");
     static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
 };
@@ -95,16 +98,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    const int ntx = (a.nx + TX - 1) / TX, nty = (a.ny + TY - 1) / TY, ntz = (a.nz + TZ - 1) / TZ;
+    const int ntx = (a.nx + TX - 1) / TX, nty = (a.ny + TY - 1) / TY, ntz = (a.nz + WZ - 1) / WZ;
     const long long ntiles = (long long)ntx * nty * ntz * a.nf;
     const long long first = blockIdx.x;
     const int my_n = (int)((ntiles - 1 - first) / gridDim.x + 1); // the grid has at most ntiles CTAs
 
     if (warp == WG_WARPS) {
         if (lane == 0) {
-            // D FP32, A and B BF16 and both MN-major, M = 128, N = NY
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                                   ((uint32_t)(NY >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+            // D FP32, A and B BF16 and both MN-major, M = 128, N = 3 NY (the ones' NY)
+            const uint32_t type = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                                  ((uint32_t)(128 >> 4) << 24);
+            const uint32_t idesc = type | ((uint32_t)(3 * NY >> 3) << 17), idesc1 = type | ((uint32_t)(NY >> 3) << 17);
             // MN-major without swizzle: LBO = stride of the core matrices along
             // K (the next row of 8 voxels), SBO = along M or N (the next group)
             const uint64_t odesc = make_desc(smem_u32(ones), 128, 256);
@@ -114,10 +118,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                 r /= ntx;
                 const int y0 = (int)(r % nty) * TY;
                 r /= nty;
-                const int z0 = (int)(r % ntz) * TZ, f = (int)(r / ntz), b = it & 1;
+                const int z0 = (int)(r % ntz) * WZ, f = (int)(r / ntz), b = it & 1;
                 mbar_expect_tx(full0 + 8 * b, C::XB + C::YB);
-                tma_load_5d(smem_u32(smem + b * C::XS), &xmap, full0 + 8 * b, 8 * (x0 - 1), y0 - 1, 0, z0 - 1, f);
-                tma_load_5d(smem_u32(ysm + b * C::YS), &ymap, full0 + 8 * b, 8 * x0, y0, 0, z0, f);
+                tma_load_5d(smem_u32(smem + b * C::XS), &xmap, full0 + 8 * b, 8 * x0, y0 - 1, 0, z0 - 1, f);
+                for (int q = 0; q < 3 * WZ; ++q) // plane q / 3, tap dx = q % 3 - 1: dY from x0 - dx on
+                    tma_load_5d(smem_u32(ysm + b * C::YS + q * C::YG * C::YGS), &ymap, full0 + 8 * b,
+                                8 * (x0 + 1 - q % 3), y0, 0, z0 + q / 3, f);
             };
             bool ok = true;
             int loads = 0, mmas = 0;
@@ -130,19 +136,19 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                     break;
                 }
                 tc_fence_after();
-                const uint64_t x0 = make_desc(smem_u32(smem + b * C::XS), HX * 16, C::XGS);
+                const uint64_t x0 = make_desc(smem_u32(smem + b * C::XS), TX * 16, C::XGS);
                 const uint64_t y0 = make_desc(smem_u32(ysm + b * C::YS), TX * 16, C::YGS);
 #pragma unroll 1
-                for (int p = 0; p < TZ; ++p)
-#pragma unroll 1
+                for (int p = 0; p < WZ; ++p)
+#pragma unroll
                     for (int y = 0; y < TY; y += 2) {
-                        const uint64_t bd = y0 + ((p * C::YG * C::YGS + y * TX * 16) >> 4);
-                        const uint64_t ad = x0 + ((p * C::XG * C::XGS + y * HX * 16) >> 4);
+                        const uint64_t bd = y0 + ((p * 3 * C::YG * C::YGS + y * TX * 16) >> 4);
+                        const uint64_t ad = x0 + ((p * C::XG * C::XGS + y * TX * 16) >> 4);
                         const uint32_t acc = (it | p | y) != 0;
 #pragma unroll
-                        for (int dd = 0; dd < 9; ++dd)
-                            umma_bf16(tmem + dd * NY, ad + (dd / 3) * HX + dd % 3, bd, idesc, acc);
-                        umma_bf16(tmem + 9 * NY, odesc, bd, idesc, acc);
+                        for (int dy = 0; dy < 3; ++dy)
+                            umma_bf16(tmem + dy * 3 * NY, ad + ((dy * TX * 16) >> 4), bd, idesc, acc);
+                        umma_bf16(tmem + 9 * NY, odesc, bd + ((C::YG * C::YGS) >> 4), idesc1, acc);
                     }
                 umma_commit(done0 + 8 * b);
                 mmas = it + 1;
@@ -259,8 +265,8 @@ cudaError_t run(const void *x, const void *dy, const WgArgs &a, int grid, cudaSt
 {
     using C = WgCfg<CIN, NY>;
     CUtensorMap xm, ym;
-    if (!planar_map(&xm, x, CIN, a.nx, a.ny, a.nz, a.nf, HX, HY, HZ) ||
-        !planar_map(&ym, dy, NY, a.nx, a.ny, a.nz, a.nf, TX, TY, TZ))
+    if (!planar_map(&xm, x, CIN, a.nx, a.ny, a.nz, a.nf, TX, HY, WZ + 2) ||
+        !planar_map(&ym, dy, NY, a.nx, a.ny, a.nz, a.nf, TX, TY, 1))
         return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<CIN, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess)
@@ -273,7 +279,7 @@ cudaError_t run(const void *x, const void *dy, const WgArgs &a, int grid, cudaSt
 
 int wgrad_ctas(int nx, int ny, int nz, int nf, int sm_count)
 {
-    const long long tiles = tc_tiles(nx, ny, nz, nf);
+    const long long tiles = (long long)((nx + TX - 1) / TX) * ((ny + TY - 1) / TY) * ((nz + WZ - 1) / WZ) * nf;
     return (int)(tiles < sm_count ? tiles : sm_count);
 }
 

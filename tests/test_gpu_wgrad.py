@@ -1,4 +1,4 @@
-"""The tensor-core weight gradient at the edges of its tiles (8 x 16 x 4
+"""The tensor-core weight gradient at the edges of its tiles (8 x 16 x 2
 voxels): crops smaller than a tile, partial tiles along every axis, one frame
 and several tiles per CTA (whose accumulators carry over).  The reference
 rounds to BF16 where the kernels do (weights, activations, the propagated

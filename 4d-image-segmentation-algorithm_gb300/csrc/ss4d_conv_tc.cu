@@ -363,10 +363,15 @@ cudaError_t conv_tc(int cin, int n, const void *x, const TcArgs &a, int sm_count
 // [9 (dy, dx)][KC][2 K groups][3N/8 N groups][8 rows][8 K] BF16, row
 // dz * N + co of block (dy, dx) holding tap 9 dz + 3 dy + dx; zero beyond
 // cout/cin
-__global__ void k_pack_tc(const float *__restrict__ w, int cout, int cin, int reverse, int cinp, int n,
-                          __nv_bfloat16 *out)
+// All of a network's blocks in one launch (blockIdx.y): seven of 3.3 us each
+// were 5 % of a training step.
+struct PackJobs {
+    PackJob v[MAX_PACKS];
+};
+__global__ void __launch_bounds__(256) k_pack_tc(const __grid_constant__ PackJobs jobs)
 {
-    const int kc_n = cinp / 16;
+    const PackJob &p = jobs.v[blockIdx.y];
+    const int kc_n = p.cinp / 16, n = p.n;
     const int total = 9 * kc_n * 2 * 3 * n * 8;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
         int r = q;
@@ -383,16 +388,16 @@ __global__ void k_pack_tc(const float *__restrict__ w, int cout, int cin, int re
         const int nr = 8 * j + row, dz = nr / n;
         const int tap = 9 * dz + dd, co = nr % n, ci = 16 * kc + 8 * h + e;
         float v = 0.f;
-        if (!reverse) {
-            if (co < cout && ci < cin)
-                v = w[((size_t)tap * cout + co) * cin + ci];
+        if (!p.reverse) {
+            if (co < p.cout && ci < p.cin)
+                v = p.w[((size_t)tap * p.cout + co) * p.cin + ci];
         } else {
             // data gradient: output channel co = the forward's input channel,
             // input channel ci = the forward's output channel
-            if (co < cin && ci < cout)
-                v = w[((size_t)(26 - tap) * cout + ci) * cin + co];
+            if (co < p.cin && ci < p.cout)
+                v = p.w[((size_t)(26 - tap) * p.cout + ci) * p.cin + co];
         }
-        out[q] = __float2bfloat16_rn(v);
+        p.out[q] = __float2bfloat16_rn(v);
     }
 }
 
@@ -411,9 +416,12 @@ void poison_if_err(const int *err, float *y, long long n, cudaStream_t st)
     k_poison_if_err<<<256, 256, 0, st>>>(err, y, n);
 }
 
-void pack_tc(const float *w, int cout, int cin, int reverse, int cinp, int n, __nv_bfloat16 *out, cudaStream_t st)
+void pack_tc(const PackJob *jobs, int njobs, cudaStream_t st)
 {
-    k_pack_tc<<<64, 256, 0, st>>>(w, cout, cin, reverse, cinp, n, out);
+    PackJobs p = {};
+    for (int q = 0; q < njobs && q < MAX_PACKS; ++q)
+        p.v[q] = jobs[q];
+    k_pack_tc<<<dim3(64, njobs), 256, 0, st>>>(p);
 }
 
 } // namespace tc

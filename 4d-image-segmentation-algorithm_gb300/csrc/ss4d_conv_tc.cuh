@@ -149,15 +149,28 @@ cudaError_t conv_tc(int cin, int n, const void *x, const TcArgs &a, int sm_count
 // weights W[27][cout][cin] FP32 -> the B blocks of a (cinp, n) convolution
 // (per (dy, dx, K chunk) the three dz taps stacked along N); reverse: the
 // data-gradient weights (taps reversed, channel roles swapped)
-void pack_tc(const float *w, int cout, int cin, int reverse, int cinp, int n, __nv_bfloat16 *out, cudaStream_t st);
+struct PackJob {
+    const float *w;
+    int cout, cin, reverse, cinp, n;
+    __nv_bfloat16 *out;
+};
+constexpr int MAX_PACKS = 8;
+void pack_tc(const PackJob *jobs, int njobs, cudaStream_t st);
 constexpr size_t packed_tc_elems(int cinp, int n) { return (size_t)27 * (cinp / 16) * 2 * n * 8; }
 // weight and bias gradient of one layer (ss4d_wgrad_tc.cu): x planar with cin
 // (16 or 32) channels of which cin_real count, dy planar with ycha (32 or 16)
 // channels of which cout count; gw [27][cout][cin_real] and gb [cout] FP32.
-// partial: wgrad_ctas() rows of 27 cout cin + cout floats
+// partial: wgrad_ctas() rows of 27 cout cin + cout floats, written by wgrad_tc;
+// reduce_grads adds the rows of several layers up into their gradients
+struct GradJob {
+    int cin, ycha, cout, cin_real;
+    float *partial, *gw, *gb;
+};
+constexpr int MAX_GRADS = 4;
 int wgrad_ctas(int nx, int ny, int nz, int nf, int sm_count);
-cudaError_t wgrad_tc(int cin, int ycha, int cout, int cin_real, const void *x, const void *dy, int nx, int ny, int nz,
-                     int nf, float *partial, float *gw, float *gb, int *err, int sm_count, cudaStream_t st);
+cudaError_t wgrad_tc(const GradJob &j, const void *x, const void *dy, int nx, int ny, int nz, int nf, int *err,
+                     int sm_count, cudaStream_t st);
+cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, cudaStream_t st);
 // y[0..n) <- NaN when *err is set (a convolution before it gave up a wait)
 void poison_if_err(const int *err, float *y, long long n, cudaStream_t st);
 

@@ -263,12 +263,15 @@ static ss4d_status pack_all(ss4d_wsnet *n)
 {
     size_t woff[4], boff[4];
     layer_offsets(woff, boff);
+    tc::PackJob jobs[tc::MAX_PACKS];
+    int q = 0;
     for (int L = 0; L < 4; ++L) {
         const Layer &l = kLayers[L];
-        tc::pack_tc(n->p + woff[L], l.cout, l.cin, 0, l.cinp, l.nout, n->wf[L], n->stream);
+        jobs[q++] = tc::PackJob{n->p + woff[L], l.cout, l.cin, 0, l.cinp, l.nout, n->wf[L]};
         if (L > 0) // data gradient: input = this layer's output gradient, output = its input channels
-            tc::pack_tc(n->p + woff[L], l.cout, l.cin, 1, l.coutp_t, 32, n->wt[L], n->stream);
+            jobs[q++] = tc::PackJob{n->p + woff[L], l.cout, l.cin, 1, l.coutp_t, 32, n->wt[L]};
     }
+    tc::pack_tc(jobs, q, n->stream);
     NCK(cudaGetLastError());
     return SS4D_OK;
 }
@@ -405,24 +408,35 @@ extern "C" ss4d_status ss4d_wsnet_forward(ss4d_wsnet *n, const void *d_x0, int n
     return forward(n, (const __nv_bfloat16 *)d_x0, nx, ny, nz, nf, false, d_out);
 }
 
-// the weight and bias gradient of layer L from its input x and output gradient dy
-static ss4d_status wgrad(ss4d_wsnet *n, int L, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, int nx, int ny, int nz,
-                         int nf, float *gw, float *gb)
+// the layers' weight-gradient jobs, their partial sums allocated
+static ss4d_status grad_jobs(ss4d_wsnet *n, int ctas, tc::GradJob jobs[4])
 {
-    const Layer &l = kLayers[L];
-    const size_t need = (size_t)tc::wgrad_ctas(nx, ny, nz, nf, n->sm) * (27 * 24 * 32 + 24); // the largest layer's
-    if (n->partial_cap < need) {
+    size_t woff[4], boff[4], part[5] = {0};
+    layer_offsets(woff, boff);
+    for (int L = 0; L < 4; ++L)
+        part[L + 1] = part[L] + (size_t)ctas * (27 * kLayers[L].cout * kLayers[L].cinp + kLayers[L].cout);
+    if (n->partial_cap < part[4]) {
         if (n->partial)
             cudaFree(n->partial);
         n->partial = nullptr;
         n->partial_cap = 0;
-        NCK(cudaMalloc((void **)&n->partial, need * 4));
-        n->partial_cap = need;
+        NCK(cudaMalloc((void **)&n->partial, part[4] * 4));
+        n->partial_cap = part[4];
     }
-    if (tc::wgrad_tc(l.cinp, l.coutp_t, l.cout, l.cin, x, dy, nx, ny, nz, nf, n->partial, gw, gb, n->err, n->sm,
-                     n->stream) != cudaSuccess)
-        n->launch_failed = 1;
+    for (int L = 0; L < 4; ++L) {
+        const Layer &l = kLayers[L];
+        jobs[L] = tc::GradJob{l.cinp, l.coutp_t, l.cout, l.cin, n->partial + part[L], n->g + woff[L], n->g + boff[L]};
+    }
     return SS4D_OK;
+}
+
+// the weight and bias gradient's partial sums of a layer from its input x and
+// output gradient dy
+static void wgrad(ss4d_wsnet *n, const tc::GradJob &j, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, int nx, int ny,
+                  int nz, int nf)
+{
+    if (tc::wgrad_tc(j, x, dy, nx, ny, nz, nf, n->err, n->sm, n->stream) != cudaSuccess)
+        n->launch_failed = 1;
 }
 
 // one Adam step on crops: x0 planar [F][2][nz][ny][nx][8] BF16 features, target
@@ -437,27 +451,27 @@ extern "C" ss4d_status ss4d_wsnet_train_step(ss4d_wsnet *n, const void *d_x0, co
     const __nv_bfloat16 *x0 = (const __nv_bfloat16 *)d_x0;
     if (forward(n, x0, nx, ny, nz, nf, true, nullptr) != SS4D_OK)
         return SS4D_ERR_CUDA;
-    size_t woff[4], boff[4];
-    layer_offsets(woff, boff);
+    const int ctas = tc::wgrad_ctas(nx, ny, nz, nf, n->sm);
+    tc::GradJob jobs[4];
+    if (grad_jobs(n, ctas, jobs) != SS4D_OK)
+        return SS4D_ERR_CUDA;
     const long long inner = (long long)(nx - 2 * margin) * (ny - 2 * margin) * (nz - 2 * margin) * nf;
     const int lb = 1024;
     k_mse<<<lb, 256, 0, n->stream>>>(n->y, d_target, nx, ny, nz, nf, margin, 1.f / (float)inner, n->dz16,
                                      n->loss_part);
     // layer 4 (3 -> out): weights and data gradient (masked by a3 > 0)
-    if (wgrad(n, 3, n->a[2], n->dz16, nx, ny, nz, nf, n->g + woff[3], n->g + boff[3]) != SS4D_OK)
-        return SS4D_ERR_CUDA;
+    wgrad(n, jobs[3], n->a[2], n->dz16, nx, ny, nz, nf);
     conv(n, 16, 32, 24, n->dz16, n->wt[3], nullptr, n->a[2], n->dz32[0], nullptr, nx, ny, nz, nf, 0);
     // layer 3
-    if (wgrad(n, 2, n->a[1], n->dz32[0], nx, ny, nz, nf, n->g + woff[2], n->g + boff[2]) != SS4D_OK)
-        return SS4D_ERR_CUDA;
+    wgrad(n, jobs[2], n->a[1], n->dz32[0], nx, ny, nz, nf);
     conv(n, 32, 32, 24, n->dz32[0], n->wt[2], nullptr, n->a[1], n->dz32[1], nullptr, nx, ny, nz, nf, 0);
     // layer 2
-    if (wgrad(n, 1, n->a[0], n->dz32[1], nx, ny, nz, nf, n->g + woff[1], n->g + boff[1]) != SS4D_OK)
-        return SS4D_ERR_CUDA;
+    wgrad(n, jobs[1], n->a[0], n->dz32[1], nx, ny, nz, nf);
     conv(n, 32, 32, 24, n->dz32[1], n->wt[1], nullptr, n->a[0], n->dz32[0], nullptr, nx, ny, nz, nf, 0);
     // layer 1
-    if (wgrad(n, 0, x0, n->dz32[0], nx, ny, nz, nf, n->g + woff[0], n->g + boff[0]) != SS4D_OK)
-        return SS4D_ERR_CUDA;
+    wgrad(n, jobs[0], x0, n->dz32[0], nx, ny, nz, nf);
+    if (tc::reduce_grads(jobs, 4, ctas, n->stream) != cudaSuccess)
+        n->launch_failed = 1;
     if (n->launch_failed)
         return nfail(SS4D_ERR_CUDA, "a tensor-core convolution could not be launched (tensor map or launch)");
     if (d_grad)

@@ -218,10 +218,16 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 }
 
 // the CTAs' partial sums, added in CTA order (eight interleaved runs of CTAs,
-// then the runs in order), into the master layout [27][cout][cin], [cout]
-__global__ void __launch_bounds__(256) k_reduce_grad(const float *__restrict__ partial, int rows, int cout, int cinp,
-                                                     int cin, float *gw, float *gb)
+// then the runs in order), into the master layout [27][cout][cin], [cout]; all
+// layers in one launch (blockIdx.y; one after the other they took 7 us each)
+struct GradJobs {
+    GradJob v[MAX_GRADS];
+};
+__global__ void __launch_bounds__(256) k_reduce_grad(const __grid_constant__ GradJobs jobs, int rows)
 {
+    const float *const partial = jobs.v[blockIdx.y].partial;
+    float *const gw = jobs.v[blockIdx.y].gw, *const gb = jobs.v[blockIdx.y].gb;
+    const int cout = jobs.v[blockIdx.y].cout, cinp = jobs.v[blockIdx.y].cin, cin = jobs.v[blockIdx.y].cin_real;
     __shared__ float part[8][33];
     const int n = 27 * cout * cin, cols = 27 * cout * cinp + cout;
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -283,29 +289,39 @@ int wgrad_ctas(int nx, int ny, int nz, int nf, int sm_count)
     return (int)(tiles < sm_count ? tiles : sm_count);
 }
 
-cudaError_t wgrad_tc(int cin, int ycha, int cout, int cin_real, const void *x, const void *dy, int nx, int ny, int nz,
-                     int nf, float *partial, float *gw, float *gb, int *err, int sm_count, cudaStream_t st)
+cudaError_t wgrad_tc(const GradJob &j, const void *x, const void *dy, int nx, int ny, int nz, int nf, int *err,
+                     int sm_count, cudaStream_t st)
 {
     WgArgs a;
     a.nx = nx;
     a.ny = ny;
     a.nz = nz;
     a.nf = nf;
-    a.cout = cout;
-    a.partial = partial;
+    a.cout = j.cout;
+    a.partial = j.partial;
     a.err = err;
     const int grid = wgrad_ctas(nx, ny, nz, nf, sm_count);
-    cudaError_t e = cudaErrorInvalidValue;
-    if (cin == 16 && ycha == 32)
-        e = run<16, 32>(x, dy, a, grid, st);
-    else if (cin == 32 && ycha == 32)
-        e = run<32, 32>(x, dy, a, grid, st);
-    else if (cin == 32 && ycha == 16)
-        e = run<32, 16>(x, dy, a, grid, st);
-    if (e != cudaSuccess)
-        return e;
-    const int n = 27 * cout * cin_real + cout;
-    k_reduce_grad<<<(n + 31) / 32, 256, 0, st>>>(partial, grid, cout, cin, cin_real, gw, gb);
+    if (j.cin == 16 && j.ycha == 32)
+        return run<16, 32>(x, dy, a, grid, st);
+    if (j.cin == 32 && j.ycha == 32)
+        return run<32, 32>(x, dy, a, grid, st);
+    if (j.cin == 32 && j.ycha == 16)
+        return run<32, 16>(x, dy, a, grid, st);
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, cudaStream_t st)
+{
+    if (njobs < 1 || njobs > MAX_GRADS)
+        return cudaErrorInvalidValue;
+    GradJobs g = {};
+    int most = 0;
+    for (int q = 0; q < njobs; ++q) {
+        g.v[q] = jobs[q];
+        const int n = 27 * jobs[q].cout * jobs[q].cin_real + jobs[q].cout;
+        most = n > most ? n : most;
+    }
+    k_reduce_grad<<<dim3((most + 31) / 32, njobs), 256, 0, st>>>(g, ctas);
     return cudaGetLastError();
 }
 

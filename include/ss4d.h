@@ -53,7 +53,7 @@ typedef enum ss4d_arith {
      * parity anchor (u agrees with the reference to rounding of pow()). */
     SS4D_ARITH_REFERENCE = 0,
     /* FP64 on a colour-split layout: fused residual, precomputed diagonal and
-     * relaxation factor, whole sweep loop in one CUDA graph.  The plain form. */
+     * relaxation factor, whole sweep loop in one launch.  The plain form. */
     SS4D_ARITH_FP64 = 1,
     /* FP32 red-black sweeps on the correction equation, FP64 residual,
      * convergence test and refinement of u; same FP64 stopping tolerance. */

@@ -403,16 +403,19 @@ __device__ __forceinline__ void voxel_coef(const Geo &g, const Split &sp, const 
     store_coef16(pick(b.coefq, col), pick(b.coefs, col), t, a32);
 }
 
+// One thread per voxel of a plane, i fastest across rows: blocks of rows'
+// chunks left 37 % of the lanes idle at nx = 161 (the step of 161 x 143 x 61 x 9
+// 6.15 ms, now 6.09).
 template <int PRE>
 __global__ void __launch_bounds__(256, PRE ? 6 : 8) k_voxel_coef_ff(Geo g, Split sp, FFConst K, SplitBufs b, int l_off,
-                                                                    PlaneOrder po)
+                                                                    FastDiv row, PlaneOrder po)
 {
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    const unsigned at = blockIdx.x * blockDim.x + threadIdx.x, jr = fdiv(at, row);
+    const int i = 1 + (int)(at - jr * row.d), j = 1 + (int)jr;
     int kk, lf;
     plane_frame(blockIdx.z, po, kk, lf);
     const int k = 1 + kk, l = 1 + l_off + lf;
-    if (i > g.nx || j > g.ny)
+    if (j > g.ny)
         return;
     const long long o = nat_index(g, i, j, k, l);
     const long long st[4] = {1, g.sy, g.sz, g.sw};
@@ -503,15 +506,13 @@ void launch_assemble_ff_faces_range(const Geo &g, const Split &s, CPtrs8 gin, in
         k_faces_ff<<<gr, dim3(FTX, FTY, 1), 0, st>>>(g, Hk, gin, has_g, K, b, f0, make_plane_order(Hk + 1, f1 - f0, kb));
     }
     if (v1 > v0) {
-        const int bx = g.nx >= 128 ? 128 : (g.nx >= 64 ? 64 : 32);
-        const int by = 256 / bx;
-        dim3 bl(bx, by, 1);
-        dim3 gr((g.nx + bx - 1) / bx, (g.ny + by - 1) / by, g.nz * (v1 - v0));
+        const dim3 gr(((unsigned)g.nx * g.ny + 255) / 256, 1, g.nz * (v1 - v0));
+        const FastDiv row = make_fastdiv((unsigned)g.nx);
         const PlaneOrder po = make_plane_order(g.nz, v1 - v0, kblock);
         if (pre)
-            k_voxel_coef_ff<1><<<gr, bl, 0, st>>>(g, s, K, b, v0 - 1, po);
+            k_voxel_coef_ff<1><<<gr, 256, 0, st>>>(g, s, K, b, v0 - 1, row, po);
         else
-            k_voxel_coef_ff<0><<<gr, bl, 0, st>>>(g, s, K, b, v0 - 1, po);
+            k_voxel_coef_ff<0><<<gr, 256, 0, st>>>(g, s, K, b, v0 - 1, row, po);
     }
 }
 

@@ -128,13 +128,13 @@ __global__ void __launch_bounds__(256) k_fdiff(Geo g, int Hk, FastDiv fpl, Split
 }
 
 // --- faces ------------------------------------------------------------------
-// A block takes a tile of FTX x FTY folded voxels (i, j) of one (m, l) plane.
+// A block takes a tile of FTX (32 or 16) x FTY folded voxels (i, j) of one (m, l) plane.
 // The central differences D_a of every voxel are formed once, by its own thread,
 // and the i- and j-faces read those of their upper neighbour from shared
 // memory (the tile plus one column and one row of halo); the k- and l-faces
 // form them at v + e_k and v + e_l.  Offsets are 32-bit (padded volumes below
 // 2^31 voxels).
-constexpr int FTX = 32, FTY = 8;
+constexpr int FTY = 8;
 
 // D_a(x) = F_a(x) + F_a(x - e_a), unnormalised (it is added again)
 __device__ __forceinline__ ff2 cdiff(const float4 *__restrict__ fa, unsigned x, unsigned sa)
@@ -231,8 +231,9 @@ __device__ __forceinline__ ff2 ghost_face_g(const CPtrs8 &gin, int has_g, unsign
 // Bound by the latency of its loads (issue 35 % busy, DRAM about half): 64
 // registers, four blocks per SM, 5.3 ms at 256^2 x 128 x 20; three blocks (80) or
 // five (48) took 0.2 and 0.6 ms more.  One voxel per thread, scalar, it took 5.9.
-__global__ void __launch_bounds__(FTX *FTY, 4) k_faces_ff(Geo g, int Hk, CPtrs8 gin, int has_g, FFConst K,
-                                                                     SplitBufs b, int l_off, PlaneOrder po)
+template <int FTX>
+__global__ void __launch_bounds__(FTX *FTY, 128 / FTX) k_faces_ff(Geo g, int Hk, CPtrs8 gin, int has_g, FFConst K,
+                                                                  SplitBufs b, int l_off, PlaneOrder po)
 {
     __shared__ float4 sD[4][FTY + 1][FTX + 1];
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -502,8 +503,17 @@ void launch_assemble_ff_faces_range(const Geo &g, const Split &s, CPtrs8 gin, in
     const int Hk = fold_of(g);
     const int kb = kblock <= 0 ? 0 : (kblock + 1) / 2; // folded planes
     if (f1 > f0) {
-        dim3 gr((g.nx + FTX - 1) / FTX, (g.ny + FTY - 1) / FTY, (Hk + 1) * (f1 - f0));
-        k_faces_ff<<<gr, dim3(FTX, FTY, 1), 0, st>>>(g, Hk, gin, has_g, K, b, f0, make_plane_order(Hk + 1, f1 - f0, kb));
+        // tiles 16 wide where they leave fewer lanes idle: 48 volumes of 24-48
+        // 19.0 -> 18.6 ms a run, a step of 161 x 143 x 61 x 9 6.09 -> 6.08; at 256
+        // wide their larger halo costs 0.5 % (228.4 -> 229.5 ms)
+        const bool narrow = (g.nx + 15) / 16 % 2 != 0;
+        const int w = narrow ? 16 : 32;
+        const dim3 gr((g.nx + w - 1) / w, (g.ny + FTY - 1) / FTY, (Hk + 1) * (f1 - f0)), bl(w, FTY, 1);
+        const PlaneOrder po = make_plane_order(Hk + 1, f1 - f0, kb);
+        if (narrow)
+            k_faces_ff<16><<<gr, bl, 0, st>>>(g, Hk, gin, has_g, K, b, f0, po);
+        else
+            k_faces_ff<32><<<gr, bl, 0, st>>>(g, Hk, gin, has_g, K, b, f0, po);
     }
     if (v1 > v0) {
         const dim3 gr(((unsigned)g.nx * g.ny + 255) / 256, 1, g.nz * (v1 - v0));

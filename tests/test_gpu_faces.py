@@ -11,7 +11,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 DIMS = [(31, 7, 3, 2), (32, 8, 4, 1), (33, 9, 5, 3), (8, 33, 2, 2), (9, 31, 1, 3), (17, 16, 6, 2), (40, 5, 7, 2),
-        (1, 40, 9, 1), (64, 64, 41, 4)]
+        (1, 40, 9, 1), (16, 9, 2, 2), (47, 7, 3, 2), (48, 8, 2, 3), (64, 64, 41, 4)]
 
 
 @pytest.mark.parametrize("h", [1.0, 0.5, 0.8])

@@ -533,6 +533,9 @@ __global__ void __cluster_dims__(RESCALE_CTAS, 1, 1) __launch_bounds__(256)
     const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) * RESCALE_CTAS;
     const int warp = (threadIdx.x >> 5) * RESCALE_CTAS + rank;
     const long long t2b = __double_as_longlong(t2);
+    // the other blocks' shared memory may be written only once they have all
+    // started, which a barrier of the cluster alone establishes
+    cluster.sync();
     for (int c = 0; c < count; ++c) {
         const double cx = bx[first + c], cy = by[first + c], cz = bz[first + c];
         const int k0 = (int)(cz - R - 0.5), j0 = (int)(cy - R - 0.5), i0 = (int)(cx - R - 0.5);

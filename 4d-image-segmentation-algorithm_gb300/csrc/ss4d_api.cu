@@ -705,7 +705,7 @@ static ss4d_status finish_stats(ss4d_solver *s, ss4d_step_stats *stats, int mixe
         stats->projected = mixed ? L.proj : 0;
     }
     if (L.status == SS4D_ERR_TIMEOUT) {
-        set_err("the persistent loop's barrier gave up a wait");
+        set_err("the persistent loop gave up: a barrier's wait ran out, or no stop within its limit of bodies");
         return SS4D_ERR_TIMEOUT;
     }
     if (L.status != SS4D_OK) {
@@ -990,9 +990,8 @@ static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixe
         CKS(dmalloc(s, (void **)&s->d_loop_parts, sizeof(double) * 4 * (a > b ? a : b)));
     }
     CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
-    const int bodies = mixed ? 4 * (p->maxNoGSIteration + 4) + 16 : p->maxNoGSIteration + 8;
     cudaError_t e = launch_loop(mixed, &V, 1, grid, LOOP_THREADS, s->d_state, s->d_params, s->d_loop_parts,
-                                s->d_group, bodies, s->loop_ahead[mixed], s->stream);
+                                s->d_group, loop_bodies(p->maxNoGSIteration, mixed), s->loop_ahead[mixed], s->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         s->loop_blocks[mixed] = -1; // from now on the graph's loop
@@ -1001,6 +1000,12 @@ static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixe
     s->launches += 1;
     *done = true;
     return SS4D_OK;
+}
+
+static ss4d_status loop_unended()
+{
+    set_err("the loop reached its limit of bodies without a stop");
+    return SS4D_ERR_TIMEOUT;
 }
 
 // the loop from the state the controller left (mode: that state's mode),
@@ -1034,7 +1039,9 @@ static ss4d_status drive_loop(ss4d_solver *s, const ss4d_params *p, int mixed, i
     }
     if (!graphed) {
         // host-driven form of the same loop: one small readback per iteration
-        for (int guard = 0; guard < 4 * (p->maxNoGSIteration + 4) + 16; ++guard) {
+        bool ended = false;
+        const int most = loop_bodies(p->maxNoGSIteration, mixed);
+        for (int body = 0; body < most && !ended; ++body) {
             if (!mixed) {
                 timed(s, SS4D_K_SWEEP64, true,
                       [&] { launch_sweep64(g, sp, cfg, 1, s->sb, s->d_params, s->d_state, s->stream); });
@@ -1060,10 +1067,11 @@ static ss4d_status drive_loop(ss4d_solver *s, const ss4d_params *p, int mixed, i
             CKS(last_launch());
             CK(cudaMemcpyAsync(s->h_state, s->d_state, sizeof(LoopState), cudaMemcpyDeviceToHost, s->stream));
             CK(cudaStreamSynchronize(s->stream));
-            if (s->h_state->stop || s->h_state->paused)
-                break;
+            ended = s->h_state->stop || s->h_state->paused;
             mode = s->h_state->mode;
         }
+        if (!ended)
+            return loop_unended();
     }
     s->last_graphed = graphed ? 1 : 0;
     return SS4D_OK;
@@ -1748,12 +1756,15 @@ extern "C" ss4d_status ss4d_seg_time_step_host(ss4d_solver *s, const ss4d_params
     // tolerance almost always does) that u is the step's result: only the
     // extrapolation history is left to write.  Otherwise the loop resumes and
     // the result of a later round goes down.
-    bool done = false;
-    for (int guard = 0; mixed && guard < 4 * (p->maxNoGSIteration + 4) + 16; ++guard) {
+    bool done = false, ended = !mixed;
+    const int most = loop_bodies(p->maxNoGSIteration, mixed); // at least one per round
+    for (int round = 0; round < most && !ended; ++round) {
         CK(cudaMemcpyAsync(s->h_state, s->d_state, sizeof(LoopState), cudaMemcpyDeviceToHost, s->stream));
         CK(cudaStreamSynchronize(s->stream));
-        if (s->h_state->stop || !s->h_state->paused)
-            break; // stopped at the step's first refinement pass: as without pausing
+        if (s->h_state->stop || !s->h_state->paused) {
+            ended = true; // stopped at the step's first refinement pass: as without pausing
+            break;
+        }
         CKS(download(UNPACK_PAUSED));
         CKS(refine_paused(s));
         CK(cudaMemcpyAsync(s->h_state, s->d_state, sizeof(LoopState), cudaMemcpyDeviceToHost, s->stream));
@@ -1764,7 +1775,7 @@ extern "C" ss4d_status ss4d_seg_time_step_host(ss4d_solver *s, const ss4d_params
                                     g.lM - 1, UNPACK_HISTORY);
                 s->launches += 1;
             }
-            done = true;
+            done = ended = true;
             break;
         }
         CKS(drive_loop(s, p, mixed, s->h_state->mode));
@@ -1775,6 +1786,8 @@ extern "C" ss4d_status ss4d_seg_time_step_host(ss4d_solver *s, const ss4d_params
     unpack_done(s, up);
     s->have_g = 0;
     ss4d_status st = finish_stats(s, stats, mixed);
+    if (!ended)
+        st = loop_unended();
     count_graph_launches(s);
     CK(cudaEventRecord(s->side_ev, s->side));
     CK(cudaStreamWaitEvent(s->stream, s->side_ev, 0));

@@ -934,9 +934,7 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
     int maxit = 0;
     for (int v = 0; v < b->n; ++v)
         maxit = p[v].maxNoGSIteration > maxit ? p[v].maxNoGSIteration : maxit;
-    // a mixed body advances a volume by at most one inner iteration, and
-    // every round adds a start and a refinement body
-    const int guard_max = b->mixed ? 4 * (maxit + 4) + 16 : maxit + 8;
+    const int most = loop_bodies(maxit, b->mixed);
     bool graphed = false, persisted = false;
     if (b->persistent) {
         BCKS(bdescribe_loop(b));
@@ -946,7 +944,7 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
             if (b->withhold_barrier) // arrival counts far below any target: no arrival completes a barrier
                 BCK(cudaMemset2DAsync(&b->d_groups->count, sizeof(LoopGroup), 0x80, sizeof(unsigned), b->n, b->stream));
             BCK(launch_loop(f, b->h_loop, b->n, b->pgrid[f], BLOOP_THREADS, b->d_st, b->d_par, b->d_loop_parts,
-                            b->d_groups, guard_max, false, b->stream));
+                            b->d_groups, most, false, b->stream));
             persisted = true;
         }
     }
@@ -964,7 +962,8 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
         }
     }
     if (!graphed && !persisted) {
-        for (int guard = 0; guard < guard_max; ++guard) {
+        int active = 1;
+        for (int body = 0; body < most && active; ++body) {
             if (b->mixed)
                 launch_body_mixed(b, 0, 0, b->stream);
             else
@@ -972,11 +971,14 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
             BCK(cudaGetLastError());
             BCK(cudaMemcpyAsync(b->h_st, b->d_st, sizeof(LoopState) * b->n, cudaMemcpyDeviceToHost, b->stream));
             BCK(cudaStreamSynchronize(b->stream));
-            int active = 0;
+            active = 0;
             for (int v = 0; v < b->n; ++v)
                 active += !b->h_st[v].stop;
-            if (!active)
-                break;
+        }
+        if (active) {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            return bfail(SS4D_ERR_TIMEOUT, "the batch's loop reached its limit of bodies without a stop");
         }
     }
     BCKS(each_volume(b, apart, [&](int v) { return solver_finish_step(b->vol[v], b->d_st + v, d_u[v]); }));
@@ -1004,7 +1006,7 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
             worst = (ss4d_status)L.status;
     }
     if (worst == SS4D_ERR_TIMEOUT)
-        return bfail(worst, "the persistent batch loop's barrier gave up a wait");
+        return bfail(worst, "the persistent batch loop gave up: a barrier's wait ran out, or no stop within its limit of bodies");
     if (worst != SS4D_OK)
         return bfail(worst, "a volume's SOR residual became non-finite");
     return SS4D_OK;

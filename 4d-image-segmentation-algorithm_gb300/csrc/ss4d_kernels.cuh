@@ -2,6 +2,8 @@
 // translation units and the host orchestration (ss4d_api.cu).
 #pragma once
 
+#include <limits.h>
+
 #include "ss4d_common.cuh"
 
 namespace ss4d {
@@ -281,6 +283,16 @@ ss4d_status solver_finish_step(ss4d_solver *s, const LoopState *d_state, double 
 ss4d_status solver_project_start(ss4d_solver *s, int pre, LoopState *d_state);
 // device time of `iters` (black + red) FP64 sweep pairs with the current shape
 ss4d_status solver_time_sweeps(ss4d_solver *s, const ss4d_params *p, int iters, float *ms);
+// More loop bodies than a loop of at most maxit iterations can take: an
+// iteration is a body, and in the mixed form every round, of one iteration at
+// least, adds a start and a refinement.  Whatever maxit is, a loop tests after
+// its first body, so that a limit of 0 or below counts as 1; one that stands
+// for "no limit" is formed in 64 bits and cut to what the kernels count.
+inline int loop_bodies(int maxit, int mixed)
+{
+    const long long n = maxit > 1 ? maxit : 1, most = mixed ? 4 * (n + 4) + 16 : n + 8;
+    return (int)(most < INT_MAX ? most : INT_MAX);
+}
 int solver_sm_count(const ss4d_solver *s);
 // what the handle launches from now on goes to `stream` (the caller orders it
 // against what went before)

@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(LOOP_MAX_THREADS, MIXED && AHEAD ? 1 : 2)
         }
     }
     if (rank == 0 && tid == 0) {
-        if (!good) {
+        if (!good || !(S.stop || (MIXED && S.paused))) { // a wait ran out, or the bodies did
             S.status = SS4D_ERR_TIMEOUT;
             S.stop = 1;
         }

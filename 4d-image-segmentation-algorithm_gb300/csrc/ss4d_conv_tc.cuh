@@ -161,7 +161,8 @@ constexpr size_t packed_tc_elems(int cinp, int n) { return (size_t)27 * (cinp / 
 // (16 or 32) channels of which cin_real count, dy planar with ycha (32 or 16)
 // channels of which cout count; gw [27][cout][cin_real] and gb [cout] FP32.
 // partial: wgrad_ctas() rows of 27 cout cin + cout floats, written by wgrad_tc;
-// reduce_grads adds the rows of several layers up into their gradients
+// reduce_grads adds the rows of several layers up into their gradients (NaN
+// where *err is set by then)
 struct GradJob {
     int cin, ycha, cout, cin_real;
     float *partial, *gw, *gb;
@@ -169,8 +170,8 @@ struct GradJob {
 constexpr int MAX_GRADS = 4;
 int wgrad_ctas(int nx, int ny, int nz, int nf, int sm_count);
 cudaError_t wgrad_tc(const GradJob &j, const void *x, const void *dy, int nx, int ny, int nz, int nf, int *err,
-                     int sm_count, cudaStream_t st);
-cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, cudaStream_t st);
+                     int withhold_loads, int sm_count, cudaStream_t st);
+cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, const int *err, cudaStream_t st);
 // y[0..n) <- NaN when *err is set (a convolution before it gave up a wait)
 void poison_if_err(const int *err, float *y, long long n, cudaStream_t st);
 

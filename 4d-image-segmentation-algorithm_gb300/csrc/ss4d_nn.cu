@@ -58,19 +58,23 @@ __global__ void k_mse(const float *__restrict__ out, const float *__restrict__ t
         partial[blockIdx.x] = acc;
 }
 
-// Adam on the FP32 master parameters
+// Adam on the FP32 master parameters; no update from a step whose gradient is
+// void (err: one of its kernels gave up a wait)
 __global__ void k_adam(float *p, const float *__restrict__ g, float *m, float *v, int n, float lr, float b1, float b2,
-                       float eps, float c1, float c2)
+                       float eps, float c1, float c2, const int *__restrict__ err)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const float gi = g[i];
+    const int failed = __ldg(err);
+    const float gi = g[i], pi = p[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+    if (failed)
+        return;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    p[i] = pi - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
 }
 
 } // namespace nn
@@ -129,13 +133,15 @@ ss4d_status nfail(ss4d_status st, const char *fmt, ...)
 
 } // namespace
 
+constexpr int LOSS_BLOCKS = 1024;
+
 struct ss4d_wsnet {
     cudaStream_t stream;
     int sm;
     size_t nparam;
     float *p, *g, *m, *v;          // master parameters, gradients, Adam moments (FP32, flat)
     __nv_bfloat16 *wf[4], *wt[4];  // forward / data-gradient weights as tcgen05 B operands (tc::pack_tc)
-    int *err;                      // set by a convolution that gave up a bounded wait (reset per forward)
+    int *err;                      // set by a kernel that gave up a bounded wait (reset per forward); follows the loss sums
     int withhold_loads;            // test of the timeout path (ss4d_wsnet_set_test_withhold_loads)
     float *bias[4];                // views into p
     // activations and gradients, sized for `cap` voxels
@@ -144,7 +150,7 @@ struct ss4d_wsnet {
     float *y;
     float *partial;                // weight-gradient partials
     size_t partial_cap;
-    float *loss_part;
+    float *loss_part;              // LOSS_BLOCKS sums
     float h_loss;
     long long step;
     int launch_failed;
@@ -174,7 +180,7 @@ extern "C" ss4d_status ss4d_wsnet_destroy(ss4d_wsnet *n)
         return SS4D_OK;
     cudaStreamSynchronize(n->stream);
     void *ptrs[] = {n->p, n->g, n->m, n->v, n->a[0], n->a[1], n->a[2], n->dz16, n->dz32[0], n->dz32[1], n->y,
-                    n->partial, n->loss_part, n->err};
+                    n->partial, n->loss_part};
     for (void *q : ptrs)
         if (q)
             cudaFree(q);
@@ -216,14 +222,13 @@ extern "C" ss4d_status ss4d_wsnet_create(void *stream, ss4d_wsnet **out)
         n->bias[L] = n->p + boff[L];
     }
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&n->err, sizeof(int));
-    if (e == cudaSuccess)
-        e = cudaMalloc((void **)&n->loss_part, 4096 * 4);
+        e = cudaMalloc((void **)&n->loss_part, (LOSS_BLOCKS + 1) * 4);
     if (e != cudaSuccess) {
         cudaGetLastError();
         ss4d_wsnet_destroy(n);
         return nfail(SS4D_ERR_ALLOC, "network allocation failed: %s", cudaGetErrorString(e));
     }
+    n->err = reinterpret_cast<int *>(n->loss_part + LOSS_BLOCKS);
     cudaMemsetAsync(n->m, 0, n->nparam * 4, n->stream);
     cudaMemsetAsync(n->v, 0, n->nparam * 4, n->stream);
     cudaMemsetAsync(n->err, 0, sizeof(int), n->stream);
@@ -243,8 +248,14 @@ extern "C" ss4d_status ss4d_wsnet_set_test_withhold_loads(ss4d_wsnet *n, int ena
 {
     if (!n)
         return nfail(SS4D_ERR_INVALID, "invalid argument: network is NULL");
-    n->withhold_loads = enable ? 1 : 0;
+    n->withhold_loads = enable;
     return SS4D_OK;
+}
+
+static ss4d_status gave_up()
+{
+    return nfail(SS4D_ERR_TIMEOUT, "a tensor-core kernel gave up a bounded wait: the prediction (a forward) or the "
+                                   "gradient (a training step, which updates nothing) was made NaN");
 }
 
 extern "C" ss4d_status ss4d_wsnet_check(ss4d_wsnet *n)
@@ -255,7 +266,7 @@ extern "C" ss4d_status ss4d_wsnet_check(ss4d_wsnet *n)
     NCK(cudaMemcpyAsync(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
     NCK(cudaStreamSynchronize(n->stream));
     if (h)
-        return nfail(SS4D_ERR_TIMEOUT, "a tensor-core convolution gave up a bounded wait; its output was made NaN");
+        return gave_up();
     return SS4D_OK;
 }
 
@@ -373,7 +384,7 @@ static void conv(ss4d_wsnet *n, int cin, int nout, int cout, const __nv_bfloat16
     a.mstride = 32;
     a.relu = relu;
     a.err = n->err;
-    a.withhold_loads = n->withhold_loads;
+    a.withhold_loads = n->withhold_loads == 1;
     if (tc::conv_tc(cin, nout, x, a, n->sm, n->stream) != cudaSuccess)
         n->launch_failed = 1;
 }
@@ -435,7 +446,7 @@ static ss4d_status grad_jobs(ss4d_wsnet *n, int ctas, tc::GradJob jobs[4])
 static void wgrad(ss4d_wsnet *n, const tc::GradJob &j, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, int nx, int ny,
                   int nz, int nf)
 {
-    if (tc::wgrad_tc(j, x, dy, nx, ny, nz, nf, n->err, n->sm, n->stream) != cudaSuccess)
+    if (tc::wgrad_tc(j, x, dy, nx, ny, nz, nf, n->err, n->withhold_loads != 0, n->sm, n->stream) != cudaSuccess)
         n->launch_failed = 1;
 }
 
@@ -456,8 +467,7 @@ extern "C" ss4d_status ss4d_wsnet_train_step(ss4d_wsnet *n, const void *d_x0, co
     if (grad_jobs(n, ctas, jobs) != SS4D_OK)
         return SS4D_ERR_CUDA;
     const long long inner = (long long)(nx - 2 * margin) * (ny - 2 * margin) * (nz - 2 * margin) * nf;
-    const int lb = 1024;
-    k_mse<<<lb, 256, 0, n->stream>>>(n->y, d_target, nx, ny, nz, nf, margin, 1.f / (float)inner, n->dz16,
+    k_mse<<<LOSS_BLOCKS, 256, 0, n->stream>>>(n->y, d_target, nx, ny, nz, nf, margin, 1.f / (float)inner, n->dz16,
                                      n->loss_part);
     // layer 4 (3 -> out): weights and data gradient (masked by a3 > 0)
     wgrad(n, jobs[3], n->a[2], n->dz16, nx, ny, nz, nf);
@@ -470,7 +480,7 @@ extern "C" ss4d_status ss4d_wsnet_train_step(ss4d_wsnet *n, const void *d_x0, co
     conv(n, 32, 32, 24, n->dz32[1], n->wt[1], nullptr, n->a[0], n->dz32[0], nullptr, nx, ny, nz, nf, 0);
     // layer 1
     wgrad(n, jobs[0], x0, n->dz32[0], nx, ny, nz, nf);
-    if (tc::reduce_grads(jobs, 4, ctas, n->stream) != cudaSuccess)
+    if (tc::reduce_grads(jobs, 4, ctas, n->err, n->stream) != cudaSuccess)
         n->launch_failed = 1;
     if (n->launch_failed)
         return nfail(SS4D_ERR_CUDA, "a tensor-core convolution could not be launched (tensor map or launch)");
@@ -481,19 +491,26 @@ extern "C" ss4d_status ss4d_wsnet_train_step(ss4d_wsnet *n, const void *d_x0, co
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.f / (1.f - powf(b1, (float)n->step)), c2 = 1.f / (1.f - powf(b2, (float)n->step));
         k_adam<<<(int)((n->nparam + 255) / 256), 256, 0, n->stream>>>(n->p, n->g, n->m, n->v, (int)n->nparam, lr, b1,
-                                                                       b2, 1e-8f, c1, c2);
+                                                                       b2, 1e-8f, c1, c2, n->err);
         if (pack_all(n) != SS4D_OK)
             return SS4D_ERR_CUDA;
     }
     NCK(cudaGetLastError());
     if (loss_out) {
-        float hp[1024];
-        NCK(cudaMemcpyAsync(hp, n->loss_part, sizeof hp, cudaMemcpyDeviceToHost, n->stream));
+        struct {
+            float part[LOSS_BLOCKS];
+            int err;
+        } h;
+        NCK(cudaMemcpyAsync(&h, n->loss_part, sizeof h, cudaMemcpyDeviceToHost, n->stream));
         NCK(cudaStreamSynchronize(n->stream));
         double s = 0;
-        for (int i = 0; i < lb; ++i)
-            s += hp[i];
+        for (int i = 0; i < LOSS_BLOCKS; ++i)
+            s += h.part[i];
         *loss_out = (float)(s / (double)inner);
+        if (h.err) {
+            n->step -= lr > 0.f; // no update was made
+            return gave_up();
+        }
     }
     return SS4D_OK;
 }

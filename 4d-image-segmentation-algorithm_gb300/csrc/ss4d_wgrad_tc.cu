@@ -63,6 +63,7 @@ struct WgArgs {
     int nx, ny, nz, nf, cout;
     float *partial; // [CTA][27 cout CIN + cout]
     int *err;
+    int withhold_loads; // test of the timeout path: issue no load, so that the wait for it runs out
 };
 
 template <int CIN, int NY>
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             };
             bool ok = true;
             int loads = 0, mmas = 0;
-            for (int it = 0; it < 2 && it < my_n; ++it, ++loads)
+            for (int it = 0; it < 2 && it < my_n && !a.withhold_loads; ++it, ++loads)
                 load(it);
             for (int it = 0; it < my_n; ++it) {
                 const int b = it & 1;
@@ -219,15 +220,19 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 
 // the CTAs' partial sums, added in CTA order (eight interleaved runs of CTAs,
 // then the runs in order), into the master layout [27][cout][cin], [cout]; all
-// layers in one launch (blockIdx.y; one after the other they took 7 us each)
+// layers in one launch (blockIdx.y; one after the other they took 7 us each).
+// A kernel of the step that gave up a wait (err) left rows, or what they were
+// formed from, unwritten: the gradient is NaN then.
 struct GradJobs {
     GradJob v[MAX_GRADS];
 };
-__global__ void __launch_bounds__(256) k_reduce_grad(const __grid_constant__ GradJobs jobs, int rows)
+__global__ void __launch_bounds__(256) k_reduce_grad(const __grid_constant__ GradJobs jobs, int rows,
+                                                     const int *__restrict__ err)
 {
     const float *const partial = jobs.v[blockIdx.y].partial;
     float *const gw = jobs.v[blockIdx.y].gw, *const gb = jobs.v[blockIdx.y].gb;
     const int cout = jobs.v[blockIdx.y].cout, cinp = jobs.v[blockIdx.y].cin, cin = jobs.v[blockIdx.y].cin_real;
+    const int failed = __ldg(err);
     __shared__ float part[8][33];
     const int n = 27 * cout * cin, cols = 27 * cout * cinp + cout;
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -243,6 +248,8 @@ __global__ void __launch_bounds__(256) k_reduce_grad(const __grid_constant__ Gra
     if (g == 0 && q < n + cout) {
         for (int k = 1; k < 8; ++k)
             s += part[k][lane];
+        if (failed)
+            s = __int_as_float(0x7fffffff);
         if (q < n)
             gw[q] = s;
         else
@@ -290,7 +297,7 @@ int wgrad_ctas(int nx, int ny, int nz, int nf, int sm_count)
 }
 
 cudaError_t wgrad_tc(const GradJob &j, const void *x, const void *dy, int nx, int ny, int nz, int nf, int *err,
-                     int sm_count, cudaStream_t st)
+                     int withhold_loads, int sm_count, cudaStream_t st)
 {
     WgArgs a;
     a.nx = nx;
@@ -300,6 +307,7 @@ cudaError_t wgrad_tc(const GradJob &j, const void *x, const void *dy, int nx, in
     a.cout = j.cout;
     a.partial = j.partial;
     a.err = err;
+    a.withhold_loads = withhold_loads;
     const int grid = wgrad_ctas(nx, ny, nz, nf, sm_count);
     if (j.cin == 16 && j.ycha == 32)
         return run<16, 32>(x, dy, a, grid, st);
@@ -310,7 +318,7 @@ cudaError_t wgrad_tc(const GradJob &j, const void *x, const void *dy, int nx, in
     return cudaErrorInvalidValue;
 }
 
-cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, cudaStream_t st)
+cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, const int *err, cudaStream_t st)
 {
     if (njobs < 1 || njobs > MAX_GRADS)
         return cudaErrorInvalidValue;
@@ -321,7 +329,7 @@ cudaError_t reduce_grads(const GradJob *jobs, int njobs, int ctas, cudaStream_t 
         const int n = 27 * jobs[q].cout * jobs[q].cin_real + jobs[q].cout;
         most = n > most ? n : most;
     }
-    k_reduce_grad<<<dim3((most + 31) / 32, njobs), 256, 0, st>>>(g, ctas);
+    k_reduce_grad<<<dim3((most + 31) / 32, njobs), 256, 0, st>>>(g, ctas, err);
     return cudaGetLastError();
 }
 

@@ -813,14 +813,16 @@ class Wsnet:
         _check(self.L.ss4d_wsnet_forward(self.h, _ptr(x0), nx, ny, nz, nf, _ptr(out)), "wsnet_forward")
 
     def check(self):
-        """synchronise; SS4DError (SS4D_ERR_TIMEOUT) if a convolution of the
-        last forward gave up a bounded wait"""
+        """synchronise; SS4DError (SS4D_ERR_TIMEOUT) if a kernel of the last
+        forward (and any backward after it) gave up a bounded wait"""
         _check(self.L.ss4d_wsnet_check(self.h), "wsnet_check")
 
-    def set_test_withhold_loads(self, on: bool):
-        """test of the timeout path: the convolutions issue no loads, so their
-        waits run out and the prediction is NaN"""
-        _check(self.L.ss4d_wsnet_set_test_withhold_loads(self.h, 1 if on else 0), "wsnet_set_test_withhold_loads")
+    def set_test_withhold_loads(self, on: bool, weight_gradients_only: bool = False):
+        """test of the timeout path: the convolutions and weight gradients (or
+        these alone) issue no loads, so their waits run out and the prediction
+        and the gradient (or the gradient alone) are NaN"""
+        _check(self.L.ss4d_wsnet_set_test_withhold_loads(self.h, (2 if weight_gradients_only else 1) if on else 0),
+               "wsnet_set_test_withhold_loads")
 
     def train_step(self, x0, target, nx: int, ny: int, nz: int, nf: int, margin: int = 0, lr: float = 1e-3,
                    grad=None) -> float:

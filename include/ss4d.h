@@ -479,16 +479,20 @@ ss4d_status ss4d_wsnet_get_params(ss4d_wsnet *n, float *h_params);
  * convolution whose bounded wait (about a second) gave up makes the whole
  * prediction NaN, which the warm start's check discards. */
 ss4d_status ss4d_wsnet_forward(ss4d_wsnet *n, const void *d_x0, int nx, int ny, int nz, int nf, float *d_out);
-/* Synchronise the network's stream; SS4D_ERR_TIMEOUT if a convolution of the
- * last forward (and any backward after it) gave up a wait, else SS4D_OK. */
+/* Synchronise the network's stream; SS4D_ERR_TIMEOUT if a kernel of the last
+ * forward (and any backward after it) gave up a wait, else SS4D_OK. */
 ss4d_status ss4d_wsnet_check(ss4d_wsnet *n);
-/* Test of the timeout path, no fault: with enable the convolutions issue no
- * halo loads, so each one's waits run out after about a second and its
- * output is made NaN. */
+/* Test of the timeout path, no fault: with enable 1 the convolutions and the
+ * weight gradients issue no loads, with enable 2 the weight gradients alone, so
+ * each one's waits run out after about a second and the prediction and the
+ * gradient, or the gradient alone, are made NaN. */
 ss4d_status ss4d_wsnet_set_test_withhold_loads(ss4d_wsnet *n, int enable);
 /* one Adam step on a batch of crops (frames F of nx*ny*nz voxels): mean
  * squared error against d_target over voxels at least `margin` from a crop's
- * border; lr == 0 only evaluates; d_grad (may be NULL) gets the gradient. */
+ * border; lr == 0 only evaluates; d_grad (may be NULL) gets the gradient.
+ * A kernel that gave up a wait makes the whole gradient NaN and the step
+ * updates nothing; with loss_out, for which the call synchronises, the step
+ * returns SS4D_ERR_TIMEOUT, else ss4d_wsnet_check does. */
 ss4d_status ss4d_wsnet_train_step(ss4d_wsnet *n, const void *d_x0, const float *d_target, int nx, int ny,
                                   int nz, int nf, int margin, float lr, float *loss_out, float *d_grad);
 /* Features of the time step from d_u (training data): assembles the step's

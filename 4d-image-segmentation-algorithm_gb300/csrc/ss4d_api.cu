@@ -94,6 +94,7 @@ struct ss4d_solver {
     int sm_count;
     int use_graph;
     int max_grid; // ss4d_solver_set_tiling's cap on the loop's grid (0: none)
+    int withhold_barrier; // test of the timeout path (ss4d_solver_set_test_withhold_barrier)
     int asm_kblock; // block order of the float-float faces and coefficient kernels (launch_assemble_ff_faces_range)
     long long launches;
     size_t bytes;
@@ -705,6 +706,7 @@ static ss4d_status finish_stats(ss4d_solver *s, ss4d_step_stats *stats, int mixe
         stats->projected = mixed ? L.proj : 0;
     }
     if (L.status == SS4D_ERR_TIMEOUT) {
+        s->have_dprev = 0; // the step left no change to extrapolate from
         set_err("the persistent loop gave up: a barrier's wait ran out, or no stop within its limit of bodies");
         return SS4D_ERR_TIMEOUT;
     }
@@ -968,6 +970,20 @@ static bool loop_persistent(const ss4d_solver *s, int mixed)
     return !mixed || s->geo.nint <= LOOP_MIXED_MAX_VOXELS;
 }
 
+// the barrier of a persistent launch to come: no arrivals yet (the test of the
+// timeout path: counts far below any target, which no arrival reaches).  The
+// launch takes the pointer from here: the barrier is allocated at first use.
+static ss4d_status reset_group(ss4d_solver *s, LoopGroup **group)
+{
+    if (!s->d_group)
+        CKS(dmalloc(s, (void **)&s->d_group, sizeof(LoopGroup)));
+    CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
+    if (s->withhold_barrier)
+        CK(cudaMemsetAsync(&s->d_group->count, 0x80, sizeof(unsigned), s->stream));
+    *group = s->d_group;
+    return SS4D_OK;
+}
+
 // launches it from the state in d_state; *done = false when it cannot run here
 static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixed, bool *done)
 {
@@ -983,15 +999,14 @@ static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixe
     if (s->max_grid > 0 && grid > s->max_grid)
         grid = s->max_grid;
     share_blocks(&V, 1, grid);
-    if (!s->d_group)
-        CKS(dmalloc(s, (void **)&s->d_group, sizeof(LoopGroup)));
     if (!s->d_loop_parts) {
         const int a = loop_grid(0, 1, LOOP_THREADS, s->sm_count), b = loop_grid(1, 1, LOOP_THREADS, s->sm_count);
         CKS(dmalloc(s, (void **)&s->d_loop_parts, sizeof(double) * 4 * (a > b ? a : b)));
     }
-    CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
+    LoopGroup *group;
+    CKS(reset_group(s, &group));
     cudaError_t e = launch_loop(mixed, &V, 1, grid, LOOP_THREADS, s->d_state, s->d_params, s->d_loop_parts,
-                                s->d_group, loop_bodies(p->maxNoGSIteration, mixed), s->loop_ahead[mixed], s->stream);
+                                group, loop_bodies(p->maxNoGSIteration, mixed), s->loop_ahead[mixed], s->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         s->loop_blocks[mixed] = -1; // from now on the graph's loop
@@ -1097,6 +1112,13 @@ static void count_graph_launches(ss4d_solver *s)
 {
     if (s->last_graphed)
         s->launches += 2LL * s->h_state->bodies + 3LL * s->h_state->opened;
+}
+
+extern "C" ss4d_status ss4d_solver_set_test_withhold_barrier(ss4d_solver *s, int enable)
+{
+    REQ(s, "solver is NULL");
+    s->withhold_barrier = enable ? 1 : 0;
+    return SS4D_OK;
 }
 
 extern "C" ss4d_status ss4d_solver_set_timing(ss4d_solver *s, int enable)
@@ -1217,8 +1239,6 @@ static ss4d_status presmooth_queue(ss4d_solver *s, const ss4d_params *p, double 
         CKS(dmalloc(s, (void **)&s->d_front, 2 * sizeof(FrontState)));
         CK(cudaMallocHost((void **)&s->h_front, 2 * sizeof(FrontState)));
     }
-    if (!s->d_group)
-        CKS(dmalloc(s, (void **)&s->d_group, sizeof(LoopGroup)));
     if (!s->d_front_parts) {
         const int a = presmooth_ff_grid(s->sm_count), b = presmooth64_grid(s->sm_count);
         CKS(dmalloc(s, (void **)&s->d_front_parts, sizeof(double) * 4 * (a > b ? a : b)));
@@ -1250,12 +1270,11 @@ static ss4d_status presmooth_queue(ss4d_solver *s, const ss4d_params *p, double 
     a.band = mixed ? fabs(p->gsTol) * 1e-6 : near_band(p->gsTol, g.nint);
     a.last = last;
     a.parts = s->d_front_parts;
-    a.group = s->d_group;
+    CKS(reset_group(s, &a.group));
     a.st = s->d_front + slot;
     const int threads = mixed ? FRONT_FF_THREADS : FRONT64_THREADS;
     const long long need = ((long long)a.F.npairs + threads - 1) / threads;
     const int grid = need < most ? (int)need : most;
-    CK(cudaMemsetAsync(s->d_group, 0, sizeof(LoopGroup), s->stream));
     CK(mixed ? launch_presmooth_ff(a, grid, s->stream) : launch_presmooth64(a, grid, s->stream));
     s->launches += 1;
     return SS4D_OK;
@@ -2146,6 +2165,11 @@ ss4d_status ss4d::solver_finish_step(ss4d_solver *s, const LoopState *d_state, d
     ss4d_status st = unpack_step(s, d_state, d_u, mixed);
     s->have_g = 0;
     return st;
+}
+
+void ss4d::solver_drop_history(ss4d_solver *s)
+{
+    s->have_dprev = 0;
 }
 
 ss4d_status ss4d::solver_time_sweeps(ss4d_solver *s, const ss4d_params *p, int iters, float *ms)

@@ -1002,6 +1002,8 @@ extern "C" ss4d_status ss4d_batch_seg_time_step(ss4d_batch *b, const ss4d_params
             stats[v].projected = b->mixed ? L.proj : 0;
             stats[v].ms = ms;
         }
+        if (L.status == SS4D_ERR_TIMEOUT)
+            solver_drop_history(b->vol[v]);
         if (L.status != SS4D_OK && worst != SS4D_ERR_TIMEOUT)
             worst = (ss4d_status)L.status;
     }

@@ -281,6 +281,8 @@ ss4d_status solver_finish_step(ss4d_solver *s, const LoopState *d_state, double 
 // whose state is *d_state, when the step's assembly applied the
 // extrapolation (pre == 2 from solver_prepare_step); nothing otherwise
 ss4d_status solver_project_start(ss4d_solver *s, int pre, LoopState *d_state);
+// the last step failed: it left no change to extrapolate from
+void solver_drop_history(ss4d_solver *s);
 // device time of `iters` (black + red) FP64 sweep pairs with the current shape
 ss4d_status solver_time_sweeps(ss4d_solver *s, const ss4d_params *p, int iters, float *ms);
 // More loop bodies than a loop of at most maxit iterations can take: an

@@ -396,8 +396,10 @@ __global__ void k_unpack(Geo g, Split sp, SplitBufs b, const LoopState *__restri
         if (terms >= 3)
             p2 = h2[s];
     }
-    const int fr = st->final_red;
+    const int fr = st->final_red, status = st->status;
     const double v = col == 0 ? pick(b.R, fr)[s] : b.Bk[s];
+    if (status == SS4D_ERR_TIMEOUT) // no result: u and the history stay
+        return;
     if (what != UNPACK_HISTORY)
         u[nat_index(g, i, j, k, l)] = v;
     if (terms > 0) {

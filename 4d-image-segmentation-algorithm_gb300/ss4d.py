@@ -190,6 +190,7 @@ def lib() -> C.CDLL:
         "ss4d_solver_set_stream": ([vp, vp], st),
         "ss4d_solver_set_arith": ([vp, C.c_int], st),
         "ss4d_solver_set_graph": ([vp, C.c_int], st),
+        "ss4d_solver_set_test_withhold_barrier": ([vp, C.c_int], st),
         "ss4d_solver_workspace_bytes": ([vp, C.POINTER(C.c_size_t)], st),
         "ss4d_solver_set_timing": ([vp, C.c_int], st),
         "ss4d_solver_set_tiling": ([vp, C.c_int, C.c_int], st),
@@ -435,6 +436,11 @@ class Solver:
 
     def set_graph(self, on: bool):
         _check(self.L.ss4d_solver_set_graph(self.h, 1 if on else 0), "set_graph")
+
+    def set_test_withhold_barrier(self, on: bool):
+        """test of the timeout path: no arrival completes a persistent
+        launch's barriers, so their waits run out (SS4D_ERR_TIMEOUT)"""
+        _check(self.L.ss4d_solver_set_test_withhold_barrier(self.h, 1 if on else 0), "set_test_withhold_barrier")
 
     def set_inner_omega(self, omega: float):
         """mixed form: relaxation factor of the FP32 sweeps (0: the step's omega_c)"""

@@ -41,7 +41,9 @@ typedef enum ss4d_status {
     SS4D_ERR_ALLOC = 2,       /* a device/host allocation failed (reference: _allocateMem_ returns false) */
     SS4D_ERR_CUDA = 3,        /* a CUDA runtime call failed; text via ss4d_last_error() */
     SS4D_ERR_NONFINITE = 4,   /* the SOR residual became NaN or Inf */
-    SS4D_ERR_TIMEOUT = 5,     /* a bounded device-side wait gave up */
+    SS4D_ERR_TIMEOUT = 5,     /* a bounded device-side wait gave up, or a loop its limit of bodies.  A time step
+                               * or solve on device arrays then leaves u's interior as it was and drops the
+                               * handle's history of changes; what other calls write is undefined */
     SS4D_ERR_UNSUPPORTED = 6, /* combination not built (e.g. unknown arithmetic mode) */
     SS4D_ERR_NO_DEVICE = 7    /* no CUDA device visible */
 } ss4d_status;
@@ -174,6 +176,12 @@ ss4d_status ss4d_solver_set_inner_omega(ss4d_solver *s, double omega);
  * loop) or drive it from the host, one readback per iteration (0).  Results
  * do not depend on it except through the residual's summation order. */
 ss4d_status ss4d_solver_set_graph(ss4d_solver *s, int enable);
+/* Test of the timeout path, no fault: with enable the barriers of the
+ * persistent loop and of the presmoothing start with arrival counts that no
+ * arrival brings to the number awaited; every block's first wait runs out
+ * after about a second and the call returns SS4D_ERR_TIMEOUT with the context
+ * usable. */
+ss4d_status ss4d_solver_set_test_withhold_barrier(ss4d_solver *s, int enable);
 /* Per-kernel timing.  While enabled, the sweep loop runs host-driven (not
  * as a graph) and every launch of the kernels below is bracketed by CUDA
  * events on the handle's stream; totals accumulate until reset. */

@@ -1265,9 +1265,13 @@ static ss4d_status presmooth_queue(ss4d_solver *s, const ss4d_params *p, double 
     a.h4 = p->h * p->h * p->h * p->h;
     a.tol = p->gsTol;
     a.maxit = p->maxNoGSIteration_sigma;
-    // float-float form: a residual is formed to about 1e-7 of itself in FP32
-    // squares, so a test within 1e-6 of gsTol is reported as near the tolerance
-    a.band = mixed ? fabs(p->gsTol) * 1e-6 : near_band(p->gsTol, g.nint);
+    // FP64 form: the order of the sum (and the squares' scaling by h^4 after
+    // it), and five roundings of values up to d U, at 2^-53 each, between this
+    // residual and the reference's.  Float-float form: the squares are summed
+    // in FP32 to about 1e-7, and the values differ from FP64's by about 1e-14.
+    a.near.rel = mixed ? 1e-6 : (double)(g.nint + 4) * 0x1p-53;
+    a.near.eps = mixed ? 0x1p-44 : 5.0 * 0x1p-53;
+    a.near.n = (double)g.nint;
     a.last = last;
     a.parts = s->d_front_parts;
     CKS(reset_group(s, &a.group));

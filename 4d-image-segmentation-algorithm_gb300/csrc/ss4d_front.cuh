@@ -28,6 +28,23 @@ struct FrontState {
     double R, R1;
 };
 
+// A stop test is reported as near the tolerance where the reference's sum
+// R' of the same residuals could lie on its other side.  With n residuals r,
+// R = h^4 sum r^2 and e the bound of what one residual's rounding may differ
+// by, |R' - R| <= rel R + 2 h^4 e sum |r| + n h^4 e^2, and sum |r| <= sqrt(n)
+// sqrt(sum r^2): rel stands for the order of the sum.  e = eps d U: a residual
+// is formed from values of at most d U, with U the largest |u|.  Where the
+// residuals are r, U <= max |image| + max |r| (the smoothing's matrix is
+// diagonally dominant by 1), and max |r| <= sqrt(R / h^4).
+struct FrontNear {
+    double rel, eps, n;
+};
+__host__ __device__ inline double front_near_band(const FrontNear &f, double d, double h4, double most, double R)
+{
+    const double e = f.eps * d * (most + sqrt(R / h4));
+    return f.rel * R + 2.0 * e * sqrt(f.n * R * h4) + f.n * h4 * e * e;
+}
+
 struct FrontArgs {
     Geo g;
     FlatIndex F;
@@ -36,7 +53,8 @@ struct FrontArgs {
     void *fold;            // float-float form: the smoothed image for the g faces (ss4d_front_ff.cu), or null
     int Hk;                // its fold
     float fold_scale;      // and the power of two it is scaled by
-    double c, omega, d, y, h4, tol, maxit, band; // d = 1 + 8c, y its reciprocal (FP64 form: for div_by_const)
+    double c, omega, d, y, h4, tol, maxit; // d = 1 + 8c, y its reciprocal (FP64 form: for div_by_const)
+    FrontNear near;
     int last; // the residual after the last iteration is wanted
     double *parts;
     LoopGroup *group;
@@ -56,6 +74,8 @@ __device__ __forceinline__ void presmooth_body(const FrontArgs &a)
     const Geo &g = a.g;
     __shared__ FrontState S;
     __shared__ int ok, stop;
+    __shared__ unsigned top;
+    __shared__ double gap; // the least |R - tol| of the tests
     const int tid = threadIdx.x;
     const unsigned nb = gridDim.x, rank = blockIdx.x, dq = nb * blockDim.x;
     unsigned target = 0;
@@ -66,7 +86,10 @@ __device__ __forceinline__ void presmooth_body(const FrontArgs &a)
         S.near = S.status = 0;
         S.R = S.R1 = 0.0;
         stop = 0;
+        top = 0;
+        gap = INFINITY;
     }
+    __syncthreads();
     auto put = [&](int colour, double acc) {
         acc = block_sum(acc);
         if (tid == 0)
@@ -106,6 +129,7 @@ __device__ __forceinline__ void presmooth_body(const FrontArgs &a)
             }
         }
     }
+    unsigned high = 0; // of the largest |value|: its upper word
     // split copy: columns x, x + 1 of both colours from the voxels 2x + 1 .. 2x + 4
     for (unsigned q = q0; q < F.npairs; q += dq) {
         int j, k, l;
@@ -116,10 +140,19 @@ __device__ __forceinline__ void presmooth_body(const FrontArgs &a)
 #pragma unroll
         for (int m = 0; m < 4; ++m)
             v[m] = i + m <= F.nx ? src[m] : 0.0;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            high = max(high, (unsigned)__double2hiint(v[m]) & 0x7fffffffu);
         // colour 0 has row phase t.p here, colour 1 the other
         static_cast<Q *>(a.P[t.p ? 0 : 1])[t.s >> 1] = A::make(v[0], v[2]);
         static_cast<Q *>(a.P[t.p ? 1 : 0])[t.s >> 1] = A::make(v[1], v[3]);
     }
+    high = __reduce_max_sync(0xffffffffu, high);
+    if ((tid & 31) == 0)
+        atomicMax(&top, high);
+    __syncthreads();
+    if (tid == 0)
+        atomicMax(&a.group->top, top);
     if (!sync(-1, 0.0)) {
         if (rank == 0 && tid == 0)
             a.st->status = SS4D_ERR_TIMEOUT;
@@ -196,8 +229,7 @@ __device__ __forceinline__ void presmooth_body(const FrontArgs &a)
                 S.R = R;
                 if (z == 1)
                     S.R1 = R;
-                if (fabs(R - a.tol) <= a.band)
-                    S.near = 1;
+                gap = fmin(gap, fabs(R - a.tol));
                 if (R > a.tol && z < a.maxit)
                     S.z = z + 1;
                 else
@@ -209,6 +241,8 @@ __device__ __forceinline__ void presmooth_body(const FrontArgs &a)
         good = ok;
     }
     if (rank == 0 && tid == 0) {
+        const double most = __hiloint2double((int)(__ldcg(&a.group->top) + 1), 0); // the next value above
+        S.near = isfinite(gap) && gap <= front_near_band(a.near, a.d, a.h4, most, fmax(a.tol, 0.0) + gap);
         S.status = good ? (isfinite(S.R) ? SS4D_OK : SS4D_ERR_NONFINITE) : SS4D_ERR_TIMEOUT;
         *a.st = S;
     }

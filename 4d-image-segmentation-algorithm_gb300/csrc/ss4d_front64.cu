@@ -1,9 +1,12 @@
 // ss4d_front64.cu — the presmoothing in the reference's FP64 arithmetic
 // (ss4d_front.cuh).  Compiled with --fmad=false: every multiply and add is
 // rounded as in the reference's build, and the voxel update keeps its
-// expression order (segmentation4D.c:366-384), so the image equals the
-// reference's bit for bit; only the residual's terms are added in another
-// order (and unscaled by h^4 until their sum is complete).
+// expression order (segmentation4D.c:366-384), so after the same number of
+// iterations the image equals the reference's bit for bit.  The stop test's
+// sum differs in rounding: a residual is formed with one rounding from the
+// update's own sum instead of three, and the terms are added in another
+// order (and unscaled by h^4 until their sum is complete).  Where that could
+// decide a test the other way it is reported (FrontNear).
 //
 // Bound by the FP64 pipe: 16 instructions per target for the update and 2 for
 // its residual, which the separate residual pass formed with 15.4 per voxel

@@ -20,7 +20,8 @@ struct LoopVol {
 struct LoopGroup {
     unsigned count;
     int err;
-    int pad_[30]; // one 128-byte line per group
+    unsigned top; // presmoothing: upper word of the image's largest |value|
+    int pad_[29]; // one 128-byte line per group
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p)

@@ -113,7 +113,9 @@ typedef struct ss4d_step_stats {
     int    near_tolerance;  /* 1 when a stop test saw |sum - gsTol| within nint * 2^-53
                                * gsTol: the reference's serial sum of the same terms
                                * could have decided that test the other way (one
-                               * iteration more or fewer); reported, not corrected   */
+                               * iteration more or fewer); reported, not corrected.
+                               * Presmoothing: within that and what the terms' own
+                               * rounding may differ by                              */
     int    projected;       /* mixed form: 1 when the first FP32 round started from the
                                projection onto the previous steps' changes
                                (ss4d_solver_set_projection)                          */

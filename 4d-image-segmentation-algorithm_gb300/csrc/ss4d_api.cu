@@ -1000,8 +1000,7 @@ static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixe
         grid = s->max_grid;
     share_blocks(&V, 1, grid);
     if (!s->d_loop_parts) {
-        const int a = loop_grid(0, 1, LOOP_THREADS, s->sm_count), b = loop_grid(1, 1, LOOP_THREADS, s->sm_count);
-        CKS(dmalloc(s, (void **)&s->d_loop_parts, sizeof(double) * 4 * (a > b ? a : b)));
+        CKS(dmalloc(s, (void **)&s->d_loop_parts, sizeof(double) * 4 * loop_most_blocks(LOOP_THREADS, s->sm_count)));
     }
     LoopGroup *group;
     CKS(reset_group(s, &group));

@@ -453,6 +453,16 @@ int loop_grid(int mixed, int nv, int threads, int sm_count)
     return resident(loop_kernel(mixed, nv, false), threads, sm_count);
 }
 
+int loop_most_blocks(int threads, int sm_count)
+{
+    int most = 0;
+    for (int q = 0; q < 4; ++q) {
+        const int n = resident(loop_kernel(q & 1, 1, q & 2), threads, sm_count);
+        most = n > most ? n : most;
+    }
+    return most;
+}
+
 // AHEAD up to three rounds per phase, in the FP64 form only where the warp it
 // gives up costs no further round (us of a step, plain -> AHEAD):
 //   FP64   32^3 x 8 (1 round) 571 -> 562, 45 x 37 x 29 x 7 (2) 722 -> 697,

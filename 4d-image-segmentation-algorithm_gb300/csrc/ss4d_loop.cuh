@@ -57,6 +57,8 @@ __device__ __forceinline__ bool group_wait(LoopGroup *gr, unsigned target)
 LoopVol make_loop_vol(const Geo &g, const Split &sp, const SplitBufs &b);
 // co-resident blocks of k_loop with that many threads on the device (0: unknown)
 int loop_grid(int mixed, int nv, int threads, int sm_count);
+// the most blocks any form of one volume's k_loop has with that many threads
+int loop_most_blocks(int threads, int sm_count);
 // the grid of one volume's k_loop, and whether it is the AHEAD form (0: unknown)
 int loop_plan(int mixed, const FlatIndex &F, int threads, int sm_count, bool *ahead);
 // deals `grid` blocks out to the volumes in proportion to their targets

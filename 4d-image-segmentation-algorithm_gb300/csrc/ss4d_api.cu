@@ -125,7 +125,7 @@ struct ss4d_solver {
     // the persistent loop (ss4d_loop.cu): its barrier and partial sums
     LoopGroup *d_group;
     double *d_loop_parts;
-    int loop_blocks[2];  // its grid per form; 0: not known, -1: the graph's loop instead
+    int loop_blocks[2];  // its grid per form; 0: not known, -1: it cannot run here (run_persistent)
     bool loop_ahead[2];  // its form (loop_plan)
     // rescale balls
     int *d_frame_first, *d_frame_count;
@@ -984,7 +984,10 @@ static ss4d_status reset_group(ss4d_solver *s, LoopGroup **group)
     return SS4D_OK;
 }
 
-// launches it from the state in d_state; *done = false when it cannot run here
+// Launches it from the state in d_state.  *done = false where the device cannot
+// hold its grid at once or has no such launch: the mixed form's loop is then the
+// graph's, the FP64 form's the host-driven one, with a readback per iteration.
+// Any other error of the launch is the call's.
 static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixed, bool *done)
 {
     *done = false;
@@ -1004,13 +1007,16 @@ static ss4d_status run_persistent(ss4d_solver *s, const ss4d_params *p, int mixe
     }
     LoopGroup *group;
     CKS(reset_group(s, &group));
-    cudaError_t e = launch_loop(mixed, &V, 1, grid, LOOP_THREADS, s->d_state, s->d_params, s->d_loop_parts,
-                                group, loop_bodies(p->maxNoGSIteration, mixed), s->loop_ahead[mixed], s->stream);
-    if (e != cudaSuccess) {
+    const cudaError_t loop_launch =
+        launch_loop(mixed, &V, 1, grid, LOOP_THREADS, s->d_state, s->d_params, s->d_loop_parts, group,
+                    loop_bodies(p->maxNoGSIteration, mixed), s->loop_ahead[mixed], s->stream);
+    if (loop_launch == cudaErrorCooperativeLaunchTooLarge || loop_launch == cudaErrorLaunchOutOfResources ||
+        loop_launch == cudaErrorNotSupported) {
         cudaGetLastError();
-        s->loop_blocks[mixed] = -1; // from now on the graph's loop
+        s->loop_blocks[mixed] = -1;
         return SS4D_OK;
     }
+    CK(loop_launch);
     s->launches += 1;
     *done = true;
     return SS4D_OK;
@@ -1234,10 +1240,10 @@ static ss4d_status presmooth_queue(ss4d_solver *s, const ss4d_params *p, double 
     const Geo &g = s->geo;
     const int mixed = s->arith == SS4D_ARITH_MIXED;
     const int most = mixed ? presmooth_ff_grid(s->sm_count) : presmooth64_grid(s->sm_count);
-    if (!s->d_front) {
+    if (!s->d_front)
         CKS(dmalloc(s, (void **)&s->d_front, 2 * sizeof(FrontState)));
+    if (!s->h_front)
         CK(cudaMallocHost((void **)&s->h_front, 2 * sizeof(FrontState)));
-    }
     if (!s->d_front_parts) {
         const int a = presmooth_ff_grid(s->sm_count), b = presmooth64_grid(s->sm_count);
         CKS(dmalloc(s, (void **)&s->d_front_parts, sizeof(double) * 4 * (a > b ? a : b)));

@@ -441,12 +441,11 @@ template <int PACK>
 static void run_fdiff(const Geo &g, const Split &s, const double *u, const SplitBufs &b, int l0, int l1, int sm_count,
                       cudaStream_t st, int withd)
 {
-    static int per_sm = 0;
-    if (!per_sm) {
+    static const int per_sm = [] { // once, whichever thread steps first
         int a = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_fdiff<PACK>, 256, 0);
-        per_sm = a > 0 ? a : 1;
-    }
+        return a > 0 ? a : 1;
+    }();
     const int Hk = fold_of(g);
     const unsigned frame = (unsigned)(g.iM * g.jM) * (Hk + 2), n = frame * (unsigned)(l1 - l0);
     const unsigned need = (n + 255) / 256, most = (unsigned)(sm_count * per_sm);

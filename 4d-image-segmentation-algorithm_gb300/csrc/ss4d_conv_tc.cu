@@ -286,17 +286,17 @@ __global__ void __launch_bounds__(32 * (EPI_WARPS + 1), 1) k_conv_tc(const __gri
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-        else
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-    }
+            p = nullptr;
+        }
+        return (PFN_cuTensorMapEncodeTiled_v12000)p;
+    }();
     return fn;
 }
 
@@ -305,13 +305,12 @@ template <int CIN, int N, int W>
 cudaError_t launch_warps(const CUtensorMap &m, const TcArgs &a, long long tiles, int sm_count, cudaStream_t st)
 {
     constexpr int threads = 32 * (W + 1);
-    static int per_sm = 0;
-    if (!per_sm) {
+    static const int per_sm = [] { // once, whichever thread comes first
         cudaFuncSetAttribute(k_conv_tc<CIN, N, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<CIN, N>::SMEM);
         int p = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k_conv_tc<CIN, N, W>, threads, TcCfg<CIN, N>::SMEM);
-        per_sm = p < 1 ? 1 : (p > 2 ? 2 : p); // tensor memory: 2 x TCOLS <= 512 columns
-    }
+        return p < 1 ? 1 : (p > 2 ? 2 : p); // tensor memory: 2 x TCOLS <= 512 columns
+    }();
     const long long cap = (long long)sm_count * per_sm;
     const int grid = (int)(tiles < cap ? tiles : cap);
     k_conv_tc<CIN, N, W><<<grid, threads, TcCfg<CIN, N>::SMEM, st>>>(m, a);

@@ -328,12 +328,11 @@ void launch_projection(const Geo &g, const Split &sp, const SweepCfg &cfg, Split
     const SweepCfg pc = make_pair_cfg(g, sp, cfg);
     // co-resident blocks only (at most the solver's grid, whose partial
     // buffer part is sized for)
-    static int per_sm = 0;
-    if (!per_sm) {
+    static const int per_sm = [] { // once, whichever thread steps first
         int a = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_proj_dots, 256, 0);
-        per_sm = a < 1 ? 1 : a;
-    }
+        return a < 1 ? 1 : a;
+    }();
     // per colour: blocks beyond the sampled tiles would add zeros
     const long long tiles = (pc.ntiles + PROJ_STRIDE - 1) / PROJ_STRIDE;
     int grid = sm_count * per_sm;

@@ -731,6 +731,8 @@ class Batch:
         return P, U, G
 
     def autotune(self, params, us, gs):
+        """tile shapes of the loops that walk tiles (set_persistent(False)):
+        the persistent loop, the default, has none"""
         P, U, G = self._args(params, us, gs)
         xt = (C.c_int * self.n)()
         kb = (C.c_int * self.n)()

@@ -823,8 +823,8 @@ def batch_line(args, steps, warmup, forms_arg, config="16x_64-192", sequential=F
     """Independent volumes (BATCH_CONFIGS: 16 of U[64..192] x U[64..192] x
     U[48..96] x U[8..24] per axis by default), single-ellipsoid scenes with
     per-volume K in [500, 2000] and tau in [0.25, 1], stepped together (the
-    SOR loop of all volumes in one persistent launch, per-volume convergence,
-    autotuned tile shapes), in the forms of --forms among fp64, mixed, extrap
+    SOR loop of all volumes in one persistent launch, per-volume convergence;
+    with --batch-loop graph the graph's loop on autotuned tile shapes), in the forms of --forms among fp64, mixed, extrap
     (mixed with the cubic extrapolated start) and proj (extrap with the
     projected start of each first round), each from the same
     start; `value` is the FP64 form's (or the first form's) aggregate
@@ -869,7 +869,9 @@ def batch_line(args, steps, warmup, forms_arg, config="16x_64-192", sequential=F
         if form in ("extrap", "proj"):
             B.set_extrapolation(EXTRAP_ORDER)
         B.set_projection(form == "proj")
-        if shapes is None:
+        if args.batch_loop == "persistent":
+            pass  # no tiles
+        elif shapes is None:
             shapes = B.autotune(params, us, gs)
         else:
             for v, (xt, kb) in enumerate(shapes):

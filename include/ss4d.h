@@ -450,10 +450,12 @@ ss4d_status ss4d_batch_set_projection(ss4d_batch *b, int enable);
  * one, whose walk has none): xt threads along x (power of two, 8..256; 0 =
  * automatic) and k-block depth k_block (>= 1).  Results do not depend on it. */
 ss4d_status ss4d_batch_set_shape(ss4d_batch *b, int v, int xt, int k_block);
-/* Autotuner: for every volume, time candidate tile shapes on that volume's
- * own sweeps (coefficients of d_u[v], d_g[8v..8v+7]; u is not modified) and
- * keep the fastest.  xt_out/kb_out (n entries each, may be NULL) receive the
- * chosen shapes. */
+/* Autotuner of the loops that walk tiles: for every volume, time candidate
+ * tile shapes on that volume's own sweeps (coefficients of d_u[v],
+ * d_g[8v..8v+7]; u is not modified) and keep the fastest, as
+ * ss4d_batch_set_shape would.  The persistent loop, the default, has no tiles
+ * and gains nothing by it: it is for ss4d_batch_set_persistent(b, 0).
+ * xt_out/kb_out (n entries each, may be NULL) receive the chosen shapes. */
 ss4d_status ss4d_batch_autotune(ss4d_batch *b, const ss4d_params *p, double *const *d_u,
                                 const double *const *d_g, int *xt_out, int *kb_out);
 /* One time step of every volume: parameters p[v], u d_u[v] (updated in

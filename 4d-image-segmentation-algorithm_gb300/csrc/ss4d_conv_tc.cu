@@ -54,21 +54,30 @@ namespace tc {
 
 // ---- the kernel ---------------------------------------------------------------
 
-// warp roles: warps 0-3 (or 0-7: warps w and w + 4 reach the same 32 lanes
+// warp roles: warps 0-3 (MASKED 0-7: warps w and w + 4 reach the same 32 lanes
 // of tensor memory and take half of the planes each) read the accumulators
-// and store; lane 0 of the last warp issues the loads and the MMAs.  Barriers, one phase per use: full[s] (the loads of the tile in
-// halo stage s landed), done[b] (the MMAs of the tile in accumulator buffer
+// and store; lane 0 of the last warp issues the loads and the MMAs.  Barriers,
+// one phase per use: full[s] (the loads of the tile in halo stage s landed), done[b] (the MMAs of the tile in accumulator buffer
 // b completed: tcgen05.commit), free[b] (the epilogue warps have read
 // buffer b).  Tile it uses stage it % STAGES and buffer it % 2.
 // A data gradient's epilogue loads its masks, 64 bytes a voxel: with eight
 // warps and the masks loaded ahead 51 -> 30 us per hidden layer at 8 crops of
-// 40x40x20 (four tiles per CTA).  Without masks, or over many tiles, the
+// 40x40x20 (four tiles per CTA).  A training step (three such convolutions
+// among its eleven products) took with four and with eight, in us: 2 tiles per SM
+// 234 and 228, 8 593 and 583, 16 1117 and 1086, 32 2112 and 2061, 63 4076 and
+// 3980; 4 frames of 128x128x64 (54) 3595 and 3521.  Without masks the
 // tensor core's operand reads set the pace and four warps, whose tensor-memory
 // reads are spread out, disturb them less (a forward of 12 frames of
 // 128x128x64 3.64 ms against 3.73).
-template <int CIN, int N, int EPI_WARPS>
-__global__ void __launch_bounds__(32 * (EPI_WARPS + 1), 1) k_conv_tc(const __grid_constant__ CUtensorMap tmap, TcArgs a)
+__host__ __device__ constexpr int epi_warps(bool masked)
 {
+    return masked ? 8 : 4;
+}
+template <int CIN, int N, bool MASKED>
+__global__ void __launch_bounds__(32 * (epi_warps(MASKED) + 1), 1)
+    k_conv_tc(const __grid_constant__ CUtensorMap tmap, TcArgs a)
+{
+    constexpr int EPI_WARPS = epi_warps(MASKED);
     using C = TcCfg<CIN, N>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -218,16 +227,14 @@ __global__ void __launch_bounds__(32 * (EPI_WARPS + 1), 1) k_conv_tc(const __gri
             int x0, y0, z0, f;
             tile_xyzf(it, x0, y0, z0, f);
             const int ox = x0 + (m & 7), oy = y0 + (m >> 3);
-            MaskRegs<N> mask[EPI_WARPS == 8 ? PL : 1];
-            auto masks = [&](int p) {
-                const int oz = z0 + p0 + p;
-                if (a.mask && ox < a.nx && oy < a.ny && oz < a.nz)
-                    load_masks<N>(a, mask[EPI_WARPS == 8 ? p : 0], f, ((long long)oz * a.ny + oy) * a.nx + ox, vol);
-            };
-            if (EPI_WARPS == 8) { // the masks come while the tensor core works on the tile
+            MaskRegs<N> mask[MASKED ? PL : 1];
+            if (MASKED) { // the masks come while the tensor core works on the tile
 #pragma unroll
-                for (int p = 0; p < PL; ++p)
-                    masks(p);
+                for (int p = 0; p < PL; ++p) {
+                    const int oz = z0 + p0 + p;
+                    if (ox < a.nx && oy < a.ny && oz < a.nz)
+                        load_masks<N>(a, mask[p], f, ((long long)oz * a.ny + oy) * a.nx + ox, vol);
+                }
             }
             // one lane waits, so that the warp stays converged for the
             // .sync.aligned tensor-memory loads
@@ -256,10 +263,10 @@ __global__ void __launch_bounds__(32 * (EPI_WARPS + 1), 1) k_conv_tc(const __gri
                 }
                 const int oz = z0 + p0 + p;
                 if (ox < a.nx && oy < a.ny && oz < a.nz)
-                    epilogue_store<N, EPI_WARPS == 8>(a, v, mask[EPI_WARPS == 8 ? p : 0], f,
-                                                      ((long long)oz * a.ny + oy) * a.nx + ox, vol);
+                    epilogue_store<N, MASKED>(a, v, mask[MASKED ? p : 0], f,
+                                              ((long long)oz * a.ny + oy) * a.nx + ox, vol);
             };
-            if (EPI_WARPS == 8) {
+            if (MASKED) {
 #pragma unroll
                 for (int p = 0; p < PL; ++p)
                     plane(p);
@@ -301,19 +308,19 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 }
 
 namespace {
-template <int CIN, int N, int W>
-cudaError_t launch_warps(const CUtensorMap &m, const TcArgs &a, long long tiles, int sm_count, cudaStream_t st)
+template <int CIN, int N, bool MASKED>
+cudaError_t launch_masked(const CUtensorMap &m, const TcArgs &a, long long tiles, int sm_count, cudaStream_t st)
 {
-    constexpr int threads = 32 * (W + 1);
+    constexpr int threads = 32 * (epi_warps(MASKED) + 1);
     static const int per_sm = [] { // once, whichever thread comes first
-        cudaFuncSetAttribute(k_conv_tc<CIN, N, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<CIN, N>::SMEM);
+        cudaFuncSetAttribute(k_conv_tc<CIN, N, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<CIN, N>::SMEM);
         int p = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k_conv_tc<CIN, N, W>, threads, TcCfg<CIN, N>::SMEM);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k_conv_tc<CIN, N, MASKED>, threads, TcCfg<CIN, N>::SMEM);
         return p < 1 ? 1 : (p > 2 ? 2 : p); // tensor memory: 2 x TCOLS <= 512 columns
     }();
     const long long cap = (long long)sm_count * per_sm;
     const int grid = (int)(tiles < cap ? tiles : cap);
-    k_conv_tc<CIN, N, W><<<grid, threads, TcCfg<CIN, N>::SMEM, st>>>(m, a);
+    k_conv_tc<CIN, N, MASKED><<<grid, threads, TcCfg<CIN, N>::SMEM, st>>>(m, a);
     return cudaGetLastError();
 }
 } // namespace
@@ -342,8 +349,8 @@ static cudaError_t launch(const void *x, const TcArgs &a, int sm_count, cudaStre
     if (!make_map(&m, x, CIN, a.nx, a.ny, a.nz, a.nf))
         return cudaErrorInvalidValue;
     const long long tiles = tc_tiles(a.nx, a.ny, a.nz, a.nf);
-    return a.mask && tiles <= 16LL * sm_count ? launch_warps<CIN, N, 8>(m, a, tiles, sm_count, st)
-                                              : launch_warps<CIN, N, 4>(m, a, tiles, sm_count, st);
+    return a.mask ? launch_masked<CIN, N, true>(m, a, tiles, sm_count, st)
+                  : launch_masked<CIN, N, false>(m, a, tiles, sm_count, st);
 }
 
 cudaError_t conv_tc(int cin, int n, const void *x, const TcArgs &a, int sm_count, cudaStream_t st)

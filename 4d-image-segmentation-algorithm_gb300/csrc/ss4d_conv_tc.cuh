@@ -88,11 +88,11 @@ __device__ __forceinline__ void load_masks(const TcArgs &a, MaskRegs<N> &m, int 
             m.q[c / 8] = __ldg(reinterpret_cast<const uint4 *>(a.mask + planar_off(f, c, a.mstride / 8, vol, vf)));
 }
 
-// one voxel's N accumulated channels -> bias, ReLU, mask (loaded AHEAD, or
-// here) -> global; voxel vf of frame f, vol voxels per frame
-template <int N, bool AHEAD>
-__device__ __forceinline__ void epilogue_store(const TcArgs &a, float (&v)[N], MaskRegs<N> &mask, int f, long long vf,
-                                               long long vol)
+// one voxel's N accumulated channels -> bias, ReLU, mask -> global; voxel vf of
+// frame f, vol voxels per frame
+template <int N, bool MASKED>
+__device__ __forceinline__ void epilogue_store(const TcArgs &a, float (&v)[N], const MaskRegs<N> &mask, int f,
+                                               long long vf, long long vol)
 {
 #pragma unroll
     for (int c = 0; c < N; ++c) {
@@ -103,9 +103,7 @@ __device__ __forceinline__ void epilogue_store(const TcArgs &a, float (&v)[N], M
             x = fmaxf(x, 0.f);
         v[c] = x;
     }
-    if (a.mask) {
-        if (!AHEAD)
-            load_masks<N>(a, mask, f, vf, vol);
+    if (MASKED) {
 #pragma unroll
         for (int c = 0; c < N; c += 8) {
             if (c >= a.mstride)

@@ -8,7 +8,9 @@ coefficient assembly, the SOR solve, the per-step rescale.  Inputs (about
 25 GB of working set) are far larger than the 129 MB L2, so no flush is
 needed between steps.
 
-Prints ONE JSON line on rank 0.  `--impl reference` times the reference's
+Prints ONE JSON line on rank 0 (a few kilobytes: figures per form and
+component; the full record with every iteration count goes to standard error,
+after "full record: ").  `--impl reference` times the reference's
 CPU algorithm instead (the compiled reference where it runs, else the C
 oracle that restates it), on all host cores.
 
@@ -53,10 +55,9 @@ EXTRAP_ORDER = 3  # the extrap form's order (ss4d_solver_set_extrapolation)
 BYTES_ASSEMBLY = 152.0
 # DRAM bytes per interior voxel of the mixed form's three assembly kernels
 # (first differences with the pack, faces, coefficient records with the first
-# refinement pass's residual), one ncu capture at 128x128x64x8: 82.7 + 142.9
-# + 190.5 (the first-difference kernel's 62.2 B per padded voxel counted per
-# interior voxel)
-TRAFFIC_ASSEMBLY = 416.1
+# refinement pass's residual), one ncu capture at 128x128x64x8: 78.2 + 145.2
+# + 188.7
+TRAFFIC_ASSEMBLY = 412.1
 TRAFFIC_PER_TARGET = {"k_sweep32": 39.8, "k_sweep64": 118.6}
 FP64_INSTR_PER_TARGET = 11.4  # k_sweep64, ncu at 128x128x64x8
 TRAFFIC_SOURCE = {"k_sweep32": "ncu capture of two launches at 256x256x128x20",
@@ -422,8 +423,9 @@ def run_ours(args, rank, world, dist):
                 "avg_ms_per_step": avg,
                 "note": "float-float arithmetic on the FP32 pipe; beyond the algorithmic bytes the kernels move "
                         "their intermediates (first differences, face quantities), the FP32 sweep records, the "
-                        "split copies of u and the first refinement pass's residual; the coefficient kernel is "
-                        "bound by the FP64 pipe (18 FP64 instructions per voxel), the faces kernel by issue"}
+                        "split copies of u and the first refinement pass's residual; the first-difference and faces "
+                        "kernels run at 64 % of the copy rate in DRAM bytes (FP64 pipe, load latency), the "
+                        "coefficient kernel at 83 %"}
 
     # error of the mixed forms against the plain FP64 form after the same steps
     err = {}
@@ -973,6 +975,50 @@ def run_conv(args):
                       "config": {"workload": f"random features {nx}x{ny}x{nz}x{nf}", "flop_per_voxel": flop // vox}}))
 
 
+def short_line(line):
+    """the record without its long parts: a line of 25 kB was cut by a reader
+    of standard output, and nothing of it could be read"""
+    def pick(d, *keys):
+        return {k: d[k] for k in keys if k in d}
+
+    out = {k: v for k, v in line.items()
+           if k == "roofline" or k == "roofline_fp64" or k == "roofline_assembly" or not k.startswith("roofline_")}
+    if "forms" in out:
+        out["forms"] = {f: dict(pick(r, "steps_per_s", "ms_per_step", "iterations_per_step", "converged"),
+                                **({"steps100": pick(r["steps100"], "steps_per_s", "iterations_mean")}
+                                   if "steps100" in r else {})) for f, r in out["forms"].items()}
+    if "error_vs_fp64" in out and out["error_vs_fp64"]:
+        out["error_vs_fp64"] = {f: pick(e, "max_rel", "mask_dice") for f, e in out["error_vs_fp64"].items()}
+    if "roofline_fp64" in out:
+        out["roofline_fp64"] = {k: v for k, v in out["roofline_fp64"].items() if k not in ("kernel_ms", "traffic_source")}
+        if out["roofline_fp64"].get("fp64_pipe"):
+            out["roofline_fp64"]["fp64_pipe"] = pick(out["roofline_fp64"]["fp64_pipe"], "instr_per_target", "frac")
+    if "parity_config3" in out:
+        out["cpu_baseline"] = {k: v for k, v in out["cpu_baseline"].items() if k != "parity_config3"}
+    for key in ("frontend", "frontend_mixed"):
+        if key in out:
+            f = out[key]
+            out[key] = dict({k: v for k, v in f.items() if k != "components"},
+                            component_ms={c: v["ms"] for c, v in f["components"].items()})
+    if "batch" in out:
+        def batch(b):
+            return dict(pick(b, "value", "unit", "ms_per_step"), workload=b["config"]["workload"],
+                        forms={f: dict(pick(r, "ms_per_step", "max_residual", "tolerance_met"),
+                                       **({"speedup_over_sequential": r["sequential"]["batch_speedup"]}
+                                          if "sequential" in r else {})) for f, r in b["forms"].items()},
+                        **({"small_volumes": batch(b["small_volumes"])} if "small_volumes" in b else {}))
+        out["batch"] = batch(out["batch"])
+
+    def digits(v):
+        if isinstance(v, dict):
+            return {k: digits(e) for k, e in v.items()}
+        if isinstance(v, list):
+            return [digits(e) for e in v]
+        return float(f"{v:.7g}") if isinstance(v, float) else v
+
+    return digits(out)
+
+
 def main():
     args = parse_args()
     rank = int(os.environ.get("RANK", 0))
@@ -1070,7 +1116,8 @@ def main():
     if dist:
         dist.destroy_process_group()
     if rank == 0:
-        print(json.dumps(line))
+        print("full record: " + json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(short_line(line)))
 
 
 if __name__ == "__main__":

@@ -228,8 +228,8 @@ __device__ __forceinline__ ff2 ghost_face_g(const CPtrs8 &gin, int has_g, unsign
 // between v and v + e_d have v and v + e_d in the extended box: all four for
 // interior v, the one along a where v's index along a is 0 (and none where
 // two indices are); frames l_off .. l_off + gridDim.z / (Hk + 1) - 1.
-// Bound by the latency of its loads (issue 35 % busy, DRAM about half): 64
-// registers, four blocks per SM, 5.3 ms at 256^2 x 128 x 20; three blocks (80) or
+// Bound by the latency of its loads (at 128 x 128 x 64 x 8 issue 45 % busy, 64 %
+// of the copy rate in DRAM bytes, 46 % of the warps): 64 registers, four blocks per SM, 5.3 ms at 256^2 x 128 x 20; three blocks (80) or
 // five (48) took 0.2 and 0.6 ms more.  One voxel per thread, scalar, it took 5.9.
 template <int FTX>
 __global__ void __launch_bounds__(FTX *FTY, 128 / FTX) k_faces_ff(Geo g, int Hk, CPtrs8 gin, int has_g, FFConst K,

@@ -8,7 +8,7 @@
 // order (and unscaled by h^4 until their sum is complete).  Where that could
 // decide a test the other way it is reported (FrontNear).
 //
-// Bound by the FP64 pipe: 16 instructions per target for the update and 2 for
+// Bound by the FP64 pipe (80 % busy): 16 instructions per target for the update and 2 for
 // its residual, which the separate residual pass formed with 15.4 per voxel
 // (the edge detector of two images of 97 x 101 x 53 x 11: 7.84 ms with 4, 7.39 with 2).
 // Two blocks of 256 per SM (90 registers, none spilled): 6.96 ms; three 7.16,

@@ -157,11 +157,13 @@ struct PairFF {
     }
 };
 
-// 62 registers, two blocks of 512 per SM: at 256^2 x 128 x 20 an image takes
-// 12.4 ms (10 iterations at 1.1 ms, the copies 1.6), at three blocks of 256 14.0, at
-// four of them 12.8, at five (48 registers) 13.6.  A half-sweep moves 2.7 GB
-// (0.40 ms at the copy rate) and keeps the FP32 pipe half busy; the kernels it
-// replaces (one thread per target, a residual pass) took 28 ms per image.
+// 62 registers, two blocks of 512 per SM.  At 256^2 x 128 x 20 an image takes
+// 13.1 ms; among launch shapes tried side by side two blocks of 512 took 12.4,
+// three of 256 14.0, four of them 12.8, five (48 registers) 13.6.  A half-sweep
+// has to move 2.7 GB (0.40 ms at the copy rate); at 192^2 x 96 x 12 the launch
+// runs at 83 % of the copy rate in DRAM bytes, its issue slots 48 % busy.  The
+// kernels it replaces (one thread per target, a residual pass) took 28 ms per
+// image.
 __global__ void __launch_bounds__(FRONT_FF_THREADS, 2) k_presmooth_ff(const __grid_constant__ FrontArgs a)
 {
     presmooth_body<PairFF>(a);
@@ -275,10 +277,12 @@ __device__ __forceinline__ void boundary_gface(const float4 *__restrict__ v0, co
 // boundaries also the face towards the ghost.  The flat index has i fastest,
 // m slowest: blocks at work together cover a few planes of all frames, whose
 // neighbouring frames and planes are then read from L2.
-// Bound by issue and the FP32 pipe (about 950 instructions per voxel with two
-// images).  At 256^2 x 128 x 20: two images 9.5 ms at five blocks of 128
-// threads (96 registers), 10.4 at 128 registers, 11.0 at 80; one image 5.1 ms at
-// 80 registers, 5.5 at 96.  The kernel it replaces (scalar float-float, every
+// Bound by latency: about 950 instructions per voxel with two images, in chains
+// of float-float operations and loads, issue 41 % busy and DRAM at 31 % of the
+// copy rate with the 28 % of the warps that 96 registers leave (192^2 x 96 x 12).
+// At 256^2 x 128 x 20: two images 9.8 ms; among register limits tried side by
+// side 9.5 ms at five blocks of 128 threads (96 registers, some spilled), 10.4 at
+// 128 registers, 11.0 at 80; one image 5.1 ms at 80 registers, 5.5 at 96.  The kernel it replaces (scalar float-float, every
 // difference formed at each of its faces) took 14.5 ms for two.
 constexpr int GFACES_THREADS = 128;
 template <bool TWO>

@@ -139,8 +139,9 @@ ss4d_status ss4d_solver_set_stream(ss4d_solver *s, void *stream);
 ss4d_status ss4d_solver_set_arith(ss4d_solver *s, ss4d_arith arith);
 /* Schedule of the colour-split sweeps: k_block = depth of the k blocks in
  * the tile order of the kernels that walk tiles (>= 1), max_grid caps the
- * persistent grid (0 = as many blocks as fit on the device).  Results do not
- * depend on either. */
+ * persistent grid (0 = as many blocks as fit on the device; half of that, a
+ * block per SM, lets two handles' loops share it).  Results do not depend on
+ * either. */
 ss4d_status ss4d_solver_set_tiling(ss4d_solver *s, int k_block, int max_grid);
 /* Block order of the mixed form's coefficient assembly (its faces and
  * coefficient kernels): 0 = frame by frame; planes >= 1 = in blocks of that

@@ -248,7 +248,7 @@ extern "C" ss4d_status ss4d_wsnet_set_test_withhold_loads(ss4d_wsnet *n, int ena
 {
     if (!n)
         return nfail(SS4D_ERR_INVALID, "invalid argument: network is NULL");
-    n->withhold_loads = enable;
+    n->withhold_loads = enable == 2 ? 2 : enable != 0;
     return SS4D_OK;
 }
 

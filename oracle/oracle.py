@@ -1,7 +1,7 @@
 """ctypes wrapper of the CPU oracle (oracle/ss4d_oracle.c) — TEST INFRASTRUCTURE ONLY.
 
 Used by tests/, __graft_entry__.smoke() and bench.py's CPU-baseline leg as
-the checker of the CUDA path; the product never imports it.  Arrays are
+the oracle of the CUDA path; the product never imports it.  Arrays are
 numpy float64 in the reference's padded layout, shape (lMax, kMax, jMax, iMax).
 Parameters are an ``ss4d_params``-layout ctypes structure (include/ss4d.h).
 """

@@ -3,7 +3,7 @@
  *
  * A CPU restatement, in plain C99, of the reference's semi-implicit
  * subjective-surfaces / mean-curvature-flow path (segmentation4D.c and
- * mcf_4D.c of 88MARK08/4D-image-segmentation-algorithm).  It is the checker
+ * mcf_4D.c of 88MARK08/4D-image-segmentation-algorithm).  It is the oracle
  * the CUDA path is compared with; nothing in the product links or calls it.
  * Only tests/, __graft_entry__.smoke() and bench.py's CPU-baseline leg load it.
  *
